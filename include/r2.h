@@ -180,7 +180,7 @@ r2_status r2_filter_scene_grid(const r2_filter_scene* scene, float voxel_size,
  * (nullable): 20 floats per voxel; d_fp16 (nullable): 8 halves per voxel
  * (density, Sxx, Syy, Szz, Sxy, Sxz, Syz, 0).  stream: cudaStream_t or NULL.
  * stats_out (nullable, host): [0]=voxels, [1]=voxels with candidate geometry,
- * [2]=kernel milliseconds of the per-voxel sampling kernel. */
+ * [2]=device milliseconds of the filter's kernels. */
 r2_status r2_filter_scene_run(r2_filter_scene* scene, const r2_filter_grid* grid,
                               const r2_filter_params* params, r2_voxel* d_out, float* d_wide,
                               uint16_t* d_fp16, void* stream, double* stats_out);
@@ -194,8 +194,9 @@ r2_status r2_filter_scene_run_eig(r2_filter_scene* scene, const r2_filter_grid* 
                                   const r2_filter_params* params, r2_voxel* d_out, float* d_wide,
                                   uint16_t* d_fp16, float* d_eig, void* stream, double* stats_out);
 /* The same LOD through the counting build of the sampling kernel (same
- * payloads, slower): counts_out[0] rays traced, [1] inner BVH nodes visited,
- * [2] triangles tested -- the operation counts behind the filter's
+ * payloads, slower): counts_out[0] rays traced, [1] inner BVH nodes visited (a
+ * walk shared by neighbouring voxels counts for each of them), [2] triangles
+ * tested by the rays -- the operation counts behind the filter's
  * arithmetic roofline.  Waits for the result. */
 r2_status r2_filter_scene_count(r2_filter_scene* scene, const r2_filter_grid* grid,
                                 const r2_filter_params* params, r2_voxel* d_out, uint64_t* counts_out);

@@ -129,7 +129,7 @@ r2_status r2_filter_scene_count(r2_filter_scene* scene, const r2_filter_grid* gr
   r2::DBuf<unsigned long long> ops(3);
   cudaStream_t s = scene->impl->stream();
   R2_CUDA(cudaMemsetAsync(ops.get(), 0, 3 * sizeof(unsigned long long), s));
-  scene->impl->run(*grid, *params, 0, d_out, nullptr, nullptr, s, nullptr, nullptr, nullptr, ops.get());
+  scene->impl->run(*grid, *params, 0, d_out, nullptr, nullptr, s, nullptr, nullptr, 0, nullptr, ops.get());
   unsigned long long h[3] = {0, 0, 0};
   ops.download(h, 3, s);
   R2_CUDA(cudaStreamSynchronize(s));
@@ -150,8 +150,8 @@ r2_status r2_filter_scene_run_eig(r2_filter_scene* scene, const r2_filter_grid* 
                                   double* stats_out) {
   R2_API_BEGIN
   R2_REQUIRE(scene && grid && params && d_out && d_eig, R2_ERR_INVALID_ARGUMENT, "null argument");
-  scene->impl->run(*grid, *params, 0, d_out, d_wide, d_fp16, (cudaStream_t)stream, stats_out, nullptr, nullptr,
-                   nullptr, d_eig);
+  scene->impl->run(*grid, *params, 0, d_out, d_wide, d_fp16, (cudaStream_t)stream, stats_out, nullptr, 0,
+                   nullptr, nullptr, d_eig);
   R2_API_END
 }
 

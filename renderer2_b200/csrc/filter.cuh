@@ -29,8 +29,17 @@ struct FilterLaunch {
   float* wide;               // nullable
   uint16_t* fp16;            // nullable
   float* eig;                // nullable: 12 floats per voxel, eigenvalues and eigenvectors of the mean S
-  uint32_t* work;            // candidate voxel ids
-  uint32_t* counters;        // [0] candidates, [1] queue head
+  // Work of this launch: the bricks brickFirst .. brickFirst + brickCount - 1
+  // (2x2x2 voxels, x fastest), the ones near triangles
+  // (bricks), the voxels to sample (entries: index and place of the candidate
+  // list in the pool, from both ends) and the counters.
+  uint32_t brickFirst, brickCount;
+  float brickOffset;         // from a brick's centre to its farthest voxel centre
+  uint32_t* bricks;
+  uint2* entries;
+  int* pool;                 // candidate lists: their length, then triangles
+  uint32_t poolWords;
+  uint32_t* counters;        // kFilterCounters of them, see below
   unsigned long long* ops;   // nullable: counting build, [0] rays, [1] inner nodes visited, [2] triangles tested
   // texture maps (nullable): 3 texture coordinates per BVH-order triangle, the
   // texels, and per material its {albedo, glossy, normal, opacity} texture (-1: none)
@@ -40,10 +49,21 @@ struct FilterLaunch {
   const int4* matTex;
 };
 
-// Host launchers.  `classify` writes the empty payload for voxels whose
-// bounding sphere overlaps no triangle box and appends the others to the
-// work list; `sample` is the persistent warp-per-voxel kernel.
-void launch_filter_classify(const FilterLaunch& L, cudaStream_t s);
+// Counters of a launch: voxels with a triangle within reach (of the whole
+// grid); then, cleared for every part of it, the bricks listed, the entries
+// taken, the entries at the end of the list, and those at its front and the
+// pool words used (one 64-bit word).
+enum { kCountSampled = 0, kCountBricks = 1, kCountTaken = 2, kCountBack = 3, kCountFront = 4, kFilterCounters = 6 };
+
+// Bricks of the grid, x fastest.
+R2_HD uint32_t brick_count(const FilterLaunch& L) {
+  return ((uint32_t)(L.nx + 1) / 2) * ((uint32_t)(L.ny + 1) / 2) * ((uint32_t)(L.nz + 1) / 2);
+}
+
+// Host launchers of one part of a grid.  `lists` writes the empty payload of
+// voxels that no triangle is near and collects the others and their candidate
+// triangles; `sample` is the persistent warp-per-voxel kernel.
+void launch_filter_lists(const FilterLaunch& L, cudaStream_t s);
 void launch_filter_sample(const FilterLaunch& L, cudaStream_t s);
 
 }  // namespace r2

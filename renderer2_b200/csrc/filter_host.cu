@@ -156,7 +156,7 @@ FilterScene::FilterScene(const float* positions, uint32_t nverts, const uint32_t
       if (anyAlpha) triAlpha_.upload(triAlpha.data(), triAlpha.size(), stream_);
     }
   }
-  counters_.alloc(2);
+  counters_.alloc(kFilterCounters);
   R2_CUDA(cudaEventCreate(&ev0_));
   R2_CUDA(cudaEventCreate(&ev1_));
   R2_CUDA(cudaStreamSynchronize(stream_));
@@ -176,9 +176,22 @@ r2_filter_grid FilterScene::grid(float voxelSize) const {
   return setup_grid(worldLo_, worldHi_, worldToModel_, voxelSize);
 }
 
+// Words of the scene's own work space: 24 per voxel up to 16 MiB, so that the
+// lists of a small dense grid fit (the 48^3 grid of 400,000 triangles needs 22
+// a voxel), then at least two per voxel (a quarter of the output; the 256^3
+// grid of 1M triangles uses 1.8) up to 64 MiB: larger grids are filtered in parts.
+static size_t work_words(size_t nvox) {
+  const size_t small = std::min<size_t>(24 * nvox, (size_t)1 << 22);
+  return std::min<size_t>(std::max(std::max<size_t>(2 * nvox, small), kFilterMinWork), (size_t)1 << 24);
+}
+
+// Most voxels of a part: at most kCandMax + 1 list words each stay below 2^32.
+constexpr size_t kMaxPart = (size_t)1 << 22;
+
 void FilterScene::run(const r2_filter_grid& g, const r2_filter_params& p, uint32_t lod, r2_voxel* d_out,
                       float* d_wide, uint16_t* d_fp16, cudaStream_t s, double* stats,
-                      uint32_t* d_work, uint32_t* d_counters, unsigned long long* d_ops, float* d_eig) {
+                      uint32_t* d_work, size_t workWords, uint32_t* d_counters, unsigned long long* d_ops,
+                      float* d_eig) {
   R2_REQUIRE(d_out, R2_ERR_INVALID_ARGUMENT, "null output");
   R2_REQUIRE(p.sggx_projection <= 1u && p.sggx_floor >= 0.0f && p.sggx_floor < 1.0f, R2_ERR_INVALID_ARGUMENT,
              "sggx_projection must be 0 or 1 and sggx_floor in [0, 1)");
@@ -234,22 +247,41 @@ void FilterScene::run(const r2_filter_grid& g, const r2_filter_params& p, uint32
   L.out = d_out;
   L.wide = d_wide;
   L.fp16 = d_fp16;
-  if (d_work) {
-    L.work = d_work;
-  } else {
-    work_.reserve(nvox);
-    L.work = work_.get();
-  }
   L.counters = d_counters ? d_counters : counters_.get();
   L.ops = d_ops;
-  R2_CUDA(cudaMemsetAsync(L.counters, 0, 2 * sizeof(uint32_t), s));
-  launch_filter_classify(L, s);
+  if (!d_work) {
+    workWords = work_words(nvox);
+    work_.reserve(workWords);
+    d_work = work_.get();
+  }
+  // half the longest diagonal of a brick's eight voxel centres
+  const V3 hx = xform_vector(L.indexToWorld, v3(0.5f, 0.0f, 0.0f)), hy = xform_vector(L.indexToWorld, v3(0.0f, 0.5f, 0.0f)),
+           hz = xform_vector(L.indexToWorld, v3(0.0f, 0.0f, 0.5f));
+  L.brickOffset = std::max(std::max(length(hx + hy + hz), length(hx + hy - hz)),
+                           std::max(length(hx - hy + hz), length(hy + hz - hx)));
+  // The grid in parts of bricks whose lists fit the work space: of W words,
+  // W / 6 voxels at most, two words each for their entries (first: they are
+  // 8-byte aligned), one per brick, and what is left for candidate lists.
+  const uint32_t total = brick_count(L);
+  const uint32_t part = (uint32_t)std::min<size_t>(total, std::min<size_t>(workWords / 6, kMaxPart) / 8);
+  R2_REQUIRE(part > 0, R2_ERR_INVALID_ARGUMENT, "filter work space too small");
+  L.entries = reinterpret_cast<uint2*>(d_work);
+  L.bricks = d_work + 16 * (size_t)part;
+  L.pool = reinterpret_cast<int*>(L.bricks + part);
+  L.poolWords = (uint32_t)std::min<size_t>(workWords - 17 * (size_t)part, 0xFFFFFFFEu);
+  R2_CUDA(cudaMemsetAsync(L.counters, 0, kFilterCounters * sizeof(uint32_t), s));
   R2_CUDA(cudaEventRecord(ev0_, s));
-  launch_filter_sample(L, s);
+  for (L.brickFirst = 0; L.brickFirst < total; L.brickFirst += L.brickCount) {
+    L.brickCount = std::min(part, total - L.brickFirst);
+    if (L.brickFirst > 0)
+      R2_CUDA(cudaMemsetAsync(L.counters + kCountBricks, 0, (kFilterCounters - kCountBricks) * sizeof(uint32_t), s));
+    launch_filter_lists(L, s);
+    launch_filter_sample(L, s);
+  }
   R2_CUDA(cudaEventRecord(ev1_, s));
   if (stats) {
     uint32_t cand = 0;
-    R2_CUDA(cudaMemcpyAsync(&cand, L.counters, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    R2_CUDA(cudaMemcpyAsync(&cand, L.counters + kCountSampled, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     R2_CUDA(cudaStreamSynchronize(s));
     float ms = 0.0f;
     R2_CUDA(cudaEventElapsedTime(&ms, ev0_, ev1_));

@@ -10,6 +10,8 @@ namespace r2 {
 r2_filter_grid setup_grid(V3 minWorld, V3 maxWorld, const M43& worldToModel, float voxelSize);
 void world_aabb(V3 mlo, V3 mhi, const M43& modelToWorld, V3* wlo, V3* whi);
 
+constexpr size_t kFilterMinWork = 1u << 16;  // least words of a work space
+
 class FilterScene {
  public:
   // uvs (nullable): 2 texture coordinates per vertex; maps (nullable): the
@@ -23,15 +25,16 @@ class FilterScene {
   FilterScene& operator=(const FilterScene&) = delete;
 
   r2_filter_grid grid(float voxelSize) const;
-  // One LOD.  d_work/d_counters (nullable) override the scene-owned work list
-  // (nx*ny*nz words) and counters (2 words).  d_ops (nullable, 3 zeroed words)
+  // One LOD.  d_work (nullable, workWords words, 8-byte aligned, at least
+  // kFilterMinWork) and d_counters (kFilterCounters words, 8-byte aligned)
+  // override the scene-owned work space and counters.  d_ops (nullable, 3 zeroed words)
   // selects the counting build of the sampling kernel, which adds the rays
   // traced, inner nodes visited and triangles tested.
   // d_eig (nullable): 12 floats per voxel, the FP64 eigendecomposition of the mean S.
   void run(const r2_filter_grid& g, const r2_filter_params& p, uint32_t lod, r2_voxel* d_out,
            float* d_wide, uint16_t* d_fp16, cudaStream_t s, double* stats,
-           uint32_t* d_work = nullptr, uint32_t* d_counters = nullptr, unsigned long long* d_ops = nullptr,
-           float* d_eig = nullptr);
+           uint32_t* d_work = nullptr, size_t workWords = 0, uint32_t* d_counters = nullptr,
+           unsigned long long* d_ops = nullptr, float* d_eig = nullptr);
 
   const DeviceBvh& bvh() const { return bvh_; }
   cudaStream_t stream() const { return stream_; }

@@ -5,20 +5,20 @@
 // allocation allowed after start-up, an embedding application that owns every
 // device allocation through its own pool, or a latency-bound caller that
 // cannot afford the device-wide synchronisation an allocation may imply.  For
-// them, r2_filter_scene_run_static filters one LOD with the voxel work list
-// and queue counters placed in a fixed scratch array that lives in this
+// them, r2_filter_scene_run_static filters one LOD with the work space and
+// counters placed in a fixed scratch array that lives in this
 // library's device image instead of a buffer allocated per call.  The scene
 // (BVH, shading data) is created beforehand, when allocation is allowed.
 //
-// The scratch holds at most kStaticMaxVoxels voxel ids (4 MiB) plus two
-// counters; every GPU that loads the library keeps it until the process ends.
+// The scratch is kStaticMaxVoxels words (4 MiB) and the counters; a grid of
+// that many voxels is worked off in six parts.  Every GPU that loads the library keeps it until the process ends.
 // Larger grids are rejected with R2_ERR_UNSUPPORTED.  All calls share the one
 // array: calls that overlap on the GPU (different streams, or different host
 // threads without ordering) race on it and must not be issued concurrently.
 // A NULL stream means the device's legacy default stream, so calls given NULL
 // run one after another whatever scene they filter.  The array keeps the
 // previous call's contents: the counters are cleared by every call before use;
-// the work list needs no clearing (each call writes the entries it reads).
+// the rest needs no clearing (each call writes the entries it reads).
 // The first call on a device resolves the array's device address with
 // cudaGetSymbolAddress (once per device, with that device current); make that
 // first call before any stream capture.  The device current at the call, and
@@ -34,7 +34,7 @@ constexpr size_t kStaticMaxVoxels = (size_t)1 << 20;
 constexpr int kStaticMaxDevices = 64;
 }  // namespace r2
 
-// Work list followed by the two queue counters.
+// Work space followed by the counters.
 static __device__ __align__(256) uint32_t g_filterScratch[r2::kStaticMaxVoxels + 64];
 
 namespace r2 {
@@ -84,6 +84,6 @@ extern "C" r2_status r2_filter_scene_run_static(r2_filter_scene* scene, const r2
   }
   uint32_t* work = r2::scratch_address(dev);
   uint32_t* counters = work + r2::kStaticMaxVoxels;
-  sc->run(*grid, *params, 0, d_out, d_wide, d_fp16, s, nullptr, work, counters);
+  sc->run(*grid, *params, 0, d_out, d_wide, d_fp16, s, nullptr, work, r2::kStaticMaxVoxels, counters);
   R2_API_END
 }

@@ -1,6 +1,8 @@
 // Request loop for render and filter jobs (see server.h).
 #include "server.h"
 
+#include "filter.cuh"
+
 #include <string.h>
 
 #include <chrono>
@@ -157,10 +159,10 @@ bool Server::start(Slot& s, ServerJob* j) {
     } else {
       const size_t nvox = (size_t)j->grid.num_voxels[0] * j->grid.num_voxels[1] * j->grid.num_voxels[2];
       s.vox.reserve_grow(nvox);
-      s.work.reserve_grow(nvox);
-      s.counters.reserve(2);
+      s.work.reserve_grow(std::max(nvox, kFilterMinWork));
+      s.counters.reserve(kFilterCounters);
       j->fscene->run(j->grid, j->fp, j->lod, s.vox.get(), nullptr, nullptr, st, nullptr, s.work.get(),
-                     s.counters.get());
+                     s.work.size(), s.counters.get());
       R2_CUDA(cudaMemcpyAsync(s.staging(j->outBytes), s.vox.get(), j->outBytes, cudaMemcpyDeviceToHost, st));
       *s.pinnedBound = 0;
     }
