@@ -290,8 +290,8 @@ typedef struct r2_render_params {
  * gives the same frames bit for bit.  0 selects the built-in default. */
 typedef struct r2_render_tuning {
   uint32_t track_steps; /* media: tracking steps a lane of the persistent tracker takes between refills (1..1024) */
-  uint32_t trav_visits; /* BVH node/leaf visits a lane takes between refill checks of the surface kernels */
-  uint32_t trav_refill; /* finished lanes of a warp (1..32) that make it take new rays */
+  uint32_t trav_visits; /* BVH nodes a lane visits at most between refill checks of the surface kernels */
+  uint32_t trav_refill; /* idle lanes of a warp (1..32) at which it ends finished rays and takes new ones */
   uint32_t wave_paths;  /* paths per wave: a wave renders the largest divisor of spp samples of every
                            pixel that keeps width*height*samples within it (at least one sample) */
   uint32_t media_rounds; /* media: queued rounds of medium boundaries per bounce (1..32) before the
@@ -303,10 +303,8 @@ typedef struct r2_render_tuning {
                            a path or shadow ray whose loop reaches it ends, and the synchronous
                            render calls return R2_ERR_DEVICE_TIMEOUT with the frame written.  The
                            reference's loops have no bound (nvdb_medium_impl.hpp:98-136, 155-186). */
-  uint32_t top_nodes;   /* surface scenes: BVH nodes 0 .. top_nodes-1 copied into each traversal block's
-                           shared memory and read from there (0: off; at most 256).  With the PLOC
-                           builder a parent's index is below its children's, so these are the top
-                           levels of the tree (of the top-level tree in two-level scenes). */
+  uint32_t top_nodes;   /* at most 256; without effect since the surface kernels traverse wide nodes,
+                           whose top levels stay in L1 */
   uint32_t sort_rays;   /* surface scenes: 1 reorders each bounce's rays after the first by direction
                            octant, dominant axis and origin cell before tracing them (a counting sort
                            over 256 keys); 0: off.  The order of rays changes no bit of a frame. */

@@ -50,7 +50,7 @@ struct __align__(16) BvhInstance {
   int root;       // the instance's BLAS root in the global node array
   int vdelta;     // hit code - global triangle index
   int identity;   // 1: object space is world space (no transform)
-  int pad;
+  int wide;       // the BLAS root among the wide nodes (wide_bvh.cuh)
 };
 
 struct BvhView {
@@ -59,8 +59,6 @@ struct BvhView {
   uint32_t ntris;
   BvhAlpha alpha;      // zero: every triangle opaque
   const BvhInstance* inst;  // two-level scenes: the instances (nodes start with the top level), else null
-  const BvhNode* top;       // nodes 0 .. ntop-1 staged in shared memory by the caller (kTop traversals)
-  int ntop;
 };
 
 R2_HD bool alpha_opaque(const BvhAlpha& a, int tri, float b1, float b2) {
@@ -256,7 +254,7 @@ R2_HD bool trace_all_have_leaf(bool mine) {
 // leaf of the instance has been tested.  The stack then holds the top-level
 // path, the marker and the instance's path: the builder bounds the sum of the
 // two heights plus two by R2_BVH_STACK.
-template <bool kAnyHit, bool kCount = false, bool kAlpha = false, bool kInst = false, bool kTop = false>
+template <bool kAnyHit, bool kCount = false, bool kAlpha = false, bool kInst = false>
 R2_HD bool trace_advance(const BvhView& bvh, TraceState& s, int* stack, float* stackT, int maxVisits) {
   int budget = maxVisits;
   while (budget > 0) {
@@ -278,19 +276,10 @@ R2_HD bool trace_advance(const BvhView& bvh, TraceState& s, int* stack, float* s
       if (kCount) ++s.nodes;
       const int cur = s.cur;
 #if defined(__CUDA_ARCH__)
-      float4 b0, b1, bz;
-      int4 ch;
-      if (kTop && cur < bvh.ntop) {
-        b0 = bvh.top[cur].b0;
-        b1 = bvh.top[cur].b1;
-        bz = bvh.top[cur].bz;
-        ch = bvh.top[cur].ch;
-      } else {
-        b0 = __ldg(&bvh.nodes[cur].b0);
-        b1 = __ldg(&bvh.nodes[cur].b1);
-        bz = __ldg(&bvh.nodes[cur].bz);
-        ch = __ldg(&bvh.nodes[cur].ch);
-      }
+      const float4 b0 = __ldg(&bvh.nodes[cur].b0);
+      const float4 b1 = __ldg(&bvh.nodes[cur].b1);
+      const float4 bz = __ldg(&bvh.nodes[cur].bz);
+      const int4 ch = __ldg(&bvh.nodes[cur].ch);
 #else
       const float4 b0 = bvh.nodes[cur].b0;
       const float4 b1 = bvh.nodes[cur].b1;

@@ -348,91 +348,18 @@ __device__ __noinline__ PhaseSample phase_sample_nc(const MediumView* M, Sggx g,
 }
 __device__ __noinline__ Ray voxel_border_nc(const MediumView* M, Ray r) { return instance_move_to_voxel_border(*M, r); }
 
-// Persistent BVH traversal with dynamic ray fetch (Aila and Laine,
-// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): the
-// lanes of a warp run their rays in rounds of `visits` node/leaf visits, and
-// as soon as `refill` lanes have finished (or all of them) the warp takes as
-// many new items from the queue with one atomic, so that lanes do not idle
-// behind the warp's longest ray.  begin(k, s, &item) starts item k (false: it
-// needed no traversal and is done); end(item, s) consumes a finished query.
-// Results do not depend on visits or refill.
-// A ray still unfinished after kMaxTraceVisits visits (a correct traversal
-// visits each node at most once) is ended as a miss and counted in *bound.
-constexpr int kMaxTraceVisits = 1 << 26;
-
-template <bool kAnyHit, bool kAlpha, bool kInst, bool kTop, class Begin, class End>
-__device__ __forceinline__ void trace_persistent(const BvhView& bvh, uint32_t n, uint32_t* taken, int visits,
-                                                 int refill, unsigned int* bound, Begin begin, End end) {
-  int stack[R2_BVH_STACK];
-  float stackT[R2_BVH_STACK];
-  TraceState s;
-  uint32_t item = 0;
-  int spent = 0;  // visits of the lane's current ray
-  bool active = false;
-  bool more = true;  // warp-uniform: the queue may still hold items
-  const int lane = threadIdx.x & 31;
-  while (true) {
-    if (more) {
-      const unsigned idle = __ballot_sync(0xffffffffu, !active);
-      const int nIdle = __popc(idle);
-      if (nIdle >= refill || idle == 0xffffffffu) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(taken, (uint32_t)nIdle);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base + (uint32_t)nIdle >= n) more = false;
-        if (!active) {
-          const uint32_t k = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-          if (k < n) {
-            active = begin(k, s, &item);
-            spent = 0;
-          }
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, active) == 0) {
-      if (!more) break;
-      continue;
-    }
-    if (active) {
-      bool done = trace_advance<kAnyHit, false, kAlpha, kInst, kTop>(bvh, s, stack, stackT, visits);
-      spent += visits;
-      if (!done && spent >= kMaxTraceVisits) {
-        s.best.tri = -1;
-        atomicAdd(bound, 1u);
-        done = true;
-      }
-      if (done) {
-        if (!kInst) {  // one level: the traversal ray is the world ray (keeps wo/wd out of the live state)
-          s.wo = s.r.o;
-          s.wd = s.r.d;
-        }
-        end(item, s);
-        active = false;
-      }
-    }
-  }
-}
-
 __device__ __forceinline__ int trav_visits(const RenderLaunch& L) { return (int)max(1u, L.travVisits); }
 __device__ __forceinline__ int trav_refill(const RenderLaunch& L) { return (int)min(32u, max(1u, L.travRefill)); }
 
 // The persistent traversal of the scene's BVH (kAlpha: alpha-tested
-// triangles; kInst: two levels).  kTop: the block first copies BVH nodes
-// 0 .. L.topNodes-1 (the host keeps the count within the tree and
-// kMaxTopNodes) into its dynamic shared memory and reads them from there.
-// Every thread of the block calls this once.
-template <bool kAnyHit, bool kAlpha, bool kInst, bool kTop, class Begin, class End>
+// triangles; kInst: two levels).  Every warp of a block of kTraceWarps warps
+// calls this once.
+constexpr int kTraceWarps = 4;
+template <bool kAnyHit, bool kAlpha, bool kInst, class Begin, class End>
 __device__ __forceinline__ void trace_scene(const RenderLaunch& L, uint32_t n, uint32_t* taken, Begin begin, End end) {
-  BvhView bvh = L.scene.bvh;
-  if (kTop) {
-    extern __shared__ BvhNode sTop[];
-    const int ntop = (int)L.topNodes;
-    for (int k = threadIdx.x; k < ntop; k += blockDim.x) sTop[k] = bvh.nodes[k];
-    __syncthreads();
-    bvh.top = sTop;
-    bvh.ntop = ntop;
-  }
-  trace_persistent<kAnyHit, kAlpha, kInst, kTop>(bvh, n, taken, trav_visits(L), trav_refill(L), L.bound, begin, end);
+  __shared__ WideWarp sRays[kTraceWarps];
+  wide_rays<kAnyHit, kAlpha, kInst>(L.scene.bvh, L.scene.wide, sRays[threadIdx.x >> 5], n, taken, trav_visits(L),
+                                    trav_refill(L), L.bound, begin, end);
 }
 
 // ------------------------------------------------------------------ ray order
@@ -542,8 +469,8 @@ __device__ __forceinline__ void extend_result(const RenderLaunch& L, uint32_t p,
 
 // One instantiation per traversal variant (no triangles; alpha test, two
 // levels, shared top nodes), each with its own register allocation.
-template <bool kTris, bool kAlpha, bool kInst, bool kTop>
-__global__ void __launch_bounds__(128, 10) k_extend(RenderLaunch L) {
+template <bool kTris, bool kAlpha, bool kInst>
+__global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) {
   const uint32_t n = *(volatile uint32_t*)&L.st.counts[L.bounce];
   const uint32_t* q = path_queue(L, L.bounce);
   if constexpr (!kTris) {
@@ -554,16 +481,18 @@ __global__ void __launch_bounds__(128, 10) k_extend(RenderLaunch L) {
       extend_result(L, p, d, scene_closest<false>(L.scene, xyz(L.st.rayO[p]), d, kDefaultTmax));
     }
   } else {
-    auto begin = [&](uint32_t k, TraceState& s, uint32_t* item) {
+    auto begin = [&](uint32_t k, V3* o, V3* d, float* tmax, uint32_t* item) {
       const uint32_t p = q[k];
       *item = p;
-      trace_begin(s, xyz(L.st.rayO[p]), xyz(L.st.rayD[p]), kDefaultTmax);
+      *o = xyz(L.st.rayO[p]);
+      *d = xyz(L.st.rayD[p]);
+      *tmax = kDefaultTmax;
       return true;
     };
-    auto end = [&](uint32_t p, const TraceState& s) {
-      extend_result(L, p, s.wd, scene_closest_after<false>(L.scene, s.wo, s.wd, kDefaultTmax, s.best));
+    auto end = [&](uint32_t p, V3 o, V3 d, const Hit& h) {
+      extend_result(L, p, d, scene_closest_after<false>(L.scene, o, d, kDefaultTmax, h));
     };
-    trace_scene<false, kAlpha, kInst, kTop>(L, n, &L.st.counts[kTravCounters + 2 * L.bounce], begin, end);
+    trace_scene<false, kAlpha, kInst>(L, n, &L.st.counts[kTravCounters + 2 * L.bounce], begin, end);
   }
 }
 
@@ -1162,8 +1091,8 @@ __device__ __forceinline__ Ray shadow_ray(float4 o, float4 d) {
 }
 
 // Visibility of every shadow record of a scene without media.
-template <bool kTris, bool kAlpha, bool kInst, bool kTop>
-__global__ void __launch_bounds__(128, 10) k_shadow_surfaces(RenderLaunch L) {
+template <bool kTris, bool kAlpha, bool kInst>
+__global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderLaunch L) {
   const uint32_t n = event_count(L);
   uint32_t traced = 0;
   if constexpr (!kTris) {
@@ -1179,7 +1108,7 @@ __global__ void __launch_bounds__(128, 10) k_shadow_surfaces(RenderLaunch L) {
       L.st.shTr[j] = tr;
     }
   } else {
-    auto begin = [&](uint32_t j, TraceState& s, uint32_t* item) {
+    auto begin = [&](uint32_t j, V3* ro, V3* rd, float* tmax, uint32_t* item) {
       const float4 o = L.st.shO[j];
       *item = j;
       if (!(o.w > 0.0f)) {  // no ray for this record
@@ -1188,21 +1117,23 @@ __global__ void __launch_bounds__(128, 10) k_shadow_surfaces(RenderLaunch L) {
       }
       ++traced;
       const Ray r = shadow_ray(o, L.st.shD[j]);
-      trace_begin(s, r.o, r.d, r.tmax);
+      *ro = r.o;
+      *rd = r.d;
+      *tmax = r.tmax;
       return true;
     };
-    auto end = [&](uint32_t j, const TraceState& s) {
-      bool occluded = s.best.tri >= 0;
+    auto end = [&](uint32_t j, V3 ro, V3 rd, const Hit& h) {
+      bool occluded = h.tri >= 0;
       if (!occluded && L.scene.nshapes > 0) {
         SceneView noTris = L.scene;
         noTris.hasTris = 0;
         Hit none;
         none.tri = -1;
-        occluded = __float_as_int(scene_closest_after<false>(noTris, s.wo, s.wd, s.best.t, none).w) != -1;
+        occluded = __float_as_int(scene_closest_after<false>(noTris, ro, rd, h.t, none).w) != -1;
       }
       L.st.shTr[j] = occluded ? 0.0f : 1.0f;
     };
-    trace_scene<true, kAlpha, kInst, kTop>(L, 2 * n, &L.st.counts[kTravCounters + 2 * L.bounce + 1], begin, end);
+    trace_scene<true, kAlpha, kInst>(L, 2 * n, &L.st.counts[kTravCounters + 2 * L.bounce + 1], begin, end);
   }
   if (L.stats) {
     for (int o = 16; o > 0; o >>= 1) traced += __shfl_down_sync(0xffffffffu, traced, o);
@@ -1359,21 +1290,15 @@ int resident_blocks(K kernel, int threads, size_t smem = 0) {
 
 int g_trackBlocks[4] = {0, 0, 0, 0};  // resident blocks of k_track<dda, sample>, by dda + 2 sample
 
-int g_travBlocks[2] = {0, 0};  // resident blocks of k_extend, k_shadow_surfaces
-
-// The surface traversal kernels by variant: alpha + 2 * two-level + 4 * top
-// nodes; 8: a scene without triangles.
+// The surface traversal kernels by variant: alpha + 2 * two-level; 4: a scene
+// without triangles.
 using RenderKernel = void (*)(RenderLaunch);
-const RenderKernel kExtendVariants[9] = {
-    k_extend<true, false, false, false>, k_extend<true, true, false, false>, k_extend<true, false, true, false>,
-    k_extend<true, true, true, false>,   k_extend<true, false, false, true>, k_extend<true, true, false, true>,
-    k_extend<true, false, true, true>,   k_extend<true, true, true, true>,   k_extend<false, false, false, false>};
-const RenderKernel kShadowVariants[9] = {
-    k_shadow_surfaces<true, false, false, false>, k_shadow_surfaces<true, true, false, false>,
-    k_shadow_surfaces<true, false, true, false>,  k_shadow_surfaces<true, true, true, false>,
-    k_shadow_surfaces<true, false, false, true>,  k_shadow_surfaces<true, true, false, true>,
-    k_shadow_surfaces<true, false, true, true>,   k_shadow_surfaces<true, true, true, true>,
-    k_shadow_surfaces<false, false, false, false>};
+const RenderKernel kExtendVariants[5] = {k_extend<true, false, false>, k_extend<true, true, false>,
+                                         k_extend<true, false, true>, k_extend<true, true, true>,
+                                         k_extend<false, false, false>};
+const RenderKernel kShadowVariants[5] = {k_shadow_surfaces<true, false, false>, k_shadow_surfaces<true, true, false>,
+                                         k_shadow_surfaces<true, false, true>, k_shadow_surfaces<true, true, true>,
+                                         k_shadow_surfaces<false, false, false>};
 
 // k_shade by variant: 4 * media + textured + 2 * two-level.
 const RenderKernel kShadeVariants[8] = {k_shade<false, false, false>, k_shade<false, true, false>,
@@ -1386,30 +1311,23 @@ int shade_variant(const RenderLaunch& L) {
 }
 
 int trav_variant(const RenderLaunch& L) {
-  if (!L.scene.hasTris) return 8;
-  return (L.scene.bvh.alpha.alphaTex ? 1 : 0) + (L.scene.bvh.inst ? 2 : 0) + (L.topNodes ? 4 : 0);
+  if (!L.scene.hasTris) return 4;
+  return (L.scene.bvh.alpha.alphaTex ? 1 : 0) + (L.scene.bvh.inst ? 2 : 0);
 }
 
 // Resident blocks of a surface traversal kernel (0: k_extend, 1:
-// k_shadow_surfaces) of a variant with topNodes BVH nodes of dynamic shared memory.
-int trav_blocks(int which, int variant, uint32_t topNodes) {
+// k_shadow_surfaces) of a variant.
+int trav_blocks(int which, int variant) {
   static std::mutex mu;
-  static std::map<std::pair<int, uint32_t>, int> cache;
+  static int cache[2][5] = {};
   std::lock_guard<std::mutex> lock(mu);
-  const int key = which * 9 + variant;
-  auto it = cache.find({key, topNodes});
-  if (it != cache.end()) return it->second;
-  const size_t smem = topNodes * sizeof(BvhNode);
-  const RenderKernel k = which == 0 ? kExtendVariants[variant] : kShadowVariants[variant];
-  const int n = resident_blocks(k, 128, smem);
-  cache[{key, topNodes}] = n;
+  int& n = cache[which][variant];
+  if (n == 0) n = resident_blocks(which == 0 ? kExtendVariants[variant] : kShadowVariants[variant], kTraceWarps * 32);
   return n;
 }
 
 void query_track_blocks() {
   if (g_trackBlocks[0] != 0) return;
-  g_travBlocks[0] = resident_blocks(kExtendVariants[0], 128);
-  g_travBlocks[1] = resident_blocks(kShadowVariants[0], 128);
   g_trackBlocks[1] = resident_blocks(k_track<true, false>, 128);
   g_trackBlocks[2] = resident_blocks(k_track<false, true>, 128);
   g_trackBlocks[3] = resident_blocks(k_track<true, true>, 128);
@@ -1487,13 +1405,11 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, Wav
         k_sort_copy<<<nblocks, 256, 0, s>>>(L);
       }
       const int tv = trav_variant(L);
-      kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv, L.topNodes)), 128,
-                            L.topNodes * sizeof(BvhNode), s>>>(L);
+      kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv)), kTraceWarps * 32, 0, s>>>(L);
       mark(1);
       kShadeVariants[shade_variant(L)]<<<nblocks * 2, 128, 0, s>>>(L);
       mark(2);
-      kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv, L.topNodes)), 128,
-                            L.topNodes * sizeof(BvhNode), s>>>(L);
+      kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, s>>>(L);
     }
     mark(3);
     k_accum<<<nblocks, 256, 0, s>>>(L);

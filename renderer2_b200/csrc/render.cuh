@@ -3,6 +3,7 @@
 #pragma once
 #include "bvh_build.cuh"
 #include "media.cuh"
+#include "wide_bvh.cuh"
 
 namespace r2 {
 
@@ -22,6 +23,7 @@ struct Shape {
 // Device view of a committed scene.
 struct SceneView {
   BvhView bvh;
+  WideView wide;           // the wide nodes that the surface kernels traverse
   const float4* triN;      // 3 per BVH-order triangle: world-space vertex normals
   const uint32_t* triMat;  // per BVH-order triangle: material index
   const Material* mats;
@@ -81,13 +83,13 @@ struct PathState {
   int2* swM;        // shadow walk: current medium, draw index of the slot's stream
 };
 
-// Most BVH nodes the surface traversals stage in shared memory (16 KB per block).
+// Most wide BVH nodes the surface traversals stage in shared memory (20 KB per block).
 constexpr uint32_t kMaxTopNodes = 256;
 // Launch tuning defaults (RenderLaunch::trackSteps, travVisits, travRefill);
 // no result depends on them.
 constexpr uint32_t kDefaultTrackSteps = 8;   // tracking steps a lane takes between refills
 constexpr uint32_t kDefaultTravVisits = 32;  // BVH visits between refill checks
-constexpr uint32_t kDefaultTravRefill = 8;   // finished lanes that trigger a refill
+constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a refill
 constexpr uint32_t kDefaultWavePaths = 1u << 22;  // paths per wave a frame's samples are grouped to
 constexpr uint32_t kDefaultMediaRounds = 2;       // queued medium-boundary rounds per bounce
 constexpr uint32_t kMaxMediaRounds = 32;
@@ -132,12 +134,11 @@ struct RenderLaunch {
   uint32_t bounce;
   uint32_t dda;       // brick-grid DDA tracking (UseBrickGrid) instead of the global majorant
   uint32_t trackSteps;  // tracking steps a lane takes between refills (tuning, >= 1)
-  uint32_t travVisits;  // BVH visits a lane takes between refill checks of the surface kernels (tuning, >= 1)
+  uint32_t travVisits;  // BVH node steps a lane takes between refill checks of the surface kernels (tuning, >= 1)
   uint32_t travRefill;  // finished lanes of a warp that trigger a refill (tuning, 1..32)
   uint32_t mediaRounds; // queued medium-boundary rounds per bounce (tuning, 1..kMaxMediaRounds)
   uint32_t trackBlocks; // persistent tracker blocks per SM (tuning; 0: every resident block)
   uint32_t trackLimit;  // steps of one tracking loop after which the path ends (1..kMaxTrackingSteps)
-  uint32_t topNodes;    // BVH nodes staged in shared memory by the surface traversals (0: none, <= kMaxTopNodes)
   uint32_t sortRays;    // surface scenes: reorder each bounce's rays by a coherence key before k_extend
   unsigned long long* stats;  // nullable: [0] path segments traced, [1] shadow rays traced
   unsigned int* bound;        // paths and shadow rays ended by a loop bound (tracking steps, boundaries)

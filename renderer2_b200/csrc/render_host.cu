@@ -299,7 +299,8 @@ void RenderScene::rebuild(cudaStream_t s) {
   builder_.build(dPos_.get(), dIdx_.get(), nt, &bvh_, s);
   bvhNodes_ = bvh_.nnodes;
   bvhHeight_ = bvh_.height;
-  buildLaunches_ = builder_.launches() + 1;
+  wide_.build(bvh_.nodes.get(), bvh_.tris.get(), nullptr, 1, nt, s);
+  buildLaunches_ = builder_.launches() + WideBvh::kLaunches + 1;
   triN_.reserve((size_t)3 * nt);
   triMat_.reserve(nt);
   if (anyUV_) triUV_.reserve((size_t)3 * nt);
@@ -312,6 +313,8 @@ void RenderScene::rebuild(cudaStream_t s) {
   const BvhAlpha alpha = view_.bvh.alpha;
   view_.bvh = bvh_.view();
   view_.bvh.alpha = alpha;
+  view_.wide = wide_.view();
+  R2_CUDA(cudaStreamSynchronize(s));  // a frame may follow on another stream
 }
 
 // Device inputs and bottom-level BVHs of the mesh assets (once per commit:
@@ -433,7 +436,18 @@ void RenderScene::build_two_level(cudaStream_t s) {
   }
   R2_REQUIRE(tlas_.height + maxHeight + 2 <= R2_BVH_STACK, R2_ERR_UNSUPPORTED,
              "two-level BVH deeper than the traversal stack");
-  for (uint32_t i = 0; i < ninst; ++i) hin[i].root = (int)nodeOff[insts[i].pool];
+  // wide roots: the top level, then the pools that have triangles
+  std::vector<uint32_t> roots(1, 0u);
+  std::vector<int> wideRoot(npool, 0);
+  for (size_t k = 0; k < npool; ++k)
+    if (ntri[k] > 0) {
+      wideRoot[k] = (int)roots.size();
+      roots.push_back(nodeOff[k]);
+    }
+  for (uint32_t i = 0; i < ninst; ++i) {
+    hin[i].root = (int)nodeOff[insts[i].pool];
+    hin[i].wide = wideRoot[insts[i].pool];
+  }
   dInst_.upload(hin.data(), ninst, s);
   dInstCode_.upload(code.data(), ninst, s);
   dInstO2W_.upload(o2w.data(), o2w.size(), s);
@@ -470,6 +484,9 @@ void RenderScene::build_two_level(cudaStream_t s) {
     launches += 2;
   }
   R2_CUDA(cudaGetLastError());
+  wide_.build(gNodes_.get(), gTris_.get(), roots.data(), (uint32_t)roots.size(), (uint32_t)(totalTris + ninst), s);
+  launches += WideBvh::kLaunches;
+  view_.wide = wide_.view();
   const BvhAlpha alpha = view_.bvh.alpha;
   memset(&view_.bvh, 0, sizeof(view_.bvh));
   view_.bvh.nodes = gNodes_.get();
@@ -717,8 +734,6 @@ RenderLaunch RenderScene::make_launch(const RenderContext& ctx, const r2_camera&
   L.mediaRounds = tuning_.media_rounds;
   L.trackBlocks = tuning_.track_blocks;
   L.trackLimit = tuning_.track_limit ? tuning_.track_limit : (uint32_t)kMaxTrackingSteps;
-  // shared-memory top nodes: surface scenes only, within the tree
-  L.topNodes = media_.empty() && view_.hasTris ? std::min(tuning_.top_nodes, bvhNodes_) : 0u;
   L.sortRays = media_.empty() && view_.hasTris && tuning_.sort_rays ? 1u : 0u;
   L.bound = ctx.bound.get();
   return L;
@@ -891,18 +906,16 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
       }
     };
     static const uint32_t wavePaths[] = {1u << 20, 1u << 21, 1u << 23, 1u << 24};
-    static const uint32_t refills[] = {2, 4, 16, 32};
+    static const uint32_t refills[] = {4, 8, 12, 24};
     static const uint32_t visits[] = {8, 16, 64, 256};
     static const uint32_t steps[] = {2, 4, 16, 32};
     static const uint32_t rounds[] = {1, 4, 8, 16};
     static const uint32_t trackBlocks[] = {2, 3, 4, 6};
-    static const uint32_t topNodes[] = {64, 128, 256};
     static const uint32_t sortRays[] = {1};
     sweep(&r2_render_tuning::wave_paths, wavePaths, 4);
     if (media_.empty()) {  // the persistent surface traversals run in scenes without media
       sweep(&r2_render_tuning::trav_refill, refills, 4);
       sweep(&r2_render_tuning::trav_visits, visits, 4);
-      sweep(&r2_render_tuning::top_nodes, topNodes, 3);
       sweep(&r2_render_tuning::sort_rays, sortRays, 1);
     } else {
       sweep(&r2_render_tuning::media_rounds, rounds, 4);

@@ -167,6 +167,7 @@ class RenderScene {
   EnvHost env_;
   DeviceBvh bvh_;
   BvhBuilder builder_;
+  WideBvh wide_;  // what the surface queries traverse, collapsed from bvh_ or gNodes_ after every build
   // two-level scenes: mesh assets in model space, their instances, the top
   // level over the instances' world boxes and the concatenated node and
   // triangle arrays (top level, then the world-space meshes, then the assets)

@@ -1,0 +1,230 @@
+// Collapse of a binary BVH into the eight-wide one (wide_bvh.cuh).
+//
+// Top down: a wide node takes the two children of its binary node and opens
+// the inner child of largest area until it has eight or only leaves.  Wide
+// nodes are numbered as they are allocated (the children of a node in a row),
+// and queue[i] keeps the binary node of wide node i, so the work of a level is
+// a range of numbers.  The first levels, a few hundred nodes, run in one block
+// (a barrier costs less than a launch), the next in launches of their own,
+// and whatever lies deeper is finished by a thread per subtree.
+#include <algorithm>
+
+#include "bvh_build.cuh"
+#include "wide_bvh.cuh"
+
+namespace r2 {
+namespace {
+
+constexpr int kTopThreads = 1024;
+constexpr uint32_t kTopItems = 1024;  // items of a level from which it is a launch of its own
+constexpr int kLevels = 3;            // levels in launches of their own
+// counters: nodes allocated, blocks done, then per launch the range of its level
+enum { kWideNodes = 0, kWideDone = 1, kWideRange = 2, kWideState = kWideRange + 2 * (kLevels + 1) };
+
+struct WideBuild {
+  const BvhNode* nodes;
+  const float4* tris;
+  uint4* out;
+  uint32_t* queue;
+  uint32_t* state;
+};
+
+struct Box {
+  V3 lo, hi;
+};
+__device__ __forceinline__ float area(const Box& b) {
+  const V3 e = b.hi - b.lo;
+  return e.x * e.y + e.y * e.z + e.z * e.x;
+}
+__device__ __forceinline__ void children_of(const BvhNode* nd, Box* b, int* ref) {
+  const float4 b0 = nd->b0, b1 = nd->b1, bz = nd->bz;
+  const int4 ch = nd->ch;
+  b[0] = Box{v3(b0.x, b0.z, bz.x), v3(b0.y, b0.w, bz.y)};
+  b[1] = Box{v3(b1.x, b1.z, bz.z), v3(b1.y, b1.w, bz.w)};
+  ref[0] = ch.x;
+  ref[1] = ch.y;
+}
+
+// One axis of a node's frame: the largest power of two 2^e in whose units the
+// extent is at most 252, and an origin one unit below the box, so that a
+// child's planes and 1/64 unit around them (far more than the traversal's
+// rounding in units) lie within 0 .. 255.
+__device__ __forceinline__ void frame_axis(float lo, float hi, float* origin, uint32_t* exponent) {
+  int e = 0;
+  const float ext = hi - lo;
+  frexpf(ext / 252.0f, &e);
+  if (!(ext > 0.0f)) e = -126;
+  e = isfinite(ext) ? max(-126, min(126, e)) : 126;
+  *exponent = (uint32_t)(e + 127);
+  *origin = lo - __uint_as_float(*exponent << 23);
+}
+__device__ __forceinline__ uint32_t plane(float x, float origin, uint32_t exponent, bool upper) {
+  const double q = ((double)x - (double)origin) / (double)__uint_as_float(exponent << 23);
+  const double r = upper ? ceil(q + 0.015625) : floor(q - 0.015625);
+  if (!(r >= 0.0)) return upper && !(r < 0.0) ? 255u : 0u;  // NaN: the whole frame
+  return (uint32_t)fmin(r, 255.0);
+}
+
+static_assert(kLeafMax <= 8, "a warp's triangle queue has room for eight of each of 32 leaves");
+
+__device__ void collapse(const WideBuild& B, uint32_t w) {
+  Box box[9];
+  int ref[9];
+  children_of(&B.nodes[B.queue[w]], box, ref);
+  int n = ref[1] == R2_BVH_NONE ? 1 : 2;
+  while (n < 8) {
+    int open = -1;
+    float largest = -1.0f;
+    for (int i = 0; i < n; ++i)
+      if (ref[i] >= 0 && area(box[i]) > largest) {
+        open = i;
+        largest = area(box[i]);
+      }
+    if (open < 0) break;
+    Box b[2];
+    int r[2];
+    children_of(&B.nodes[ref[open]], b, r);
+    box[open] = b[0];
+    ref[open] = r[0];
+    box[n] = b[1];
+    ref[n] = r[1];
+    if (r[1] != R2_BVH_NONE) ++n;
+  }
+  Box all = box[0];
+  for (int i = 1; i < n; ++i) all = Box{vmin(all.lo, box[i].lo), vmax(all.hi, box[i].hi)};
+  // children to slots: the pair of child and free slot whose octant fits best, again and again
+  int slotOf[8], childAt[8];
+  for (int k = 0; k < 8; ++k) slotOf[k] = childAt[k] = -1;
+  for (int round = 0; round < n; ++round) {
+    float best = -INFINITY;
+    int bc = -1, bs = -1;
+    for (int c = 0; c < n; ++c) {
+      if (slotOf[c] >= 0) continue;
+      const V3 off = (box[c].lo + box[c].hi) - (all.lo + all.hi);
+      for (int k = 0; k < 8; ++k) {
+        if (childAt[k] >= 0) continue;
+        const float fit = (k & 1 ? off.x : -off.x) + (k & 2 ? off.y : -off.y) + (k & 4 ? off.z : -off.z);
+        if (bc < 0 || fit > best) {
+          best = fit;
+          bc = c;
+          bs = k;
+        }
+      }
+    }
+    slotOf[bc] = bs;
+    childAt[bs] = bc;
+  }
+  uint32_t inner = 0, leaf = 0;
+  for (int k = 0; k < 8; ++k)
+    if (childAt[k] >= 0) (ref[childAt[k]] >= 0 ? inner : leaf) |= 1u << k;
+  const uint32_t firstChild = inner ? atomicAdd(&B.state[kWideNodes], (uint32_t)__popc(inner)) : 0u;
+  float px, py, pz;
+  uint32_t ex, ey, ez;
+  frame_axis(all.lo.x, all.hi.x, &px, &ex);
+  frame_axis(all.lo.y, all.hi.y, &py, &ey);
+  frame_axis(all.lo.z, all.hi.z, &pz, &ez);
+  uint32_t q[6][2] = {};  // lo.x lo.y lo.z hi.x hi.y hi.z of the eight slots
+  uint32_t child = firstChild, leafWord[8] = {}, instances = 0;
+  for (int k = 0; k < 8; ++k) {
+    const int c = childAt[k];
+    if (c < 0) continue;
+    const Box& b = box[c];
+    const int half = k >> 2, shift = 8 * (k & 3);
+    q[0][half] |= plane(b.lo.x, px, ex, false) << shift;
+    q[1][half] |= plane(b.lo.y, py, ey, false) << shift;
+    q[2][half] |= plane(b.lo.z, pz, ez, false) << shift;
+    q[3][half] |= plane(b.hi.x, px, ex, true) << shift;
+    q[4][half] |= plane(b.hi.y, py, ey, true) << shift;
+    q[5][half] |= plane(b.hi.z, pz, ez, true) << shift;
+    if (ref[c] >= 0) {
+      B.queue[child++] = (uint32_t)ref[c];
+    } else {
+      leafWord[k] = (uint32_t)~ref[c];
+      if (bvh_leaf_count(ref[c]) == 0) instances = 1u;
+    }
+  }
+  uint4* out = B.out + kWideWords * (size_t)w;
+  out[0] = make_uint4(__float_as_uint(px), __float_as_uint(py), __float_as_uint(pz), ex | ey << 8 | ez << 16 | inner << 24);
+  out[1] = make_uint4(firstChild, leaf, instances, 0u);
+  out[2] = make_uint4(q[0][0], q[0][1], q[1][0], q[1][1]);
+  out[3] = make_uint4(q[2][0], q[2][1], q[3][0], q[3][1]);
+  out[4] = make_uint4(q[4][0], q[4][1], q[5][0], q[5][1]);
+  out[5] = make_uint4(leafWord[0], leafWord[1], leafWord[2], leafWord[3]);
+  out[6] = make_uint4(leafWord[4], leafWord[5], leafWord[6], leafWord[7]);
+}
+
+// The first levels: wide nodes 0 .. nroots-1, whose binary nodes are in the
+// queue, and down from them.
+__global__ void __launch_bounds__(kTopThreads) k_wide_top(WideBuild B, uint32_t nroots) {
+  if (threadIdx.x == 0) B.state[kWideNodes] = nroots;
+  __syncthreads();
+  uint32_t first = 0, end = nroots;
+  while (first < end && end - first < kTopItems) {
+    for (uint32_t w = first + threadIdx.x; w < end; w += kTopThreads) collapse(B, w);
+    __syncthreads();
+    first = end;
+    end = *(volatile uint32_t*)&B.state[kWideNodes];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    B.state[kWideRange] = first;
+    B.state[kWideRange + 1] = end;
+  }
+}
+
+// One level; the last block to finish writes the range of the next.
+__global__ void __launch_bounds__(64) k_wide_level(WideBuild B, int level) {
+  const uint32_t first = B.state[kWideRange + 2 * level], end = B.state[kWideRange + 2 * level + 1];
+  for (uint32_t w = first + blockIdx.x * blockDim.x + threadIdx.x; w < end; w += gridDim.x * blockDim.x) collapse(B, w);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&B.state[kWideDone], 1u) == gridDim.x - 1) {
+    B.state[kWideDone] = 0u;
+    B.state[kWideRange + 2 * (level + 1)] = end;
+    B.state[kWideRange + 2 * (level + 1) + 1] = *(volatile uint32_t*)&B.state[kWideNodes];
+  }
+}
+
+// The rest, each subtree depth first by one thread: the stack holds the
+// children still to do of every node above, one entry per level.
+__global__ void __launch_bounds__(64) k_wide_rest(WideBuild B) {
+  const uint32_t first = B.state[kWideRange + 2 * kLevels], end = B.state[kWideRange + 2 * kLevels + 1];
+  for (uint32_t w = first + blockIdx.x * blockDim.x + threadIdx.x; w < end; w += gridDim.x * blockDim.x) {
+    uint2 stack[R2_BVH_STACK];  // next node, nodes left
+    int sp = 0;
+    stack[sp++] = make_uint2(w, 1u);
+    while (sp > 0) {
+      const uint32_t node = stack[sp - 1].x;
+      ++stack[sp - 1].x;
+      if (--stack[sp - 1].y == 0u) --sp;
+      collapse(B, node);
+      const uint4* n = B.out + kWideWords * (size_t)node;
+      const uint32_t children = (uint32_t)__popc(n[0].w >> 24);
+      if (children) stack[sp++] = make_uint2(n[1].x, children);
+    }
+  }
+}
+
+}  // namespace
+
+void WideBvh::build(const BvhNode* nodes, const float4* tris, const uint32_t* roots, uint32_t nroots, uint32_t nleaves,
+                    cudaStream_t s) {
+  // A node with fewer than eight children has leaves alone: of W nodes with L
+  // leaves below R roots, 7 L / 12 + R bounds W (L / 2 nodes of two leaves, an
+  // inner node per eight nodes).
+  const size_t cap = (size_t)nleaves * 7 / 12 + nroots + 8;
+  nodes_.reserve(cap * kWideWords);
+  queue_.reserve(cap);
+  state_.reserve(kWideState);
+  R2_CUDA(cudaMemsetAsync(state_.get(), 0, kWideState * sizeof(uint32_t), s));
+  if (roots) R2_CUDA(cudaMemcpyAsync(queue_.get(), roots, nroots * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  else R2_CUDA(cudaMemsetAsync(queue_.get(), 0, sizeof(uint32_t), s));
+  const WideBuild B = {nodes, tris, nodes_.get(), queue_.get(), state_.get()};
+  k_wide_top<<<1, kTopThreads, 0, s>>>(B, nroots);
+  const int blocks = sm_count() * 4;
+  for (int level = 0; level < kLevels; ++level) k_wide_level<<<blocks, 64, 0, s>>>(B, level);
+  k_wide_rest<<<blocks, 64, 0, s>>>(B);
+  R2_CUDA(cudaGetLastError());
+}
+
+}  // namespace r2
