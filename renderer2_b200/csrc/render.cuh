@@ -90,7 +90,13 @@ constexpr uint32_t kMaxTopNodes = 256;
 constexpr uint32_t kDefaultTrackSteps = 8;   // tracking steps a lane takes between refills
 constexpr uint32_t kDefaultTravVisits = 32;  // BVH visits between refill checks
 constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a refill
-constexpr uint32_t kDefaultWavePaths = 1u << 22;  // paths per wave a frame's samples are grouped to
+// Paths per wave a frame's samples are grouped to.  A wave's later bounces hold
+// a few per cent of its paths, so larger waves keep the traversals' lanes and
+// the launches full: 64 samples of 1024x1024, 98.3 / 87.3 / 81.5 ms with 4M / 8M /
+// 16M paths (4 GB of state at 16M).  Served jobs share the device and keep
+// waves of kServeWavePaths; a frame whose 16M paths do not fit falls back to them.
+constexpr uint32_t kDefaultWavePaths = 1u << 24;
+constexpr uint32_t kServeWavePaths = 1u << 22;
 constexpr uint32_t kDefaultMediaRounds = 2;       // queued medium-boundary rounds per bounce
 constexpr uint32_t kMaxMediaRounds = 32;
 // Media counters of a bounce (PathState::mc): [3r] segments queued in round r,

@@ -634,15 +634,23 @@ void RenderScene::commit() {
   committed_ = true;
 }
 
+// A quarter of a power of two, so that a wave just above one does not double
+// the state.
 uint32_t RenderContext::capacity_for(uint32_t n) {
   uint64_t c = 1u << 16;
   while (c < n) c <<= 1;
+  for (uint64_t part = c / 8 * 5; part < c; part += c / 8)
+    if (n <= part) {
+      c = part;
+      break;
+    }
   return (uint32_t)std::min<uint64_t>(c, 0x80000000ull);
 }
 
 void RenderContext::ensure(uint32_t n, bool media) {
   n = capacity_for(n);
   if (n > cap_) {
+    cap_ = 0;  // should an allocation fail
     rayO_.alloc(n); rayD_.alloc(n); T_.alloc(n); L_.alloc(n); hit_.alloc(n);
     shO_.alloc(2 * (size_t)n); shD_.alloc(2 * (size_t)n); shPre_.alloc(2 * (size_t)n); shT_.alloc(n);
     q0_.alloc(n); q1_.alloc(n); qh_.alloc(n); qs_.alloc(n); shTr_.alloc(2 * (size_t)n);
@@ -651,6 +659,7 @@ void RenderContext::ensure(uint32_t n, bool media) {
     cap_ = n;
   }
   if (media && n > mediaCap_) {
+    mediaCap_ = 0;
     shX_.alloc(2 * (size_t)n);
     evA_.alloc(n); evB_.alloc(n); evC_.alloc(n); evD_.alloc(n);
     mc_.alloc((size_t)kCountersPerBounce * 64);
@@ -669,6 +678,19 @@ size_t RenderContext::bytes_for(uint32_t n, bool media) {
   // media: records (4 float4 + float2), shadow tmax/medium, round queues and walk state
   if (media) b += (size_t)n * (16 + 48 + 8 + 16 + 16 + 64 + 16 + 32 + 16) + 16 * 64 * 4;
   return b + (size_t)n * 12;  // frame
+}
+
+void RenderContext::release() {
+  cap_ = mediaCap_ = 0;
+  for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &jO_, &jD_,
+                          &swP_})
+    b->release();
+  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &pj_, &rl0_, &rl1_, &sl0_, &sl1_, &cl_}) b->release();
+  shTr_.release();
+  shX_.release();
+  evD_.release();
+  jM_.release();
+  swM_.release();
 }
 
 void RenderContext::fill(PathState* st) const {
@@ -748,8 +770,17 @@ void RenderScene::render(const r2_camera& c, const r2_render_params& p, float* d
   RenderContext& ctx = ctx_;
   if (!s) s = ctx.stream;
   const uint32_t npix = c.width * c.height;
-  const uint32_t S = wave_spp(npix, p.spp);
-  ctx.ensure(npix * S, !media_.empty());
+  uint32_t S = wave_spp(npix, p.spp);
+  const uint32_t small = wave_spp(npix, p.spp, serve_wave_paths());
+  try {
+    ctx.ensure(npix * S, !media_.empty());
+  } catch (const Error& e) {  // not enough memory for large waves
+    if (e.code != R2_ERR_OUT_OF_MEMORY || small == S) throw;
+    cudaGetLastError();
+    ctx.release();
+    S = small;
+    ctx.ensure(npix * S, !media_.empty());
+  }
   RenderLaunch L = make_launch(ctx, c, p, d_frame, S);
   R2_CUDA(cudaMemsetAsync(ctx.bound.get(), 0, sizeof(unsigned int), s));
   const int nblocks = wave_blocks(npix * S);

@@ -39,8 +39,10 @@ class RenderContext {
   RenderContext& operator=(const RenderContext&) = delete;
 
   // Buffers for at least npix paths (media: the tracking-round state too),
-  // grown to a power of two so that renders of varying size reallocate rarely.
+  // grown in steps so that renders of varying size reallocate rarely.
   void ensure(uint32_t npix, bool media);
+  // Gives the path buffers back (after an ensure that ran out of memory).
+  void release();
   void fill(PathState* st) const;
   // Device bytes a render of npix paths needs (buffers as ensure grows them + frame).
   static size_t bytes_for(uint32_t npix, bool media);
@@ -128,6 +130,8 @@ class RenderScene {
   // within the tuning's paths per wave, or maxWavePaths if smaller and nonzero
   // (at least one sample).
   uint32_t wave_spp(uint32_t npix, uint32_t spp, uint32_t maxWavePaths = 0) const;
+  // The cap on served jobs' waves: none when the tuning sets the paths per wave.
+  uint32_t serve_wave_paths() const { return tuning_.wave_paths ? 0u : kServeWavePaths; }
   // Launch tuning (0 fields: the defaults) and the autotuner that sets it.
   void set_tuning(const r2_render_tuning& t);
   r2_render_tuning tuning() const { return tuning_; }

@@ -9,12 +9,6 @@
 
 namespace r2 {
 
-// Paths per wave of a render job: 0 keeps the scene's tuning.  A wave of a
-// few million paths fills the GPU by itself (capping waves at 1M paths so that
-// concurrent jobs would share the GPU made single jobs 1.7x slower), so slots
-// mainly overlap one job's host work and copies with another's kernels.
-constexpr uint32_t kServeWavePaths = 0;
-
 // Bytes of a buffer grown to a power of two (DBuf::reserve_grow).
 static size_t grow_bytes(size_t n) {
   size_t c = 1;
@@ -82,9 +76,10 @@ double Server::now() const {
   return duration<double>(steady_clock::now().time_since_epoch()).count() - t0_;
 }
 
-size_t Server::render_bytes(const RenderScene& scene, const r2_camera& cam, const r2_render_params& rp) {
+size_t Server::render_bytes(const RenderScene& scene, const r2_camera& cam, const r2_render_params& rp,
+                            uint32_t maxWave) {
   const uint32_t npix = cam.width * cam.height;
-  return RenderContext::bytes_for(npix * scene.wave_spp(npix, rp.spp, kServeWavePaths), scene.has_media()) +
+  return RenderContext::bytes_for(npix * scene.wave_spp(npix, rp.spp, maxWave ? maxWave : scene.serve_wave_paths()), scene.has_media()) +
          grow_bytes((size_t)npix * 12);
 }
 
@@ -95,7 +90,10 @@ uint64_t Server::submit(std::unique_ptr<ServerJob> job) {
     const uint32_t npix = j->cam.width * j->cam.height;
     R2_REQUIRE(npix > 0 && j->rp.spp > 0 && j->rp.max_depth > 0 && j->rp.max_depth <= 60, R2_ERR_INVALID_ARGUMENT,
                "bad render job");
-    j->bytes = render_bytes(*j->scene, j->cam, j->rp);
+    // large waves of a tuned scene only where the budget has room for them
+    j->maxWave = j->scene->serve_wave_paths();
+    if (render_bytes(*j->scene, j->cam, j->rp, j->maxWave) > budget_) j->maxWave = kServeWavePaths;
+    j->bytes = render_bytes(*j->scene, j->cam, j->rp, j->maxWave);
     j->outBytes = (size_t)npix * 12;
   } else {
     R2_REQUIRE(j->fscene, R2_ERR_INVALID_ARGUMENT, "filter job needs a filter scene");
@@ -153,7 +151,7 @@ bool Server::start(Slot& s, ServerJob* j) {
     if (j->kind == 0) {
       const uint32_t npix = j->cam.width * j->cam.height;
       s.frame.reserve_grow((size_t)npix * 3);
-      j->scene->render_graph(s.ctx, j->cam, j->rp, s.frame.get(), st, kServeWavePaths);
+      j->scene->render_graph(s.ctx, j->cam, j->rp, s.frame.get(), st, j->maxWave);
       R2_CUDA(cudaMemcpyAsync(s.staging(j->outBytes), s.frame.get(), j->outBytes, cudaMemcpyDeviceToHost, st));
       R2_CUDA(cudaMemcpyAsync(s.pinnedBound, s.ctx.bound.get(), sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     } else {

@@ -35,6 +35,7 @@ struct ServerJob {
   r2_camera cam;
   r2_render_params rp;
   float* rgbOut = nullptr;
+  uint32_t maxWave = 0;    // cap on the paths per wave (0: the tuning's)
   // filter
   FilterScene* fscene = nullptr;
   r2_filter_grid grid;
@@ -54,7 +55,9 @@ class Server {
  public:
   Server(uint32_t slots, uint64_t hbmBudget);
   // Device bytes a render job is admitted with (its slot's wave buffers and frame).
-  static size_t render_bytes(const RenderScene& scene, const r2_camera& cam, const r2_render_params& rp);
+  // maxWave: cap on the paths per wave (0: the one served jobs have by default).
+  static size_t render_bytes(const RenderScene& scene, const r2_camera& cam, const r2_render_params& rp,
+                             uint32_t maxWave = 0);
   ~Server();  // finishes the admitted and queued jobs, then stops
   Server(const Server&) = delete;
   Server& operator=(const Server&) = delete;
