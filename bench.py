@@ -50,8 +50,8 @@ FILTER_BYTES_PER_VOXEL = 36.0
 # hierarchy 1, bottom-up 1, emission 1, shading gather 1
 FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # no measured FP32 figure on this pool
 # media scenes:
-#   extend phase (k_resolve rounds, k_track, k_collide): queue id 4 + ray in/out 64 + throughput in/out 32 + hit record 16 = 116 B per segment
-#   shadow phase (k_shadow_resolve rounds, k_track): record origin 16 + direction 16 + tmax/medium 8 + queue id 4 + transmittance 4 = 48 B per slot
+#   extend phase (k_walk, k_collide): queue id 4 + ray in/out 64 + throughput in/out 32 + hit record 16 = 116 B per segment
+#   shadow phase (k_shadow_surfaces, k_walk): record origin 16 + direction 16 + tmax/medium 8 + queue id 4 + transmittance 4 = 48 B per slot
 #   k_shade<true>: hit 16 + ray 32 + throughput 16 + radiance 16 + 2 records x 64 + continuation 48 = 256 B per segment
 VOLUME_EXTEND_BYTES_PER_SEGMENT = 116.0
 SHADOW_MEDIA_BYTES_PER_SLOT = 48.0

@@ -294,8 +294,8 @@ typedef struct r2_render_tuning {
   uint32_t trav_refill; /* idle lanes of a warp (1..32) at which it ends finished rays and takes new ones */
   uint32_t wave_paths;  /* paths per wave: a wave renders the largest divisor of spp samples of every
                            pixel that keeps width*height*samples within it (at least one sample) */
-  uint32_t media_rounds; /* media: queued rounds of medium boundaries per bounce (1..32) before the
-                            remaining boundaries of a path are walked in one pass */
+  uint32_t media_rounds; /* at most 32; without effect since a path's medium boundaries are walked in
+                            one persistent kernel */
   uint32_t track_blocks; /* media: blocks per SM of the persistent trackers (at most the resident
                             blocks; 0: all of them) */
   uint32_t track_limit; /* media: bound on the steps of one tracking loop (delta / ratio tracking of
@@ -400,8 +400,8 @@ r2_status r2_scene_set_vertices(r2_scene* scene, const float* positions, const f
 /* Renders one frame into device memory d_rgb (width*height*3 floats).
  * stats_out (nullable, 8 doubles): [0] paths, [1] milliseconds of the frame on
  * the stream, [2] path segments traced, [3] shadow rays traced, [4..7]
- * milliseconds of the extend / shade / shadow / accumulate kernels of one
- * (the middle) wave, which renders r2_scene_wave_samples samples of every
+ * milliseconds of the extend / shade / shadow / accumulate kernels (a bounce's
+ * shadow rays overlap the next one's extension) of one (the middle) wave, which renders r2_scene_wave_samples samples of every
  * pixel.  With stats_out the call waits for the frame and returns
  * R2_ERR_DEVICE_TIMEOUT (frame still written) if a loop bound ended any path:
  * 2^20 tracking steps, 64 medium boundaries within a bounce, 256 along a

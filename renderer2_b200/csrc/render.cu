@@ -59,14 +59,17 @@ __device__ __forceinline__ V3 xyz(float4 v) { return v3(v.x, v.y, v.z); }
 // whole launch description to local memory.
 __device__ __forceinline__ uint32_t* pick(uint32_t* const (&a)[2], uint32_t i) { return i ? a[1] : a[0]; }
 __device__ __forceinline__ uint32_t* path_queue(const RenderLaunch& L, uint32_t b) { return pick(L.st.q, b & 1u); }
-// Events of the bounce (surface hits, then medium collisions) and the path of event i.
+// The bounce's event list (surface hits from the front, medium collisions from
+// the back), its events (hits, then collisions) and the path of event i.  Two
+// lists, by turns: a bounce's shadow rays still run while the next is extended.
+__device__ __forceinline__ uint32_t* event_list(const RenderLaunch& L) { return pick(L.st.qe, L.bounce & 1u); }
 __device__ __forceinline__ uint32_t event_count(const RenderLaunch& L) {
   return *(volatile uint32_t*)&L.st.counts[kHitCounters + L.bounce] +
          *(volatile uint32_t*)&L.st.counts[kScatterCounters + L.bounce];
 }
 __device__ __forceinline__ uint32_t event_path(const RenderLaunch& L, uint32_t i) {
   const uint32_t nh = *(volatile uint32_t*)&L.st.counts[kHitCounters + L.bounce];
-  return i < nh ? L.st.qh[i] : L.st.qs[i - nh];
+  return event_list(L)[i < nh ? i : L.wavePaths - 1u - (i - nh)];
 }
 
 // Entry distance of a ray into a BVH node's child box, or INFINITY when the
@@ -162,9 +165,8 @@ __device__ __forceinline__ int media_first(const SceneView& S, V3 o, V3 d, float
 
 // Closest hit over triangles, analytic shapes and (kMedia) medium boxes.
 // Code: >= 0 triangle, -1 miss, -2 - i shape i, kMediumCodeBase - m medium m.
-// scene_closest_after finishes the query from the triangles' result h.
-template <bool kMedia>
-__device__ __forceinline__ float4 scene_closest_after(const SceneView& S, V3 o, V3 d, float tmax, const Hit& h) {
+// surface_closest_after finishes the surface query from the triangles' result h.
+__device__ __forceinline__ float4 surface_closest_after(const SceneView& S, V3 o, V3 d, float tmax, const Hit& h) {
   float t = tmax, b1 = 0.0f, b2 = 0.0f;
   int code = -1;
   if (h.tri >= 0) {
@@ -208,24 +210,24 @@ __device__ __forceinline__ float4 scene_closest_after(const SceneView& S, V3 o, 
       code = -2 - i;
     }
   }
-  if (kMedia && S.nmedia > 0) {
-    float tm;
-    const int m = media_first(S, o, d, tmax, &tm);
-    if (m >= 0 && tm < t) {
-      t = tm;
-      b1 = b2 = 0.0f;
-      code = kMediumCodeBase - m;
-    }
-  }
   return make_float4(t, b1, b2, __int_as_float(code));
 }
 
+// With media the first box boundary is found first and bounds the surface
+// query, which then ends at the next box instead of walking the whole scene
+// (a surface at exactly the boundary's distance still wins, so the bound is the
+// next float): the same hit as both queries over the whole ray.
 template <bool kMedia>
 __device__ __forceinline__ float4 scene_closest(const SceneView& S, V3 o, V3 d, float tmax) {
+  float tm = INFINITY;
+  const int m = kMedia && S.nmedia > 0 ? media_first(S, o, d, tmax, &tm) : -1;
+  if (m >= 0) tmax = fminf(tmax, __uint_as_float(__float_as_uint(tm) + 1u));  // tm >= 0
   Hit h;
   h.tri = -1;
   if (S.hasTris) h = bvh_trace<false>(S.bvh, o, d, tmax);
-  return scene_closest_after<kMedia>(S, o, d, tmax, h);
+  float4 r = surface_closest_after(S, o, d, tmax, h);
+  if (m >= 0 && tm < r.x) r = make_float4(tm, 0.0f, 0.0f, __int_as_float(kMediumCodeBase - m));
+  return r;
 }
 
 // Any surface (triangle or shape) along the ray.
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(RenderLaunch L) {
     __syncthreads();
     if (h[threadIdx.x]) base[threadIdx.x] = atomicAdd(&L.st.sortBins[threadIdx.x], h[threadIdx.x]);
     __syncthreads();
-    if (i < n) L.st.qs[base[key] + rank] = p;
+    if (i < n) event_list(L)[base[key] + rank] = p;  // the list is filled after the sort
     __syncthreads();
   }
 }
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(RenderLaunch L) {
 __global__ void __launch_bounds__(256) k_sort_copy(RenderLaunch L) {
   const uint32_t n = *(volatile uint32_t*)&L.st.counts[L.bounce];
   uint32_t* q = path_queue(L, L.bounce);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) q[i] = L.st.qs[i];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) q[i] = event_list(L)[i];
 }
 
 // Closest hit of every live path (scenes without media).  A path that hits a
@@ -464,7 +466,7 @@ __device__ __forceinline__ void extend_result(const RenderLaunch& L, uint32_t p,
   } else {
     L.st.hit[p] = h;
   }
-  push_queue(L.st.qh, &L.st.counts[kHitCounters + L.bounce], __float_as_int(h.w) != -1, p);
+  push_queue(event_list(L), &L.st.counts[kHitCounters + L.bounce], __float_as_int(h.w) != -1, p);
 }
 
 // One instantiation per traversal variant (no triangles; alpha test, two
@@ -490,7 +492,7 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) 
       return true;
     };
     auto end = [&](uint32_t p, V3 o, V3 d, const Hit& h) {
-      extend_result(L, p, d, scene_closest_after<false>(L.scene, o, d, kDefaultTmax, h));
+      extend_result(L, p, d, surface_closest_after(L.scene, o, d, kDefaultTmax, h));
     };
     trace_scene<false, kAlpha, kInst>(L, n, &L.st.counts[kTravCounters + 2 * L.bounce], begin, end);
   }
@@ -502,14 +504,18 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) 
 // end of the path by a medium rule; material-less medium hits are passed
 // through without counting a bounce (the reference's `--bounces; continue`).
 //
-// Tracking runs apart from the closest-hit work: a resolve round takes a path
-// up to its first segment that needs tracking and queues that segment; the
-// persistent k_track resolves queued segments, refilling a lane as soon as its
-// segment ends, and either ends the path's bounce (collision, dead path) or
-// passes the path to the next round, which continues from the segment's far
-// boundary.  The last round tracks inline.  Every segment draws from its own
-// stream (purpose kPurposeMedium + j, j = medium boundaries met in the bounce)
-// and the steps repeat the loop's operations, so the split changes no result.
+// A persistent kernel (k_walk) gives each lane a path and alternates, warp by
+// warp, between finding the next boundaries (resolve_path, up to the path's
+// first segment that needs tracking) and stepping along the segments; a lane
+// whose path is done takes the next one.  So lanes wait neither for the warp's
+// longest path nor, between segments, for a launch, as they did when rounds of
+// queued segments alternated between two kernels (1,200 trees, delta tracking,
+// 36.4 -> 24.1 ms; a 128^3 crown through its brick grid 9.0 -> 7.5 ms).  In the
+// forest most rounds still run with few lanes: paths are few and differ much
+// in length.  Making the box search resumable too was no faster (26.6 ms), nor
+// were caps on registers for 6 or 8 blocks an SM.  Every segment draws from
+// its own stream (purpose kPurposeMedium + j, j = medium boundaries met in the
+// bounce), so the order of the work changes no result.
 
 // Reserves one slot per calling lane of a warp-aggregated counter.
 __device__ __forceinline__ uint32_t warp_reserve(uint32_t* counter) {
@@ -530,16 +536,27 @@ __device__ __forceinline__ RngStream rng_resume(uint32_t pixel, uint32_t seed, u
   return r;
 }
 
-template <bool kInline>
-__device__ __forceinline__ void resolve_path(const RenderLaunch& L, uint32_t p, bool fresh, uint32_t* jobCounter) {
+// A segment to track: a ray in world space, the medium and the number of its
+// stream (paths: the boundary j, shadow rays: the draw to resume at).
+struct Segment {
+  V3 o, d;
+  float tmax;
+  int med;
+  uint32_t stream;
+};
+
+// Takes path p (fresh: at the start of the bounce; else past the segment that
+// ends at its pending boundary hit) to its next segment that needs tracking
+// (true), or to its event.
+__device__ __forceinline__ bool resolve_path(const RenderLaunch& L, uint32_t p, bool fresh, Segment* out) {
   const SceneView& S = L.scene;
   const float4 ro = L.st.rayO[p], rd = L.st.rayD[p];
   V3 o = xyz(ro), d = xyz(rd);
   int med = __float_as_int(ro.w);
   float tmax = rd.w;
-  V3 T = xyz(L.st.T[p]);
+  const V3 T = xyz(L.st.T[p]);
   int j = 0;
-  if (!fresh) {  // k_track passed the segment that ends at the pending boundary hit
+  if (!fresh) {
     const float4 h = L.st.hit[p];
     const int mi = kMediumCodeBase - __float_as_int(h.w);
     const Ray nr = ray_offset(make_ray(o + d * h.x, normalize(d), kDefaultTmax), d);
@@ -554,9 +571,6 @@ __device__ __forceinline__ void resolve_path(const RenderLaunch& L, uint32_t p, 
   for (; j < kMaxPassThrough; ++j) {
     hr = scene_closest<true>(S, o, d, tmax);
     const int c = __float_as_int(hr.w);
-    MediumEvent ev;
-    ev.hit = 0;
-    int evMed = -1;
     bool dead = false;
     if (c <= kMediumCodeBase) {
       const int mi = kMediumCodeBase - c;
@@ -578,37 +592,18 @@ __device__ __forceinline__ void resolve_path(const RenderLaunch& L, uint32_t p, 
           }
         }
       }
-      if (segMed >= 0) {
-        if (kInline) {
-          RngStream rs = rng_stream(path_pixel(L, p), L.seed, path_sample(L, p), L.bounce,
-                                    kPurposeMedium + (uint32_t)j);
-          T = T * instance_sample(S.media[segMed], seg, L.dda != 0, rs, &ev, &err, (int)L.trackLimit);
-          evMed = segMed;
-          if (err) dead = true;
-        } else {  // queue the segment; the path waits at this boundary hit
-          const uint32_t k = warp_reserve(jobCounter);
-          L.st.jO[k] = f4(seg.o, seg.tmax);
-          L.st.jD[k] = f4(seg.d, __int_as_float(segMed));
-          L.st.jM[k] = make_uint2(p, (uint32_t)j);
-          L.st.rayO[p] = f4(o, __int_as_float(med));
-          L.st.rayD[p] = f4(d, tmax);
-          L.st.hit[p] = hr;
-          L.st.pj[p] = (uint32_t)j;
-          return;
-        }
+      if (segMed >= 0) {  // the path waits at this boundary hit
+        *out = Segment{seg.o, seg.d, seg.tmax, segMed, (uint32_t)j};
+        L.st.rayO[p] = f4(o, __int_as_float(med));
+        L.st.rayD[p] = f4(d, tmax);
+        L.st.hit[p] = hr;
+        L.st.pj[p] = (uint32_t)j;
+        return true;
       }
       if (!dead && (T.x == 0.0f || T.y == 0.0f || T.z == 0.0f)) dead = true;
     }
     if (dead) {
       hr.w = __int_as_float(kEventDead);
-      break;
-    }
-    if (ev.hit) {
-      L.st.evA[p] = f4(ev.pos, ev.ior);
-      L.st.evB[p] = f4(ev.normal, __int_as_float(evMed));
-      L.st.evC[p] = make_float4(ev.S[0], ev.S[1], ev.S[2], ev.S[3]);
-      L.st.evD[p] = make_float2(ev.S[4], ev.S[5]);
-      hr.w = __int_as_float(kEventScatter);
       break;
     }
     if (c <= kMediumCodeBase) {  // material-less hit: continue from it without counting a bounce
@@ -626,39 +621,17 @@ __device__ __forceinline__ void resolve_path(const RenderLaunch& L, uint32_t p, 
   if (err) atomicAdd(L.bound, 1u);
   L.st.rayO[p] = f4(o, __int_as_float(med));
   L.st.rayD[p] = f4(d, tmax);
-  L.st.T[p] = f4(T, 0.0f);
   L.st.hit[p] = hr;
+  return false;
 }
 
-// Round `round` of path extension: round 0 takes the bounce's live paths,
-// later rounds the paths k_track passed; kInline tracks instead of queueing.
-template <bool kFirst, bool kInline>
-__global__ void __launch_bounds__(128) k_resolve(RenderLaunch L, int round) {
-  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce;
-  const uint32_t n = kFirst ? *(volatile uint32_t*)&L.st.counts[L.bounce] : *(volatile uint32_t*)&mc[3 * (round - 1) + 2];
-  const uint32_t* list = kFirst ? path_queue(L, L.bounce) : pick(L.st.rl, (uint32_t)(round - 1) & 1u);
-  uint32_t* jobs = &mc[3 * round];
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) resolve_path<kInline>(L, list[i], kFirst, jobs);
-}
-
-// End of a tracked path segment without a collision: a pass (or an error).
-__device__ __forceinline__ void finish_pass(const RenderLaunch& L, uint32_t p, int st, uint32_t* nextCount,
-                                            uint32_t* nextList) {
+// End of a tracked path segment without a collision; true: the path goes on.
+__device__ __forceinline__ bool finish_pass(const RenderLaunch& L, uint32_t p, int st) {
   const V3 T = xyz(L.st.T[p]);
-  bool dead = false;
-  if (st == kTrackError) {
-    atomicAdd(L.bound, 1u);
-    dead = true;
-  }
-  if (!dead && (T.x == 0.0f || T.y == 0.0f || T.z == 0.0f)) dead = true;
-  if (dead) {
-    float4 h = L.st.hit[p];
-    h.w = __int_as_float(kEventDead);
-    L.st.hit[p] = h;
-  } else {
-    nextList[warp_reserve(nextCount)] = p;
-  }
+  if (st == kTrackError) atomicAdd(L.bound, 1u);
+  if (st != kTrackError && !(T.x == 0.0f || T.y == 0.0f || T.z == 0.0f)) return true;
+  L.st.hit[p].w = __int_as_float(kEventDead);
+  return false;
 }
 
 // A collision: the tracking-space ray and parameter are parked in evA/evB and
@@ -670,7 +643,7 @@ __device__ __forceinline__ void finish_collide(const RenderLaunch& L, uint32_t p
   L.st.cl[warp_reserve(&mc[kCollideCounter])] = p;
 }
 
-// Collision events of the bounce's queued segments (sampleInternal /
+// Collision events of the bounce's segments (sampleInternal /
 // sampleDDA on acceptance), the albedo weight, and the dead-path rule.
 template <bool kDDA>
 __global__ void __launch_bounds__(128) k_collide(RenderLaunch L) {
@@ -698,120 +671,19 @@ __global__ void __launch_bounds__(128) k_collide(RenderLaunch L) {
   }
 }
 
-// End of a tracked shadow segment: the walk's transmittance absorbs it.
-__device__ __forceinline__ void finish_tr(const RenderLaunch& L, uint32_t slot, int st, const TrackState& s,
-                                          uint32_t* nextCount, uint32_t* nextList) {
-  if (st == kTrackError) {
-    atomicAdd(L.bound, 1u);
-    L.st.shTr[slot] = 0.0f;
-    return;
-  }
+// End of a tracked shadow segment: the walk's transmittance absorbs it; true:
+// the walk goes on.
+__device__ __forceinline__ bool finish_tr(const RenderLaunch& L, uint32_t slot, int st, const TrackState& s) {
   const float4 w = L.st.swP[slot];
   const float tr = w.w * s.tr;
-  if (tr == 0.0f) {
+  if (st == kTrackError) atomicAdd(L.bound, 1u);
+  if (st == kTrackError || tr == 0.0f) {
     L.st.shTr[slot] = 0.0f;
-    return;
+    return false;
   }
   L.st.swP[slot] = make_float4(w.x, w.y, w.z, tr);
-  L.st.swM[slot] = make_int2(L.st.swM[slot].x, (int)s.rng.idx);
-  nextList[warp_reserve(nextCount)] = slot;
-}
-
-// Persistent tracking of the queued segments of round `round`: every lane
-// holds one segment, advances it L.trackSteps steps at a time, and takes the
-// next queued segment as soon as its own ends.  With the brick-grid DDA a
-// lane that reaches a tentative collision holds it (pending) while the other
-// lanes keep stepping across majorant cells, and the pending collisions are
-// tested together once they are at least half of the warp's running lanes:
-// the test (Philox draws, indirection and atlas lookups) is the long branch
-// of a step, and divergent tests left most lanes idle.
-template <bool kDDA, bool kSample>
-__global__ void __launch_bounds__(128) k_track(RenderLaunch L, int round) {
-  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce + (kSample ? 0 : kShadowCounters);
-  const uint32_t njobs = *(volatile uint32_t*)&mc[3 * round];
-  uint32_t* taken = &mc[3 * round + 1];
-  uint32_t* nextCount = &mc[3 * round + 2];
-  uint32_t* nextList = kSample ? pick(L.st.rl, (uint32_t)round & 1u) : pick(L.st.sl, (uint32_t)round & 1u);
-  const int lane = threadIdx.x & 31;
-  TrackState s;
-  uint32_t owner = 0;
-  int med = 0;
-  bool active = false, drained = false, pending = false;
-  for (;;) {
-    const bool need = !active && !drained;
-    const unsigned want = __ballot_sync(0xffffffffu, need);
-    if (want) {
-      const int leader = __ffs(want) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(taken, (uint32_t)__popc(want));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (base + (uint32_t)__popc(want) >= njobs) drained = true;  // warp-uniform
-      if (need) {
-        const uint32_t k = base + (uint32_t)__popc(want & ((1u << lane) - 1u));
-        if (k < njobs) {
-          const float4 jo = L.st.jO[k], jd = L.st.jD[k];
-          const uint2 jm = L.st.jM[k];
-          owner = jm.x;
-          med = __float_as_int(jd.w);
-          if (kSample) {
-            s.rng = rng_stream(path_pixel(L, owner), L.seed, path_sample(L, owner), L.bounce, kPurposeMedium + jm.y);
-          } else {
-            const uint32_t op = event_path(L, owner >> 1);
-            s.rng = rng_resume(path_pixel(L, op), L.seed, path_sample(L, op), L.bounce,
-                               kPurposeShadowTr + (owner & 1u), jm.y);
-          }
-          const int st = track_init<kDDA, kSample>(L.scene.media[med], make_ray(xyz(jo), xyz(jd), jo.w), &s,
-                                                     (int)L.trackLimit);
-          if (st == kTrackRunning) {
-            active = true;
-          } else if (kSample) {
-            finish_pass(L, owner, st, nextCount, nextList);
-          } else {
-            finish_tr(L, owner, st, s, nextCount, nextList);
-          }
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, active)) {
-      if (drained) break;
-      continue;
-    }
-    if (kDDA) {
-      for (uint32_t k = 0; k < L.trackSteps; ++k) {
-        if (!__any_sync(0xffffffffu, active)) break;
-        int st = kTrackRunning;
-        if (active && !pending) {
-          st = track_dda_advance<kSample>(L.scene.media[med], s);
-          if (st == kTrackPending) {
-            pending = true;
-            st = kTrackRunning;
-          }
-        }
-        const unsigned held = __ballot_sync(0xffffffffu, pending);
-        const unsigned running = __ballot_sync(0xffffffffu, active && st == kTrackRunning);
-        if (held && 2 * __popc(held) >= __popc(running) && pending) {
-          st = track_dda_collide<kSample>(L.scene.media[med], s);
-          pending = false;
-        }
-        if (active && st != kTrackRunning) {
-          if (kSample && st == kTrackCollide) finish_collide(L, owner, med, s);
-          else if (kSample) finish_pass(L, owner, st, nextCount, nextList);
-          else finish_tr(L, owner, st, s, nextCount, nextList);
-          active = false;
-        }
-      }
-    } else {
-      for (uint32_t k = 0; k < L.trackSteps && active; ++k) {
-        const int st = track_step<kDDA, kSample>(L.scene.media[med], s);
-        if (st != kTrackRunning) {
-          if (kSample && st == kTrackCollide) finish_collide(L, owner, med, s);
-          else if (kSample) finish_pass(L, owner, st, nextCount, nextList);
-          else finish_tr(L, owner, st, s, nextCount, nextList);
-          active = false;
-        }
-      }
-    }
-  }
+  L.st.swM[slot].y = (int)s.rng.idx;
+  return true;
 }
 
 // Surface shading: direct() at a surface and the sampleF continuation
@@ -1036,8 +908,10 @@ __global__ void __launch_bounds__(256) k_events(RenderLaunch L) {
         L.st.L[p] = f4(xyz(L.st.L[p]) + le * xyz(L.st.T[p]), 0.0f);
       }
     }
-    push_queue(L.st.qs, &L.st.counts[kScatterCounters + L.bounce], code == kEventScatter, p);
-    push_queue(L.st.qh, &L.st.counts[kHitCounters + L.bounce], code != -1 && code != kEventDead && code != kEventScatter,
+    if (code == kEventScatter)
+      event_list(L)[L.wavePaths - 1u - warp_reserve(&L.st.counts[kScatterCounters + L.bounce])] = p;
+    __syncwarp();
+    push_queue(event_list(L), &L.st.counts[kHitCounters + L.bounce], code != -1 && code != kEventDead && code != kEventScatter,
                p);
   }
 }
@@ -1085,12 +959,14 @@ __global__ void __launch_bounds__(128, kMedia ? 6 : 8) k_shade(RenderLaunch L) {
 // The first segment of CDeviceScene::intersectTr for a shadow record: the
 // record holds the normal-offset origin o and direction d with the offset
 // ray's length t1, and intersectTr traces CRay::spawnRay(o, o + d * t1).
-__device__ __forceinline__ Ray shadow_ray(float4 o, float4 d) {
+// With media the length is the record's own (shX).
+__device__ __forceinline__ Ray shadow_ray(const RenderLaunch& L, uint32_t j, float4 o, float4 d) {
   const V3 p0 = xyz(o);
-  return spawn_ray(p0, p0 + xyz(d) * d.w);
+  return spawn_ray(p0, p0 + xyz(d) * (L.scene.nmedia > 0 ? L.st.shX[j].x : d.w));
 }
 
-// Visibility of every shadow record of a scene without media.
+// Visibility of every shadow record: 0 behind a surface, else 1 (which k_walk
+// replaces by the transmittance of the media).
 template <bool kTris, bool kAlpha, bool kInst>
 __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderLaunch L) {
   const uint32_t n = event_count(L);
@@ -1101,7 +977,7 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
       const float4 o = L.st.shO[j];
       float tr = 0.0f;
       if (o.w > 0.0f) {
-        const Ray r = shadow_ray(o, L.st.shD[j]);
+        const Ray r = shadow_ray(L, j, o, L.st.shD[j]);
         tr = scene_occluded(L.scene, r.o, r.d, r.tmax) ? 0.0f : 1.0f;
         ++traced;
       }
@@ -1116,7 +992,7 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
         return false;
       }
       ++traced;
-      const Ray r = shadow_ray(o, L.st.shD[j]);
+      const Ray r = shadow_ray(L, j, o, L.st.shD[j]);
       *ro = r.o;
       *rd = r.d;
       *tmax = r.tmax;
@@ -1129,7 +1005,7 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
         noTris.hasTris = 0;
         Hit none;
         none.tri = -1;
-        occluded = __float_as_int(scene_closest_after<false>(noTris, ro, rd, h.t, none).w) != -1;
+        occluded = __float_as_int(surface_closest_after(noTris, ro, rd, h.t, none).w) != -1;
       }
       L.st.shTr[j] = occluded ? 0.0f : 1.0f;
     };
@@ -1146,14 +1022,14 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
 // CDeviceScene::intersectTr as direct() uses it: 0 when the walk ends on a
 // surface (materials do not emit), else the product of the media's
 // ratio-tracking estimates.  A surface anywhere on the ray ends the walk there,
-// so the any-hit test decides that case; without one the walk visits only
-// medium boxes, segment by segment through CRay::spawnRay towards the fixed
-// far point p1, multiplying Tr when a segment leaves the current medium.  As
-// for path extension, segments that need tracking are queued for k_track and
-// the walk resumes after them; the last round tracks inline.  The slot's
-// stream (purpose kPurposeShadowTr + slot parity) continues across segments.
-template <bool kInline>
-__device__ __forceinline__ void shadow_walk(const RenderLaunch& L, uint32_t slot, bool fresh, uint32_t* jobCounter) {
+// so the any-hit test decides that case (k_shadow_surfaces); without one the
+// walk visits only medium boxes, segment by segment through CRay::spawnRay
+// towards the fixed far point p1, multiplying Tr when a segment leaves the
+// current medium.  Takes the slot to its next segment that needs tracking
+// (true) or to its end.  The slot's stream (purpose kPurposeShadowTr + slot
+// parity) continues across segments; *segments counts them.
+__device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot, bool fresh, Segment* out,
+                                            int* segments) {
   const SceneView& S = L.scene;
   const float4 o4 = L.st.shO[slot], d4 = L.st.shD[slot];
   const float2 x = L.st.shX[slot];
@@ -1163,11 +1039,6 @@ __device__ __forceinline__ void shadow_walk(const RenderLaunch& L, uint32_t slot
   float tr;
   uint32_t idx;
   if (fresh) {
-    const Ray r0 = spawn_ray(o, o + d * x.x);
-    if (scene_occluded(S, r0.o, r0.d, r0.tmax)) {
-      L.st.shTr[slot] = 0.0f;
-      return;
-    }
     p0 = o;
     cur = __float_as_int(x.y);
     tr = 1.0f;
@@ -1181,13 +1052,7 @@ __device__ __forceinline__ void shadow_walk(const RenderLaunch& L, uint32_t slot
     idx = (uint32_t)m.y;
   }
   const V3 p1 = o + d * x.x;
-  RngStream rs;
-  if (kInline) {
-    const uint32_t op = event_path(L, slot >> 1);
-    rs = rng_resume(path_pixel(L, op), L.seed, path_sample(L, op), L.bounce, kPurposeShadowTr + (slot & 1u), idx);
-  }
-  int err = 0;
-  for (int k = 0; k < kMaxShadowSegments; ++k) {
+  for (; *segments < kMaxShadowSegments; ++*segments) {
     const V3 off = offset_ray_origin(p0, normalize(p1 - p0));
     const float tl = length(p1 - off);
     const V3 dir = (p1 - p0) / tl;
@@ -1196,54 +1061,131 @@ __device__ __forceinline__ void shadow_walk(const RenderLaunch& L, uint32_t slot
     if (hitM >= 0 && !(best < tl)) hitM = -1;
     if (hitM < 0) {
       L.st.shTr[slot] = tr;
-      if (err) atomicAdd(L.bound, 1u);
-      return;
+      return false;
     }
     if (cur >= 0 && hitM == cur) {
-      if (kInline) {
-        tr *= instance_tr(S.media[cur], make_ray(off, dir, best), L.dda != 0, rs, &err, (int)L.trackLimit);
-      } else {
-        const uint32_t k2 = warp_reserve(jobCounter);
-        L.st.jO[k2] = f4(off, best);
-        L.st.jD[k2] = f4(dir, __int_as_float(cur));
-        L.st.jM[k2] = make_uint2(slot, idx);
-        L.st.swP[slot] = f4(off + dir * best, tr);
-        L.st.swM[slot] = make_int2(-1, (int)idx);
-        return;
-      }
+      *out = Segment{off, dir, best, cur, idx};
+      L.st.swP[slot] = f4(off + dir * best, tr);
+      L.st.swM[slot] = make_int2(-1, (int)idx);
+      ++*segments;
+      return true;
     }
     p0 = off + dir * best;
     cur = cur < 0 ? hitM : -1;
   }
   atomicAdd(L.bound, 1u);
   L.st.shTr[slot] = 0.0f;
+  return false;
 }
 
-template <bool kFirst, bool kInline>
-__global__ void __launch_bounds__(128) k_shadow_resolve(RenderLaunch L, int round) {
-  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce + kShadowCounters;
-  const uint32_t n = kFirst ? 2 * event_count(L) : *(volatile uint32_t*)&mc[3 * (round - 1) + 2];
-  const uint32_t* list = kFirst ? nullptr : pick(L.st.sl, (uint32_t)(round - 1) & 1u);
-  uint32_t* jobs = &mc[3 * round];
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const uint32_t slot = kFirst ? i : list[i];
-    if (kFirst) {
-      const bool traced = L.st.shO[slot].w > 0.0f;
-      if (L.stats) {
-        const unsigned m = __ballot_sync(__activemask(), traced);
-        if ((threadIdx.x & 31) == (unsigned)(__ffs(__activemask()) - 1) && m)
-          atomicAdd(&L.stats[1], (unsigned long long)__popc(m));
-      }
-      if (!traced) {
-        L.st.shTr[slot] = 0.0f;
-        continue;
+// Lanes at a boundary that make a warp look for their next one: the search is
+// long, so it waits for company unless no lane is tracking.
+constexpr int kResolveLanes = 16;
+
+// The bounce's paths (kSample) or shadow rays through the media.  With the
+// brick-grid DDA a lane that reaches a tentative collision holds it (pending)
+// while the other lanes keep stepping across majorant cells, and the pending
+// collisions are tested together once they are at least half of the warp's
+// tracking lanes: the test (Philox draws, indirection and atlas lookups) is the
+// long branch of a step.
+template <bool kDDA, bool kSample>
+__global__ void __launch_bounds__(128) k_walk(RenderLaunch L) {
+  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce;
+  uint32_t* taken = &mc[kSample ? kPathCounter : kShadowCounter];
+  const uint32_t n = kSample ? *(volatile uint32_t*)&L.st.counts[L.bounce] : 2 * event_count(L);
+  const uint32_t* list = path_queue(L, L.bounce);
+  const int lane = threadIdx.x & 31;
+  enum { kIdle, kResolve, kTracking, kEnded };
+  int mode = kIdle;
+  bool fresh = false, drained = false, pending = false;
+  TrackState s;
+  uint32_t owner = 0;
+  int med = 0, segments = 0;
+  // what a tracking status means for the lane
+  const auto after = [&](int st) {
+    if (kSample && st == kTrackCollide) {
+      finish_collide(L, owner, med, s);
+      return (int)kIdle;
+    }
+    fresh = false;
+    return (int)((kSample ? finish_pass(L, owner, st) : finish_tr(L, owner, st, s)) ? kResolve : kIdle);
+  };
+  for (;;) {
+    if (!drained) {
+      const unsigned want = __ballot_sync(0xffffffffu, mode == kIdle);
+      if (want) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(taken, (uint32_t)__popc(want));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base + (uint32_t)__popc(want) >= n) drained = true;  // warp-uniform
+        const uint32_t k = base + (uint32_t)__popc(want & ((1u << lane) - 1u));
+        if (mode == kIdle && k < n) {
+          owner = kSample ? list[k] : k;
+          // shadow records without a ray, or behind a surface, are done
+          if (kSample || L.st.shTr[owner] != 0.0f) {
+            mode = kResolve;
+            fresh = true;
+            segments = 0;
+          }
+        }
       }
     }
-    shadow_walk<kInline>(L, slot, kFirst, jobs);
+    const unsigned resolving = __ballot_sync(0xffffffffu, mode == kResolve);
+    const unsigned tracking = __ballot_sync(0xffffffffu, mode == kTracking);
+    if (!resolving && !tracking) {
+      if (drained) break;
+      continue;
+    }
+    if (!tracking || __popc(resolving) >= kResolveLanes) {
+      if (mode == kResolve) {
+        Segment seg;
+        if (kSample ? resolve_path(L, owner, fresh, &seg) : shadow_walk(L, owner, fresh, &seg, &segments)) {
+          med = seg.med;
+          if (kSample) {
+            s.rng = rng_stream(path_pixel(L, owner), L.seed, path_sample(L, owner), L.bounce, kPurposeMedium + seg.stream);
+          } else {
+            const uint32_t op = event_path(L, owner >> 1);
+            s.rng = rng_resume(path_pixel(L, op), L.seed, path_sample(L, op), L.bounce,
+                               kPurposeShadowTr + (owner & 1u), seg.stream);
+          }
+          const int st = track_init<kDDA, kSample>(L.scene.media[med], make_ray(seg.o, seg.d, seg.tmax), &s,
+                                                   (int)L.trackLimit);
+          mode = st == kTrackRunning ? kTracking : after(st);
+          pending = false;
+        } else {
+          mode = kIdle;
+        }
+      }
+      continue;
+    }
+    int ended = kTrackRunning;
+    for (uint32_t k = 0; k < L.trackSteps; ++k) {
+      if (2 * __popc(__ballot_sync(0xffffffffu, mode == kTracking)) <= __popc(tracking)) break;
+      int st = kTrackRunning;
+      if (kDDA) {
+        if (mode == kTracking && !pending) {
+          st = track_dda_advance<kSample>(L.scene.media[med], s);
+          if (st == kTrackPending) {
+            pending = true;
+            st = kTrackRunning;
+          }
+        }
+        const unsigned held = __ballot_sync(0xffffffffu, pending);
+        const unsigned running = __ballot_sync(0xffffffffu, mode == kTracking && st == kTrackRunning);
+        if (held && 2 * __popc(held) >= __popc(running) && pending) {
+          st = track_dda_collide<kSample>(L.scene.media[med], s);
+          pending = false;
+        }
+      } else if (mode == kTracking) {
+        st = track_step<kDDA, kSample>(L.scene.media[med], s);
+      }
+      if (mode == kTracking && st != kTrackRunning) {
+        mode = kEnded;
+        ended = st;
+      }
+    }
+    if (mode == kEnded) mode = after(ended);  // the ends of a round together
   }
-  if (kFirst && L.stats && blockIdx.x == 0 && threadIdx.x == 0)
-    atomicAdd(&L.stats[0], (unsigned long long)L.st.counts[L.bounce]);
 }
 
 __global__ void __launch_bounds__(256) k_accum(RenderLaunch L) {
@@ -1288,7 +1230,7 @@ int resident_blocks(K kernel, int threads, size_t smem = 0) {
   return std::max(1, n) * sm_count();
 }
 
-int g_trackBlocks[4] = {0, 0, 0, 0};  // resident blocks of k_track<dda, sample>, by dda + 2 sample
+int g_trackBlocks[4] = {0, 0, 0, 0};  // resident blocks of k_walk<dda, sample>, by dda + 2 sample
 
 // The surface traversal kernels by variant: alpha + 2 * two-level; 4: a scene
 // without triangles.
@@ -1328,15 +1270,15 @@ int trav_blocks(int which, int variant) {
 
 void query_track_blocks() {
   if (g_trackBlocks[0] != 0) return;
-  g_trackBlocks[1] = resident_blocks(k_track<true, false>, 128);
-  g_trackBlocks[2] = resident_blocks(k_track<false, true>, 128);
-  g_trackBlocks[3] = resident_blocks(k_track<true, true>, 128);
-  g_trackBlocks[0] = resident_blocks(k_track<false, false>, 128);
+  g_trackBlocks[1] = resident_blocks(k_walk<true, false>, 128);
+  g_trackBlocks[2] = resident_blocks(k_walk<false, true>, 128);
+  g_trackBlocks[3] = resident_blocks(k_walk<true, true>, 128);
+  g_trackBlocks[0] = resident_blocks(k_walk<false, false>, 128);
 }
 
 __global__ void k_advance_sample(uint32_t* sample, uint32_t n) { *sample += n; }
 
-void launch_track(const RenderLaunch& L, bool sample, int round, cudaStream_t s) {
+void launch_walk(const RenderLaunch& L, bool sample, cudaStream_t s) {
   query_track_blocks();
   const int which = (L.dda ? 1 : 0) + (sample ? 2 : 0);
   // all resident blocks, or L.trackBlocks per SM (fewer warps per SM can
@@ -1345,57 +1287,44 @@ void launch_track(const RenderLaunch& L, bool sample, int round, cudaStream_t s)
   for (int i = 0; i < 4; ++i)
     b[i] = L.trackBlocks ? std::max(1, std::min(g_trackBlocks[i], (int)L.trackBlocks * sm_count())) : g_trackBlocks[i];
   switch (which) {
-    case 0: k_track<false, false><<<b[0], 128, 0, s>>>(L, round); break;
-    case 1: k_track<true, false><<<b[1], 128, 0, s>>>(L, round); break;
-    case 2: k_track<false, true><<<b[2], 128, 0, s>>>(L, round); break;
-    default: k_track<true, true><<<b[3], 128, 0, s>>>(L, round); break;
+    case 0: k_walk<false, false><<<b[0], 128, 0, s>>>(L); break;
+    case 1: k_walk<true, false><<<b[1], 128, 0, s>>>(L); break;
+    case 2: k_walk<false, true><<<b[2], 128, 0, s>>>(L); break;
+    default: k_walk<true, true><<<b[3], 128, 0, s>>>(L); break;
   }
 }
 
 }  // namespace
 
-void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, WaveTimer* tm) {
+void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, const WaveSide& side, WaveTimer* tm) {
   RenderLaunch L = L0;
   if (L.trackSteps == 0) L.trackSteps = kDefaultTrackSteps;
   if (L.travVisits == 0) L.travVisits = kDefaultTravVisits;
   if (L.travRefill == 0) L.travRefill = kDefaultTravRefill;
-  if (L.mediaRounds == 0) L.mediaRounds = kDefaultMediaRounds;
-  const int rounds = (int)std::min<uint32_t>(L.mediaRounds, kMaxMediaRounds);
   query_track_blocks();
   const bool media = L.scene.nmedia > 0;
-  int ev = 0;
-  auto mark = [&](int kind) {
+  int ev = 0, last[2] = {-1, -1};
+  // kind: what ran on the stream since its last mark (-1: nothing to time)
+  auto mark = [&](int kind, bool onSide = false) {
     if (!tm) return;
-    R2_CUDA(cudaEventRecord(tm->ev[ev], s));
+    R2_CUDA(cudaEventRecord(tm->ev[ev], onSide ? side.stream : s));
     tm->kind[ev] = kind;
-    ++ev;
+    tm->since[ev] = last[onSide];
+    last[onSide] = ev++;
   };
   R2_CUDA(cudaMemsetAsync(L.st.counts, 0, sizeof(uint32_t) * kCountsSize, s));
   if (media) R2_CUDA(cudaMemsetAsync(L.st.mc, 0, sizeof(uint32_t) * kCountersPerBounce * L.maxDepth, s));
   mark(-1);
   k_camera<<<nblocks, 256, 0, s>>>(L);
   mark(0);
+  const int tv = trav_variant(L);
   for (uint32_t b = 0; b < L.maxDepth; ++b) {
     L.bounce = b;
     if (media) {
-      k_resolve<true, false><<<nblocks * 2, 128, 0, s>>>(L, 0);
-      for (int r = 0; r < rounds; ++r) {
-        launch_track(L, true, r, s);
-        if (r + 1 < rounds) k_resolve<false, false><<<nblocks * 2, 128, 0, s>>>(L, r + 1);
-        else k_resolve<false, true><<<nblocks * 2, 128, 0, s>>>(L, r + 1);
-      }
+      launch_walk(L, true, s);
       if (L.dda) k_collide<true><<<nblocks * 2, 128, 0, s>>>(L);
       else k_collide<false><<<nblocks * 2, 128, 0, s>>>(L);
       k_events<<<nblocks, 256, 0, s>>>(L);
-      mark(1);
-      kShadeVariants[4 + shade_variant(L)]<<<nblocks * 2, 128, 0, s>>>(L);
-      mark(2);
-      k_shadow_resolve<true, false><<<nblocks * 2, 128, 0, s>>>(L, 0);
-      for (int r = 0; r < rounds; ++r) {
-        launch_track(L, false, r, s);
-        if (r + 1 < rounds) k_shadow_resolve<false, false><<<nblocks * 2, 128, 0, s>>>(L, r + 1);
-        else k_shadow_resolve<false, true><<<nblocks * 2, 128, 0, s>>>(L, r + 1);
-      }
     } else {
       if (L.sortRays && b > 0) {
         R2_CUDA(cudaMemsetAsync(L.st.sortBins, 0, 256 * sizeof(uint32_t), s));
@@ -1404,17 +1333,28 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, Wav
         k_sort_scatter<<<nblocks, 256, 0, s>>>(L);
         k_sort_copy<<<nblocks, 256, 0, s>>>(L);
       }
-      const int tv = trav_variant(L);
       kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv)), kTraceWarps * 32, 0, s>>>(L);
-      mark(1);
-      kShadeVariants[shade_variant(L)]<<<nblocks * 2, 128, 0, s>>>(L);
-      mark(2);
-      kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, s>>>(L);
     }
-    mark(3);
-    k_accum<<<nblocks, 256, 0, s>>>(L);
-    mark(4);
+    mark(1);
+    if (b > 0) {  // the last bounce's shadow records are free
+      R2_CUDA(cudaStreamWaitEvent(s, side.join, 0));
+      mark(-1);
+    }
+    kShadeVariants[(media ? 4 : 0) + shade_variant(L)]<<<nblocks * 2, 128, 0, s>>>(L);
+    mark(2);
+    // the bounce's shadow rays beside the next bounce's extension
+    R2_CUDA(cudaEventRecord(side.fork, s));
+    R2_CUDA(cudaStreamWaitEvent(side.stream, side.fork, 0));
+    mark(-1, true);
+    kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, side.stream>>>(L);
+    if (media) launch_walk(L, false, side.stream);
+    mark(3, true);
+    k_accum<<<nblocks, 256, 0, side.stream>>>(L);
+    mark(4, true);
+    R2_CUDA(cudaEventRecord(side.join, side.stream));
   }
+  R2_CUDA(cudaStreamWaitEvent(s, side.join, 0));
+  mark(-1);
   k_finish<<<nblocks, 256, 0, s>>>(L);
   mark(5);
   if (L.sampleDev) k_advance_sample<<<1, 1, 0, s>>>(L.sampleDev, L.waveSpp);

@@ -54,8 +54,8 @@ struct PathState {
   float4* hit;      // t, b1, b2, event code (int bits: >= 0 triangle, -1 miss, -2 - i shape i,
                     // kEventScatter medium collision, kEventDead path ended by a medium rule)
   uint32_t* q[2];   // ping-pong queues of live path ids
-  uint32_t* qh;     // paths of the bounce that hit a surface (k_extend, or k_events with media)
-  uint32_t* qs;     // media: paths of the bounce with a medium collision (k_events); surfaces: ray sort output
+  uint32_t* qe[2];  // event lists of even and odd bounces: paths that hit a surface from the front, paths with
+                    // a medium collision from the back (also the ray sort's output, before they are filled)
   uint32_t* sortBins;  // 256 key counters of the ray sort
   uint32_t* counts; // [bounce] live path count entering the bounce; from kTravCounters on,
                     // per bounce the rays taken by the persistent surface traversals
@@ -71,14 +71,9 @@ struct PathState {
   float4* evB;      // collision normal, medium index (int bits)
   float4* evC;      // SGGX S xx yy zz xy
   float2* evD;      // SGGX S xz yz
-  uint32_t* mc;     // per-bounce counters of the tracking rounds
-  uint32_t* pj;     // per path: medium boundaries met in the bounce when its segment was queued
-  float4* jO;       // queued segments: origin, tmax
-  float4* jD;       //                  direction, medium (int bits)
-  uint2* jM;        //                  owner (path or shadow slot), stream purpose / draw index
-  uint32_t* rl[2];  // paths resumed in the next round (round r writes list r & 1)
-  uint32_t* sl[2];  // shadow slots resumed in the next round
-  uint32_t* cl;     // paths whose queued segment ended in a collision
+  uint32_t* mc;     // per-bounce media counters
+  uint32_t* pj;     // per path: medium boundaries met in the bounce up to the segment it tracks
+  uint32_t* cl;     // paths whose segment ended in a collision
   float4* swP;      // shadow walk: next origin, transmittance so far
   int2* swM;        // shadow walk: current medium, draw index of the slot's stream
 };
@@ -87,7 +82,7 @@ struct PathState {
 constexpr uint32_t kMaxTopNodes = 256;
 // Launch tuning defaults (RenderLaunch::trackSteps, travVisits, travRefill);
 // no result depends on them.
-constexpr uint32_t kDefaultTrackSteps = 8;   // tracking steps a lane takes between refills
+constexpr uint32_t kDefaultTrackSteps = 16;  // tracking steps a lane takes between refills
 constexpr uint32_t kDefaultTravVisits = 32;  // BVH visits between refill checks
 constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a refill
 // Paths per wave a frame's samples are grouped to.  A wave's later bounces hold
@@ -97,14 +92,11 @@ constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a re
 // waves of kServeWavePaths; a frame whose 16M paths do not fit falls back to them.
 constexpr uint32_t kDefaultWavePaths = 1u << 24;
 constexpr uint32_t kServeWavePaths = 1u << 22;
-constexpr uint32_t kDefaultMediaRounds = 2;       // queued medium-boundary rounds per bounce
-constexpr uint32_t kMaxMediaRounds = 32;
-// Media counters of a bounce (PathState::mc): [3r] segments queued in round r,
-// [3r+1] segments taken, [3r+2] entries of list r + 1; path extension from 0,
-// shadow rays from kShadowCounters, then the collision list's entries.
-constexpr int kShadowCounters = 3 * (kMaxMediaRounds + 1);
-constexpr int kCollideCounter = 2 * kShadowCounters;
-constexpr int kCountersPerBounce = (kCollideCounter + 4) & ~3;
+// media_rounds of a tuning, default and largest: accepted, without effect.
+constexpr uint32_t kDefaultMediaRounds = 2, kMaxMediaRounds = 32;
+// Media counters of a bounce (PathState::mc): paths and shadow slots taken by
+// k_walk, entries of the collision list.
+enum { kPathCounter = 0, kShadowCounter = 1, kCollideCounter = 2, kCountersPerBounce = 4 };
 
 // PathState::counts layout: [0, 64) live paths per bounce, then two counters
 // per bounce (extension rays taken, shadow records taken), then the surface
@@ -142,7 +134,6 @@ struct RenderLaunch {
   uint32_t trackSteps;  // tracking steps a lane takes between refills (tuning, >= 1)
   uint32_t travVisits;  // BVH node steps a lane takes between refill checks of the surface kernels (tuning, >= 1)
   uint32_t travRefill;  // finished lanes of a warp that trigger a refill (tuning, 1..32)
-  uint32_t mediaRounds; // queued medium-boundary rounds per bounce (tuning, 1..kMaxMediaRounds)
   uint32_t trackBlocks; // persistent tracker blocks per SM (tuning; 0: every resident block)
   uint32_t trackLimit;  // steps of one tracking loop after which the path ends (1..kMaxTrackingSteps)
   uint32_t sortRays;    // surface scenes: reorder each bounce's rays by a coherence key before k_extend
@@ -150,19 +141,33 @@ struct RenderLaunch {
   unsigned int* bound;        // paths and shadow rays ended by a loop bound (tracking steps, boundaries)
 };
 
-// Optional per-kernel timing of one wave: events recorded after each launch;
-// kind: -1 start, 0 camera, 1 extend, 2 shade, 3 shadow, 4 accum, 5 finish.
+// Optional timing of one wave: events recorded after each stage; kind: -1
+// start, 0 camera, 1 extend, 2 shade, 3 shadow, 4 accum, 5 finish; since: the
+// event the stage's time counts from (the last on its stream).
 struct WaveTimer {
-  static constexpr int kMax = 6 + 4 * 64;
+  static constexpr int events(int depth) { return 6 + 6 * depth; }
+  static constexpr int kMax = 6 + 6 * 64;
+  int made = 0;  // events created
   cudaEvent_t ev[kMax];
-  int kind[kMax];
+  int kind[kMax], since[kMax];
   int n = 0;
 };
 
-// One wave (L.waveSpp consecutive samples of every pixel).  With L.sampleDev
-// the last launch advances the device sample counter by L.waveSpp, so a
-// captured wave replays as the next samples.
-void launch_render_wave(const RenderLaunch& L, int nblocks, cudaStream_t s, WaveTimer* tm = nullptr);
+// The second stream of a wave, on which a bounce's shadow rays are traced and
+// accumulated while the next bounce is extended (the tail of a persistent
+// kernel leaves most of the GPU free), and the events that fork and join it:
+// 1,200 trees 24.1 -> 21.3 ms, moving spheres at 853x480 4.16 -> 3.95 ms.
+struct WaveSide {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
+// One wave (L.waveSpp consecutive samples of every pixel) on s and side, which
+// rejoins s before the wave ends.  With L.sampleDev the last launch advances
+// the device sample counter by L.waveSpp, so a captured wave replays as the
+// next samples.
+void launch_render_wave(const RenderLaunch& L, int nblocks, cudaStream_t s, const WaveSide& side,
+                        WaveTimer* tm = nullptr);
 // Occupancy queries of the persistent kernels, done before any capture.
 void prepare_render_launches();
 

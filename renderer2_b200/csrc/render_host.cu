@@ -94,6 +94,9 @@ void build_env(const float* rgb, int W, int H, EnvHost* e) {
 
 RenderContext::RenderContext() {
   R2_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  R2_CUDA(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking));
+  R2_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
+  R2_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
   R2_CUDA(cudaEventCreate(&ev0));
   R2_CUDA(cudaEventCreate(&ev1));
   bound.alloc(1);
@@ -103,9 +106,15 @@ RenderContext::RenderContext() {
 RenderContext::~RenderContext() {
   if (stream) cudaStreamSynchronize(stream);
   if (timer)
-    for (int i = 0; i < WaveTimer::kMax; ++i) cudaEventDestroy(timer->ev[i]);
+    for (int i = 0; i < timer->made; ++i) cudaEventDestroy(timer->ev[i]);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
+  if (side.fork) cudaEventDestroy(side.fork);
+  if (side.join) cudaEventDestroy(side.join);
+  if (side.stream) {
+    cudaStreamSynchronize(side.stream);
+    cudaStreamDestroy(side.stream);
+  }
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -663,9 +672,7 @@ void RenderContext::ensure(uint32_t n, bool media) {
     shX_.alloc(2 * (size_t)n);
     evA_.alloc(n); evB_.alloc(n); evC_.alloc(n); evD_.alloc(n);
     mc_.alloc((size_t)kCountersPerBounce * 64);
-    pj_.alloc(n); rl0_.alloc(n); rl1_.alloc(n); cl_.alloc(n);
-    sl0_.alloc(2 * (size_t)n); sl1_.alloc(2 * (size_t)n);
-    jO_.alloc(2 * (size_t)n); jD_.alloc(2 * (size_t)n); jM_.alloc(2 * (size_t)n);
+    pj_.alloc(n); cl_.alloc(n);
     swP_.alloc(2 * (size_t)n); swM_.alloc(2 * (size_t)n);
     mediaCap_ = n;
   }
@@ -675,37 +682,32 @@ size_t RenderContext::bytes_for(uint32_t n, bool media) {
   n = capacity_for(n);
   // per path: 5 float4 state + 3 x 2 float4 records + float4 throughput + 4 queue ids + 2 transmittances
   size_t b = (size_t)n * (5 * 16 + 6 * 16 + 16 + 16 + 8) + kCountsSize * 4;
-  // media: records (4 float4 + float2), shadow tmax/medium, round queues and walk state
-  if (media) b += (size_t)n * (16 + 48 + 8 + 16 + 16 + 64 + 16 + 32 + 16) + 16 * 64 * 4;
+  // media: shadow tmax/medium, events (3 float4 + float2), two words and the walk state
+  if (media) b += (size_t)n * (16 + 48 + 8 + 8 + 32 + 16) + 16 * 64 * 4;
   return b + (size_t)n * 12;  // frame
 }
 
 void RenderContext::release() {
   cap_ = mediaCap_ = 0;
-  for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &jO_, &jD_,
-                          &swP_})
+  for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &swP_})
     b->release();
-  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &pj_, &rl0_, &rl1_, &sl0_, &sl1_, &cl_}) b->release();
+  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &pj_, &cl_}) b->release();
   shTr_.release();
   shX_.release();
   evD_.release();
-  jM_.release();
   swM_.release();
 }
 
 void RenderContext::fill(PathState* st) const {
   st->rayO = rayO_.get(); st->rayD = rayD_.get(); st->T = T_.get(); st->L = L_.get(); st->hit = hit_.get();
-  st->q[0] = q0_.get(); st->q[1] = q1_.get(); st->qh = qh_.get(); st->qs = qs_.get(); st->counts = counts_.get();
+  st->q[0] = q0_.get(); st->q[1] = q1_.get(); st->qe[0] = qh_.get(); st->qe[1] = qs_.get(); st->counts = counts_.get();
   st->sortBins = sortBins_.get();
   st->shO = shO_.get(); st->shD = shD_.get(); st->shPre = shPre_.get(); st->shT = shT_.get();
   st->shTr = shTr_.get();
   if (mediaCap_ > 0) {
     st->shX = shX_.get();
     st->evA = evA_.get(); st->evB = evB_.get(); st->evC = evC_.get(); st->evD = evD_.get();
-    st->mc = mc_.get(); st->pj = pj_.get();
-    st->rl[0] = rl0_.get(); st->rl[1] = rl1_.get(); st->cl = cl_.get();
-    st->sl[0] = sl0_.get(); st->sl[1] = sl1_.get();
-    st->jO = jO_.get(); st->jD = jD_.get(); st->jM = jM_.get();
+    st->mc = mc_.get(); st->pj = pj_.get(); st->cl = cl_.get();
     st->swP = swP_.get(); st->swM = swM_.get();
   }
 }
@@ -753,7 +755,6 @@ RenderLaunch RenderScene::make_launch(const RenderContext& ctx, const r2_camera&
   L.trackSteps = tuning_.track_steps;
   L.travVisits = tuning_.trav_visits;
   L.travRefill = tuning_.trav_refill;
-  L.mediaRounds = tuning_.media_rounds;
   L.trackBlocks = tuning_.track_blocks;
   L.trackLimit = tuning_.track_limit ? tuning_.track_limit : (uint32_t)kMaxTrackingSteps;
   L.sortRays = media_.empty() && view_.hasTris && tuning_.sort_rays ? 1u : 0u;
@@ -789,17 +790,16 @@ void RenderScene::render(const r2_camera& c, const r2_render_params& p, float* d
     ctx.statBuf.reserve(2);
     R2_CUDA(cudaMemsetAsync(ctx.statBuf.get(), 0, 2 * sizeof(unsigned long long), s));
     L.stats = ctx.statBuf.get();
-    if (!ctx.timer) {
-      ctx.timer.reset(new WaveTimer());
-      for (int i = 0; i < WaveTimer::kMax; ++i) R2_CUDA(cudaEventCreate(&ctx.timer->ev[i]));
-    }
+    if (!ctx.timer) ctx.timer.reset(new WaveTimer());
+    WaveTimer& t = *ctx.timer;
+    for (; t.made < WaveTimer::events(p.max_depth); ++t.made) R2_CUDA(cudaEventCreate(&t.ev[t.made]));
   }
   R2_CUDA(cudaEventRecord(ctx.ev0, s));
   for (uint32_t smp = 0; smp < p.spp; smp += S) {
     L.sample = smp;
     // the middle wave of a frame is timed kernel by kernel when statistics are requested
     const bool timed = stats && smp <= p.spp / 2 && p.spp / 2 < smp + S;
-    launch_render_wave(L, nblocks, s, timed ? ctx.timer.get() : nullptr);
+    launch_render_wave(L, nblocks, s, ctx.side, timed ? ctx.timer.get() : nullptr);
   }
   R2_CUDA(cudaEventRecord(ctx.ev1, s));
   if (stats) {
@@ -810,10 +810,11 @@ void RenderScene::render(const r2_camera& c, const r2_render_params& p, float* d
     R2_CUDA(cudaMemcpy(cnt, ctx.statBuf.get(), sizeof(cnt), cudaMemcpyDeviceToHost));
     double kms[6] = {0, 0, 0, 0, 0, 0};
     for (int i = 1; i < ctx.timer->n; ++i) {
+      const int k = ctx.timer->kind[i];
+      if (k < 0) continue;
       float d = 0.0f;
-      R2_CUDA(cudaEventElapsedTime(&d, ctx.timer->ev[i - 1], ctx.timer->ev[i]));
-      int k = ctx.timer->kind[i];
-      if (k >= 0 && k < 6) kms[k] += d;
+      R2_CUDA(cudaEventElapsedTime(&d, ctx.timer->ev[ctx.timer->since[i]], ctx.timer->ev[i]));
+      kms[k] += d;
     }
     stats[0] = (double)npix * p.spp;
     stats[1] = ms;
@@ -848,7 +849,7 @@ void RenderScene::render_graph(RenderContext& ctx, const r2_camera& c, const r2_
   } guard{cap};
   R2_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   try {
-    launch_render_wave(L, wave_blocks(npix * S), cap, nullptr);
+    launch_render_wave(L, wave_blocks(npix * S), cap, ctx.side);
   } catch (...) {
     cudaGraph_t g = nullptr;
     cudaStreamEndCapture(cap, &g);
@@ -903,7 +904,7 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
     float best = 1e30f;
     for (int rep = 0; rep < 2; ++rep) {
       R2_CUDA(cudaEventRecord(ctx.ev0, s));
-      launch_render_wave(L, wave_blocks(npix * S), s, nullptr);
+      launch_render_wave(L, wave_blocks(npix * S), s, ctx.side);
       R2_CUDA(cudaEventRecord(ctx.ev1, s));
       R2_CUDA(cudaEventSynchronize(ctx.ev1));
       float ms = 0.0f;
@@ -940,7 +941,6 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
     static const uint32_t refills[] = {4, 8, 12, 24};
     static const uint32_t visits[] = {8, 16, 64, 256};
     static const uint32_t steps[] = {2, 4, 16, 32};
-    static const uint32_t rounds[] = {1, 4, 8, 16};
     static const uint32_t trackBlocks[] = {2, 3, 4, 6};
     static const uint32_t sortRays[] = {1};
     sweep(&r2_render_tuning::wave_paths, wavePaths, 4);
@@ -949,7 +949,6 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
       sweep(&r2_render_tuning::trav_visits, visits, 4);
       sweep(&r2_render_tuning::sort_rays, sortRays, 1);
     } else {
-      sweep(&r2_render_tuning::media_rounds, rounds, 4);
       sweep(&r2_render_tuning::track_steps, steps, 4);
       sweep(&r2_render_tuning::track_blocks, trackBlocks, 4);
     }
@@ -1001,7 +1000,7 @@ RenderBatch::RenderBatch(const std::vector<RenderScene*>& scenes, const std::vec
     for (size_t i = 0; i < n; ++i) {
       cudaStream_t b = ctx_[i]->stream;
       R2_CUDA(cudaStreamWaitEvent(b, evs[n], 0));
-      launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, nullptr);
+      launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, ctx_[i]->side);
       R2_CUDA(cudaEventRecord(evs[i], b));
       R2_CUDA(cudaStreamWaitEvent(cap, evs[i], 0));
     }

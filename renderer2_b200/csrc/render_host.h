@@ -38,7 +38,7 @@ class RenderContext {
   RenderContext(const RenderContext&) = delete;
   RenderContext& operator=(const RenderContext&) = delete;
 
-  // Buffers for at least npix paths (media: the tracking-round state too),
+  // Buffers for at least npix paths (media: the walks' state too),
   // grown in steps so that renders of varying size reallocate rarely.
   void ensure(uint32_t npix, bool media);
   // Gives the path buffers back (after an ensure that ran out of memory).
@@ -51,6 +51,7 @@ class RenderContext {
   uint32_t bound_hits(cudaStream_t s);
 
   cudaStream_t stream = nullptr;
+  WaveSide side;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DBuf<unsigned int> bound;
   DBuf<uint32_t> sampleDev;
@@ -64,9 +65,8 @@ class RenderContext {
   DBuf<float> shTr_;
   DBuf<float2> shX_, evD_;
   DBuf<float4> evA_, evB_, evC_;
-  DBuf<uint32_t> mc_, pj_, rl0_, rl1_, sl0_, sl1_, cl_;
-  DBuf<float4> jO_, jD_, swP_;
-  DBuf<uint2> jM_;
+  DBuf<uint32_t> mc_, pj_, cl_;
+  DBuf<float4> swP_;
   DBuf<int2> swM_;
 };
 
