@@ -310,13 +310,38 @@ int resolve_bvh_method(bool filterScene) {
 
 // Steps 3-7 over primitive boxes whose centroid bounds are in cb_; with
 // d_pos/d_idx the BVH-ordered triangle array is gathered too.
+DBuf<uint8_t> BvhBuilder::take_scratch() {
+  DBuf<uint8_t> mem = std::move(mem_);
+  for (DBuf<float4>* b : {&triLo_, &triHi_, &leafLo_, &leafHi_, &nodeLo_, &nodeHi_, &cLo_[0], &cLo_[1], &cHi_[0], &cHi_[1]})
+    b->release();
+  for (DBuf<int>* b : {&left_, &right_, &first_, &last_, &nodeParent_, &leafParent_, &nodeHeight_, &collapse_, &flags_,
+                       &cRef_[0], &cRef_[1], &nn_, &count_, &leafPos_})
+    b->release();
+  for (DBuf<uint32_t>* b : {&cb_, &sorted_, &sort_.valsAlt, &sort_.hist, &sort_.partials}) b->release();
+  keys_.release();
+  sort_.keysAlt.release();
+  nodeCost_.release();
+  return mem;
+}
+
+void BvhBuilder::reserve(uint32_t n, bool tris) {
+  const bool usePloc = n > 1 && resolve_bvh_method(filterScene_) == kBvhPloc;
+  const size_t ni = n > 1 ? n - 1 : 1, p = usePloc ? n : 0, k = usePloc ? 0 : ni, b = tris ? n : 0;
+  reserve_together(mem_, part(triLo_, b), part(triHi_, b), part(cb_, 6), part(keys_, n), part(sorted_, p),
+                   part(sort_.keysAlt, n), part(sort_.valsAlt, n), part(sort_.hist, RadixSortScratch::hist_size(n)),
+                   part(sort_.partials, RadixSortScratch::partials_size(n)), part(left_, ni), part(right_, ni),
+                   part(first_, ni), part(last_, k), part(nodeParent_, ni), part(leafParent_, n), part(leafLo_, n),
+                   part(leafHi_, n), part(nodeLo_, ni), part(nodeHi_, ni), part(nodeCost_, ni), part(nodeHeight_, ni),
+                   part(collapse_, ni), part(flags_, k), part(cRef_[0], p), part(cRef_[1], p), part(cLo_[0], p),
+                   part(cLo_[1], p), part(cHi_[0], p), part(cHi_[1], p), part(nn_, p), part(count_, usePloc ? ni : 0),
+                   part(leafPos_, p));
+}
+
 void BvhBuilder::from_boxes(const float4* triLo, const float4* triHi, uint32_t ntris, const float* d_pos,
                             const uint32_t* d_idx, DeviceBvh* out, cudaStream_t s) {
   const int n = (int)ntris;
-  keys_.reserve(n);
   out->order.reserve(n);
   const bool usePloc = n > 1 && resolve_bvh_method(filterScene_) == kBvhPloc;
-  if (usePloc) sorted_.reserve(n);
   uint32_t* sorted = usePloc ? sorted_.get() : out->order.get();
   k_morton<<<(n + 255) / 256, 256, 0, s>>>(triLo, triHi, ntris, cb_.get(), keys_.get(), sorted);
   const int sortLaunches = radix_sort_pairs(keys_.get(), sorted, ntris, 63, &sort_, s);
@@ -349,10 +374,6 @@ void BvhBuilder::from_boxes(const float4* triLo, const float4* triHi, uint32_t n
     return;
   }
   const int ni = n - 1;
-  left_.reserve(ni); right_.reserve(ni); first_.reserve(ni); last_.reserve(ni);
-  nodeParent_.reserve(ni); leafParent_.reserve(n);
-  leafLo_.reserve(n); leafHi_.reserve(n); nodeLo_.reserve(ni); nodeHi_.reserve(ni);
-  nodeCost_.reserve(ni); nodeHeight_.reserve(ni); collapse_.reserve(ni); flags_.reserve(ni);
   // parents default to -1 so a malformed hierarchy ends the bottom-up walk
   R2_CUDA(cudaMemsetAsync(nodeParent_.get(), 0xFF, sizeof(int) * ni, s));
   R2_CUDA(cudaMemsetAsync(leafParent_.get(), 0xFF, sizeof(int) * n, s));
@@ -384,9 +405,7 @@ void BvhBuilder::build(const float* d_pos, const uint32_t* d_idx, uint32_t ntris
   R2_REQUIRE(ntris > 0, R2_ERR_INVALID_ARGUMENT, "BVH over zero triangles");
   R2_REQUIRE(ntris < (1u << 26), R2_ERR_UNSUPPORTED, "BVH supports fewer than 2^26 triangles");
   leafMax_ = kLeafMax;
-  triLo_.reserve(ntris);
-  triHi_.reserve(ntris);
-  cb_.reserve(6);
+  reserve(ntris, true);
   k_init_bounds<<<1, 32, 0, s>>>(cb_.get());
   int nb = (int)std::min<uint32_t>((ntris + 255) / 256, (uint32_t)sm_count() * 8);
   k_tri_bounds<<<nb, 256, 0, s>>>(d_pos, d_idx, ntris, triLo_.get(), triHi_.get(), cb_.get());
@@ -400,7 +419,7 @@ void BvhBuilder::build_boxes(const float4* d_lo, const float4* d_hi, uint32_t nb
   R2_REQUIRE(leafMax >= 1 && leafMax <= kLeafMax, R2_ERR_INVALID_ARGUMENT, "leaf size out of range");
   leafMax_ = leafMax;
   R2_REQUIRE(nboxes < (1u << 26), R2_ERR_UNSUPPORTED, "BVH supports fewer than 2^26 boxes");
-  cb_.reserve(6);
+  reserve(nboxes, false);
   k_init_bounds<<<1, 32, 0, s>>>(cb_.get());
   int nb = (int)std::min<uint32_t>((nboxes + 255) / 256, (uint32_t)sm_count() * 8);
   k_box_bounds<<<nb, 256, 0, s>>>(d_lo, d_hi, nboxes, cb_.get());

@@ -62,13 +62,19 @@ class BvhBuilder {
                    int leafMax = kLeafMax);
   // Kernels the last build launched.
   int launches() const { return launches_; }
+  // The scratch, for other use once the builds on it are done; the builder
+  // allocates its own again when it builds again.
+  DBuf<uint8_t> take_scratch();
   // BVHs of filter scenes (their kBvhAuto default differs).
   void set_filter_scene(bool f) { filterScene_ = f; }
 
  private:
   void from_boxes(const float4* lo, const float4* hi, uint32_t n, const float* d_pos, const uint32_t* d_idx,
                   DeviceBvh* out, cudaStream_t s);
+  // Scratch of a build over n primitives (tris: and their boxes), in one allocation.
+  void reserve(uint32_t n, bool tris);
   int ploc(const float4* lo, const float4* hi, int n, DeviceBvh* out, cudaStream_t s);
+  DBuf<uint8_t> mem_;
   DBuf<float4> triLo_, triHi_, leafLo_, leafHi_, nodeLo_, nodeHi_;
   DBuf<float4> cLo_[2], cHi_[2];
   DBuf<uint64_t> keys_;

@@ -427,13 +427,6 @@ BvhBuilder::~BvhBuilder() {
 int BvhBuilder::ploc(const float4* triLo, const float4* triHi, int n, DeviceBvh* out, cudaStream_t s) {
   const int ni = n - 1;
   if (!hostState_) R2_CUDA(cudaMallocHost((void**)&hostState_, sizeof(PlocState)));
-  leafLo_.reserve(n); leafHi_.reserve(n);
-  cRef_[0].reserve(n); cRef_[1].reserve(n);
-  cLo_[0].reserve(n); cLo_[1].reserve(n); cHi_[0].reserve(n); cHi_[1].reserve(n);
-  nn_.reserve(n);
-  left_.reserve(ni); right_.reserve(ni); nodeParent_.reserve(ni); leafParent_.reserve(n);
-  nodeLo_.reserve(ni); nodeHi_.reserve(ni); nodeCost_.reserve(ni); nodeHeight_.reserve(ni);
-  collapse_.reserve(ni); count_.reserve(ni); first_.reserve(ni); leafPos_.reserve(n);
   const int nbMax = (n + kPlocBlock - 1) / kPlocBlock;
   blockCounts_.reserve(nbMax);
   state_.reserve((sizeof(PlocState) + sizeof(int) - 1) / sizeof(int));

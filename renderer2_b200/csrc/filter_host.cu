@@ -73,6 +73,18 @@ static int grid_for(uint32_t n) {
   return (int)std::max<uint32_t>(1u, std::min<uint32_t>((n + 255) / 256, (uint32_t)sm_count() * 16));
 }
 
+// Words of the scene's own work space: the scratch of its BVH build where that
+// has four per voxel; else 24 per voxel up to 16 MiB, so that the lists of a
+// small dense grid fit (the 48^3 grid of 400,000 triangles needs 22 a voxel),
+// then at least two per voxel (a quarter of the output; the 256^3 grid of 1M
+// triangles uses 1.8) up to kMaxWork: larger grids are filtered in parts.
+constexpr size_t kMaxWork = (size_t)1 << 24;
+static size_t work_words(size_t nvox, size_t have) {
+  if (have >= std::min(std::max(4 * nvox, kFilterMinWork), kMaxWork)) return have;
+  const size_t small = std::min<size_t>(24 * nvox, (size_t)1 << 22);
+  return std::min<size_t>(std::max(std::max<size_t>(2 * nvox, small), kFilterMinWork), kMaxWork);
+}
+
 // SAABB::transform (include/intersect/aabb.hpp:9-13): only the min and max
 // corners are transformed.
 void world_aabb(V3 mlo, V3 mhi, const M43& modelToWorld, V3* wlo, V3* whi) {
@@ -94,10 +106,10 @@ FilterScene::FilterScene(const float* positions, uint32_t nverts, const uint32_t
   // model bounds and argument checks on the host; the world-space vertices
   // (the filter traces in world space) and the per-triangle gathers on the device
   V3 lo = v3(INFINITY), hi = v3(-INFINITY);
-  for (uint32_t v = 0; v < nverts; ++v) {
-    const V3 p = v3(positions[3 * v], positions[3 * v + 1], positions[3 * v + 2]);
-    lo = vmin(lo, p);
-    hi = vmax(hi, p);
+  for (uint32_t v = 0; v < nverts; ++v) {  // comparisons, not fminf calls: NaNs are passed over alike
+    const float x = positions[3 * v], y = positions[3 * v + 1], z = positions[3 * v + 2];
+    lo = v3(x < lo.x ? x : lo.x, y < lo.y ? y : lo.y, z < lo.z ? z : lo.z);
+    hi = v3(x > hi.x ? x : hi.x, y > hi.y ? y : hi.y, z > hi.z ? z : hi.z);
   }
   for (size_t i = 0; i < (size_t)3 * ntris; ++i)
     R2_REQUIRE(indices[i] < nverts, R2_ERR_INVALID_ARGUMENT, "triangle index out of range");
@@ -109,18 +121,24 @@ FilterScene::FilterScene(const float* positions, uint32_t nverts, const uint32_t
   modelHi_ = hi;
   world_aabb(lo, hi, modelToWorld_, &worldLo_, &worldHi_);
   ntris_ = ntris;
+  // inputs of the build and the scene's own arrays: one allocation each
+  DBuf<uint8_t> inputs;
   DBuf<float> dmodel, dpos, dnrm;
   DBuf<uint32_t> didx, dmat;
-  dmodel.upload(positions, (size_t)3 * nverts, stream_);
-  dpos.alloc((size_t)3 * nverts);
+  const size_t nv3 = (size_t)3 * nverts, nt3 = (size_t)3 * ntris;
+  reserve_together(inputs, part(dmodel, nv3), part(dpos, nv3), part(dnrm, nv3), part(didx, nt3),
+                   part(dmat, triMaterial ? ntris : 0));
+  reserve_together(store_, part(bvh_.nodes, std::max<size_t>(ntris - 1, 1)), part(bvh_.tris, nt3), part(bvh_.order, ntris),
+                   part(triN_, nt3), part(triMat_, ntris), part(mats_, nmaterials), part(counters_, kFilterCounters));
+  dmodel.upload(positions, nv3, stream_);
   k_world_points<<<grid_for(nverts), 256, 0, stream_>>>(dmodel.get(), nverts, modelToWorld_, dpos.get());
   R2_CUDA(cudaGetLastError());
-  didx.upload(indices, (size_t)3 * ntris, stream_);
-  build_bvh(dpos.get(), didx.get(), ntris, &bvh_, stream_, true);
-  dnrm.upload(normals, (size_t)3 * nverts, stream_);
+  didx.upload(indices, nt3, stream_);
+  BvhBuilder builder;
+  builder.set_filter_scene(true);
+  builder.build(dpos.get(), didx.get(), ntris, &bvh_, stream_);
+  dnrm.upload(normals, nv3, stream_);
   if (triMaterial) dmat.upload(triMaterial, ntris, stream_);
-  triN_.alloc((size_t)3 * ntris);
-  triMat_.alloc(ntris);
   k_order_normals<<<grid_for(ntris), 256, 0, stream_>>>(bvh_.order.get(), didx.get(), dnrm.get(),
                                                         triMaterial ? dmat.get() : nullptr, ntris, triN_.get(),
                                                         triMat_.get());
@@ -156,10 +174,12 @@ FilterScene::FilterScene(const float* positions, uint32_t nverts, const uint32_t
       if (anyAlpha) triAlpha_.upload(triAlpha.data(), triAlpha.size(), stream_);
     }
   }
-  counters_.alloc(kFilterCounters);
   R2_CUDA(cudaEventCreate(&ev0_));
   R2_CUDA(cudaEventCreate(&ev1_));
   R2_CUDA(cudaStreamSynchronize(stream_));
+  workMem_ = builder.take_scratch();
+  if (workMem_.bytes() > sizeof(uint32_t) * kMaxWork) workMem_.release();
+  else work_.view(reinterpret_cast<uint32_t*>(workMem_.get()), workMem_.bytes() / sizeof(uint32_t));
 }
 
 FilterScene::~FilterScene() {
@@ -174,15 +194,6 @@ FilterScene::~FilterScene() {
 r2_filter_grid FilterScene::grid(float voxelSize) const {
   R2_REQUIRE(voxelSize > 0.0f, R2_ERR_INVALID_ARGUMENT, "voxel size must be positive");
   return setup_grid(worldLo_, worldHi_, worldToModel_, voxelSize);
-}
-
-// Words of the scene's own work space: 24 per voxel up to 16 MiB, so that the
-// lists of a small dense grid fit (the 48^3 grid of 400,000 triangles needs 22
-// a voxel), then at least two per voxel (a quarter of the output; the 256^3
-// grid of 1M triangles uses 1.8) up to 64 MiB: larger grids are filtered in parts.
-static size_t work_words(size_t nvox) {
-  const size_t small = std::min<size_t>(24 * nvox, (size_t)1 << 22);
-  return std::min<size_t>(std::max(std::max<size_t>(2 * nvox, small), kFilterMinWork), (size_t)1 << 24);
 }
 
 // Most voxels of a part: at most kCandMax + 1 list words each stay below 2^32.
@@ -250,8 +261,12 @@ void FilterScene::run(const r2_filter_grid& g, const r2_filter_params& p, uint32
   L.counters = d_counters ? d_counters : counters_.get();
   L.ops = d_ops;
   if (!d_work) {
-    workWords = work_words(nvox);
-    work_.reserve(workWords);
+    const size_t words = work_words(nvox, work_.size());
+    if (words > work_.size()) {
+      work_.alloc(words);
+      workMem_.release();
+    }
+    workWords = work_.size();
     d_work = work_.get();
   }
   // half the longest diagonal of a brick's eight voxel centres

@@ -49,6 +49,7 @@ class FilterScene {
   M43 modelToWorld_, worldToModel_;
   V3 modelLo_, modelHi_, worldLo_, worldHi_;
   uint32_t ntris_ = 0;
+  DBuf<uint8_t> store_, workMem_;  // the scene's arrays; the build's scratch, kept as work space
   DeviceBvh bvh_;
   DBuf<float4> triN_;
   DBuf<uint32_t> triMat_;

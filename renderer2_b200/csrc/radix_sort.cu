@@ -185,10 +185,11 @@ uint32_t rs_blocks(uint32_t n) { return (n + kRsTile - 1) / kRsTile; }
 void RadixSortScratch::reserve(uint32_t n) {
   keysAlt.reserve(n);
   valsAlt.reserve(n);
-  const size_t L = (size_t)rs_blocks(n) * kRsBins;
-  hist.reserve(L);
-  partials.reserve((L + kScanPart - 1) / kScanPart);
+  hist.reserve(hist_size(n));
+  partials.reserve(partials_size(n));
 }
+size_t RadixSortScratch::hist_size(uint32_t n) { return (size_t)rs_blocks(n) * kRsBins; }
+size_t RadixSortScratch::partials_size(uint32_t n) { return (hist_size(n) + kScanPart - 1) / kScanPart; }
 
 void exclusive_scan_inplace(uint32_t* data, uint32_t n, DBuf<uint32_t>* partials, cudaStream_t s) {
   if (n == 0) return;

@@ -12,6 +12,9 @@ struct RadixSortScratch {
   DBuf<uint32_t> hist;      // digit-major block histograms, then their exclusive prefix
   DBuf<uint32_t> partials;  // per-partition sums of the prefix pass
   void reserve(uint32_t n);
+  // Elements of hist and partials for n pairs.
+  static size_t hist_size(uint32_t n);
+  static size_t partials_size(uint32_t n);
 };
 
 // data[0..n) becomes its exclusive prefix sum (n <= 2^24; partials: scratch,

@@ -305,15 +305,15 @@ void RenderScene::rebuild(cudaStream_t s) {
   }
   const uint32_t nt = (uint32_t)(hIdx_.size() / 3);
   R2_REQUIRE(nt > 0 && dIdx_.get(), R2_ERR_INVALID_ARGUMENT, "scene has no committed triangles");
+  const size_t nt3 = 3 * (size_t)nt;
+  reserve_together(treeMem_, part(bvh_.nodes, std::max<size_t>(nt - 1, 1)), part(bvh_.tris, nt3), part(bvh_.order, nt),
+                   part(triN_, nt3), part(triMat_, nt), part(triUV_, anyUV_ ? nt3 : 0),
+                   part(triAlpha_, dTriAlphaIn_.get() ? nt : 0));
   builder_.build(dPos_.get(), dIdx_.get(), nt, &bvh_, s);
   bvhNodes_ = bvh_.nnodes;
   bvhHeight_ = bvh_.height;
   wide_.build(bvh_.nodes.get(), bvh_.tris.get(), nullptr, 1, nt, s);
   buildLaunches_ = builder_.launches() + WideBvh::kLaunches + 1;
-  triN_.reserve((size_t)3 * nt);
-  triMat_.reserve(nt);
-  if (anyUV_) triUV_.reserve((size_t)3 * nt);
-  if (dTriAlphaIn_.get()) triAlpha_.reserve(nt);
   k_gather_shading<<<(nt + 255) / 256, 256, 0, s>>>(bvh_.order.get(), nt, dIdx_.get(), dNrm_.get(), dTriMatIn_.get(),
                                                     anyUV_ ? dUV_.get() : nullptr, dTriAlphaIn_.get(), triN_.get(),
                                                     triMat_.get(), anyUV_ ? triUV_.get() : nullptr,
@@ -536,6 +536,8 @@ void RenderScene::commit() {
   if (sceneUV && !anyUV_) hUV_.assign(2 * (hPos_.size() / 3), 0.0f);  // world meshes without coordinates: (0, 0)
   anyAlpha_ = false;
   if (nt > 0) {
+    reserve_together(inputMem_, part(dPos_, hPos_.size()), part(dNrm_, hNrm_.size()), part(dIdx_, hIdx_.size()),
+                     part(dTriMatIn_, hTriMat_.size()), part(dUV_, sceneUV ? hUV_.size() : 0));
     dPos_.upload(hPos_.data(), hPos_.size(), s);
     dNrm_.upload(hNrm_.data(), hNrm_.size(), s);
     dIdx_.upload(hIdx_.data(), hIdx_.size(), s);
@@ -660,20 +662,18 @@ void RenderContext::ensure(uint32_t n, bool media) {
   n = capacity_for(n);
   if (n > cap_) {
     cap_ = 0;  // should an allocation fail
-    rayO_.alloc(n); rayD_.alloc(n); T_.alloc(n); L_.alloc(n); hit_.alloc(n);
-    shO_.alloc(2 * (size_t)n); shD_.alloc(2 * (size_t)n); shPre_.alloc(2 * (size_t)n); shT_.alloc(n);
-    q0_.alloc(n); q1_.alloc(n); qh_.alloc(n); qs_.alloc(n); shTr_.alloc(2 * (size_t)n);
-    counts_.alloc(kCountsSize);
-    sortBins_.alloc(256);
+    const size_t m = n, m2 = 2 * m;
+    reserve_together(mem_, part(rayO_, m), part(rayD_, m), part(T_, m), part(L_, m), part(hit_, m), part(shO_, m2),
+                     part(shD_, m2), part(shPre_, m2), part(shT_, m), part(q0_, m), part(q1_, m), part(qh_, m),
+                     part(qs_, m), part(shTr_, m2), part(counts_, kCountsSize), part(sortBins_, 256));
     cap_ = n;
   }
   if (media && n > mediaCap_) {
     mediaCap_ = 0;
-    shX_.alloc(2 * (size_t)n);
-    evA_.alloc(n); evB_.alloc(n); evC_.alloc(n); evD_.alloc(n);
-    mc_.alloc((size_t)kCountersPerBounce * 64);
-    pj_.alloc(n); cl_.alloc(n);
-    swP_.alloc(2 * (size_t)n); swM_.alloc(2 * (size_t)n);
+    const size_t m = n, m2 = 2 * m;
+    reserve_together(mediaMem_, part(shX_, m2), part(evA_, m), part(evB_, m), part(evC_, m), part(evD_, m),
+                     part(mc_, (size_t)kCountersPerBounce * 64), part(pj_, m), part(cl_, m), part(swP_, m2),
+                     part(swM_, m2));
     mediaCap_ = n;
   }
 }
@@ -691,11 +691,13 @@ void RenderContext::release() {
   cap_ = mediaCap_ = 0;
   for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &swP_})
     b->release();
-  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &pj_, &cl_}) b->release();
+  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &counts_, &sortBins_, &mc_, &pj_, &cl_}) b->release();
   shTr_.release();
   shX_.release();
   evD_.release();
   swM_.release();
+  mem_.release();
+  mediaMem_.release();
 }
 
 void RenderContext::fill(PathState* st) const {

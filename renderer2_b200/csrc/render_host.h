@@ -60,6 +60,7 @@ class RenderContext {
 
  private:
   uint32_t cap_ = 0, mediaCap_ = 0;
+  DBuf<uint8_t> mem_, mediaMem_;  // the path buffers, in one allocation each
   DBuf<float4> rayO_, rayD_, T_, L_, hit_, shO_, shD_, shPre_, shT_;
   DBuf<uint32_t> q0_, q1_, qh_, qs_, counts_, sortBins_;
   DBuf<float> shTr_;
@@ -206,6 +207,7 @@ class RenderScene {
   DBuf<float> dPos_, dNrm_, dUV_;
   DBuf<uint32_t> dIdx_, dTriMatIn_;
   DBuf<int> dTriAlphaIn_;
+  DBuf<uint8_t> inputMem_, treeMem_;  // one allocation for the inputs, one for what a build writes
   DBuf<float4> triN_;
   DBuf<uint32_t> triMat_;
   DBuf<Material> mats_;

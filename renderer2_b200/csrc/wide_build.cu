@@ -213,9 +213,7 @@ void WideBvh::build(const BvhNode* nodes, const float4* tris, const uint32_t* ro
   // leaves below R roots, 7 L / 12 + R bounds W (L / 2 nodes of two leaves, an
   // inner node per eight nodes).
   const size_t cap = (size_t)nleaves * 7 / 12 + nroots + 8;
-  nodes_.reserve(cap * kWideWords);
-  queue_.reserve(cap);
-  state_.reserve(kWideState);
+  reserve_together(mem_, part(nodes_, cap * kWideWords), part(queue_, cap), part(state_, kWideState));
   R2_CUDA(cudaMemsetAsync(state_.get(), 0, kWideState * sizeof(uint32_t), s));
   if (roots) R2_CUDA(cudaMemcpyAsync(queue_.get(), roots, nroots * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   else R2_CUDA(cudaMemsetAsync(queue_.get(), 0, sizeof(uint32_t), s));

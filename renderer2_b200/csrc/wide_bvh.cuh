@@ -59,6 +59,7 @@ class WideBvh {
   static constexpr int kLaunches = 5;  // kernels of a build
 
  private:
+  DBuf<uint8_t> mem_;
   DBuf<uint4> nodes_;
   DBuf<uint32_t> queue_, state_;  // binary node of each wide node; counters
 };
