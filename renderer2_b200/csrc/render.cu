@@ -213,36 +213,30 @@ __device__ __forceinline__ float4 surface_closest_after(const SceneView& S, V3 o
   return make_float4(t, b1, b2, __int_as_float(code));
 }
 
-// With media the first box boundary is found first and bounds the surface
-// query, which then ends at the next box instead of walking the whole scene
-// (a surface at exactly the boundary's distance still wins, so the bound is the
-// next float): the same hit as both queries over the whole ray.
-template <bool kMedia>
-__device__ __forceinline__ float4 scene_closest(const SceneView& S, V3 o, V3 d, float tmax) {
-  float tm = INFINITY;
-  const int m = kMedia && S.nmedia > 0 ? media_first(S, o, d, tmax, &tm) : -1;
-  if (m >= 0) tmax = fminf(tmax, __uint_as_float(__float_as_uint(tm) + 1u));  // tm >= 0
+__device__ __forceinline__ float4 surface_closest(const SceneView& S, V3 o, V3 d, float tmax) {
   Hit h;
   h.tri = -1;
   if (S.hasTris) h = bvh_trace<false>(S.bvh, o, d, tmax);
-  float4 r = surface_closest_after(S, o, d, tmax, h);
-  if (m >= 0 && tm < r.x) r = make_float4(tm, 0.0f, 0.0f, __int_as_float(kMediumCodeBase - m));
-  return r;
+  return surface_closest_after(S, o, d, tmax, h);
 }
 
-// Any surface (triangle or shape) along the ray.
-__device__ __forceinline__ bool scene_occluded(const SceneView& S, V3 o, V3 d, float tmax) {
-  if (S.hasTris) {
-    Hit h = bvh_trace<true>(S.bvh, o, d, tmax);
-    if (h.tri >= 0) return true;
+// With media boxes too.  The first box boundary is found first and bounds the
+// surface query, which then ends at the next box instead of walking the whole
+// scene (a surface at exactly the boundary's distance still wins, so the bound
+// is the next float): the same hit as both queries over the whole ray.
+// surface (nullable): the surface query's result over the whole ray.
+__device__ __forceinline__ float4 scene_closest(const SceneView& S, V3 o, V3 d, float tmax, const float4* surface) {
+  float tm = INFINITY;
+  const int m = media_first(S, o, d, tmax, &tm);
+  float4 r;
+  if (surface) {
+    r = *surface;
+  } else {
+    if (m >= 0) tmax = fminf(tmax, __uint_as_float(__float_as_uint(tm) + 1u));  // tm >= 0
+    r = surface_closest(S, o, d, tmax);
   }
-  if (S.nshapes > 0) {
-    SceneView noTris = S;
-    noTris.hasTris = 0;
-    const float4 r = scene_closest<false>(noTris, o, d, tmax);
-    if (__float_as_int(r.w) != -1) return true;
-  }
-  return false;
+  if (m >= 0 && tm < r.x) r = make_float4(tm, 0.0f, 0.0f, __int_as_float(kMediumCodeBase - m));
+  return r;
 }
 
 __device__ __forceinline__ uint32_t push_queue(uint32_t* q, uint32_t* count, bool pred, uint32_t value) {
@@ -322,6 +316,7 @@ __device__ __noinline__ EnvEval env_le_nc(EnvMap e, V3 d) {
   r.Le = env_le(e, d, &r.pdf);
   return r;
 }
+__device__ __noinline__ V3 env_radiance_nc(EnvMap e, V3 d) { return env_radiance(e, d); }
 __device__ __noinline__ U4 philox_nc(U4 ctr, uint32_t k0, uint32_t k1) { return philox4x32_10(ctr, k0, k1); }
 
 // Phase functions of a medium collision (SGGX, or Henyey-Greenstein for media
@@ -453,20 +448,28 @@ __global__ void __launch_bounds__(256) k_sort_copy(RenderLaunch L) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) q[i] = event_list(L)[i];
 }
 
-// Closest hit of every live path (scenes without media).  A path that hits a
-// surface goes to the bounce's hit queue (shading, shadow rays and
+// Closest surface hit of every live path.  With media it is kept for k_walk, in
+// the path's hit record.  Without, a path that hits a surface goes to the bounce's hit queue (shading, shadow rays and
 // accumulation then run over hits only); a miss ends the path here with the
 // environment term of the first bounce (k_shade's miss rule).
 __device__ __forceinline__ void extend_result(const RenderLaunch& L, uint32_t p, V3 d, float4 h) {
+  if (L.scene.nmedia > 0) {
+    L.st.hit[p] = h;
+    return;
+  }
   if (__float_as_int(h.w) == -1) {
     if (L.bounce == 0) {
-      const V3 le = env_le_nc(L.scene.env, d).Le;
+      const V3 le = env_radiance_nc(L.scene.env, d);
       L.st.L[p] = f4(xyz(L.st.L[p]) + le * xyz(L.st.T[p]), 0.0f);
     }
   } else {
     L.st.hit[p] = h;
   }
   push_queue(event_list(L), &L.st.counts[kHitCounters + L.bounce], __float_as_int(h.w) != -1, p);
+}
+
+__device__ __forceinline__ float extend_tmax(const RenderLaunch& L, uint32_t p) {
+  return L.scene.nmedia > 0 ? L.st.rayD[p].w : kDefaultTmax;
 }
 
 // One instantiation per traversal variant (no triangles; alpha test, two
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) 
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
       const uint32_t p = q[i];
       const V3 d = xyz(L.st.rayD[p]);
-      extend_result(L, p, d, scene_closest<false>(L.scene, xyz(L.st.rayO[p]), d, kDefaultTmax));
+      extend_result(L, p, d, surface_closest(L.scene, xyz(L.st.rayO[p]), d, extend_tmax(L, p)));
     }
   } else {
     auto begin = [&](uint32_t k, V3* o, V3* d, float* tmax, uint32_t* item) {
@@ -488,11 +491,11 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) 
       *item = p;
       *o = xyz(L.st.rayO[p]);
       *d = xyz(L.st.rayD[p]);
-      *tmax = kDefaultTmax;
+      *tmax = extend_tmax(L, p);
       return true;
     };
     auto end = [&](uint32_t p, V3 o, V3 d, const Hit& h) {
-      extend_result(L, p, d, surface_closest_after(L.scene, o, d, kDefaultTmax, h));
+      extend_result(L, p, d, surface_closest_after(L.scene, o, d, extend_tmax(L, p), h));
     };
     trace_scene<false, kAlpha, kInst>(L, n, &L.st.counts[kTravCounters + 2 * L.bounce], begin, end);
   }
@@ -569,7 +572,8 @@ __device__ __forceinline__ bool resolve_path(const RenderLaunch& L, uint32_t p, 
   float4 hr = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(kEventDead));
   int err = 0;
   for (; j < kMaxPassThrough; ++j) {
-    hr = scene_closest<true>(S, o, d, tmax);
+    const float4 first = fresh && j == 0 ? L.st.hit[p] : hr;  // k_extend's
+    hr = scene_closest(S, o, d, tmax, fresh && j == 0 ? &first : nullptr);
     const int c = __float_as_int(hr.w);
     bool dead = false;
     if (c <= kMediumCodeBase) {
@@ -581,7 +585,7 @@ __device__ __forceinline__ bool resolve_path(const RenderLaunch& L, uint32_t p, 
         else segMed = med;
       } else {  // entering: find the far side, track through
         const Ray mr = ray_offset(make_ray(o + d * hr.x, normalize(d), kDefaultTmax), d);
-        const float4 he = scene_closest<true>(S, mr.o, mr.d, mr.tmax);
+        const float4 he = scene_closest(S, mr.o, mr.d, mr.tmax, nullptr);
         const int ce = __float_as_int(he.w);
         if (ce != -1) {
           if (ce <= kMediumCodeBase && kMediumCodeBase - ce != mi) {
@@ -904,7 +908,7 @@ __global__ void __launch_bounds__(256) k_events(RenderLaunch L) {
       p = q[i];
       code = __float_as_int(L.st.hit[p].w);
       if (code == -1 && L.bounce == 0) {
-        const V3 le = env_le_nc(L.scene.env, xyz(L.st.rayD[p])).Le;
+        const V3 le = env_radiance_nc(L.scene.env, xyz(L.st.rayD[p]));
         L.st.L[p] = f4(xyz(L.st.L[p]) + le * xyz(L.st.T[p]), 0.0f);
       }
     }
@@ -940,7 +944,7 @@ __global__ void __launch_bounds__(128, kMedia ? 6 : 8) k_shade(RenderLaunch L) {
       const V3 T = xyz(L.st.T[p]);
       if (code == -1 || code == kEventDead) {
         if (code == -1 && L.bounce == 0) {
-          const V3 le = env_le_nc(L.scene.env, d).Le;
+          const V3 le = env_radiance_nc(L.scene.env, d);
           L.st.L[p] = f4(xyz(L.st.L[p]) + le * T, 0.0f);
         }
         const float4 z = make_float4(0, 0, 0, 0);
@@ -978,7 +982,9 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
       float tr = 0.0f;
       if (o.w > 0.0f) {
         const Ray r = shadow_ray(L, j, o, L.st.shD[j]);
-        tr = scene_occluded(L.scene, r.o, r.d, r.tmax) ? 0.0f : 1.0f;
+        Hit none;
+        none.tri = -1;
+        tr = __float_as_int(surface_closest_after(L.scene, r.o, r.d, r.tmax, none).w) != -1 ? 0.0f : 1.0f;
         ++traced;
       }
       L.st.shTr[j] = tr;
@@ -1001,11 +1007,9 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
     auto end = [&](uint32_t j, V3 ro, V3 rd, const Hit& h) {
       bool occluded = h.tri >= 0;
       if (!occluded && L.scene.nshapes > 0) {
-        SceneView noTris = L.scene;
-        noTris.hasTris = 0;
         Hit none;
         none.tri = -1;
-        occluded = __float_as_int(surface_closest_after(noTris, ro, rd, h.t, none).w) != -1;
+        occluded = __float_as_int(surface_closest_after(L.scene, ro, rd, h.t, none).w) != -1;
       }
       L.st.shTr[j] = occluded ? 0.0f : 1.0f;
     };
@@ -1321,6 +1325,7 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
   for (uint32_t b = 0; b < L.maxDepth; ++b) {
     L.bounce = b;
     if (media) {
+      kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv)), kTraceWarps * 32, 0, s>>>(L);
       launch_walk(L, true, s);
       if (L.dda) k_collide<true><<<nblocks * 2, 128, 0, s>>>(L);
       else k_collide<false><<<nblocks * 2, 128, 0, s>>>(L);

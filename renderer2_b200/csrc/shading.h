@@ -410,12 +410,22 @@ R2_HD float dist2d_pdf(const EnvMap& e, float px, float py) {
   return lower * ((float)ur - ys) + upper * (ys - (float)lr);
 }
 
-// CEnvironmentMap::le (environmentmap.hpp:44-55).
-R2_HD V3 env_le(const EnvMap& e, V3 d, float* pdf) {
-  float theta = acosf(clampf(d.y, -1.0f, 1.0f));
+// CEnvironmentMap::le (environmentmap.hpp:44-55); env_radiance: without the pdf.
+R2_HD void env_coords(V3 d, float* theta, float* x, float* y) {
+  *theta = acosf(clampf(d.y, -1.0f, 1.0f));
   float p = atan2f(d.x, d.z);
   float phi = p < 0.0f ? (float)((double)p + 2.0 * kPiD) : p;
-  float x = (float)((double)phi / (2.0 * kPiD)), y = (float)((double)theta / kPiD);
+  *x = (float)((double)phi / (2.0 * kPiD));
+  *y = (float)((double)*theta / kPiD);
+}
+R2_HD V3 env_radiance(const EnvMap& e, V3 d) {
+  float theta, x, y;
+  env_coords(d, &theta, &x, &y);
+  return env_lookup(e, x, y);
+}
+R2_HD V3 env_le(const EnvMap& e, V3 d, float* pdf) {
+  float theta, x, y;
+  env_coords(d, &theta, &x, &y);
   float st = sinf(theta);
   *pdf = st == 0.0f ? 0.0f : (float)((double)dist2d_pdf(e, x, y) / (2.0 * kPiD * kPiD * (double)st));
   return env_lookup(e, x, y);

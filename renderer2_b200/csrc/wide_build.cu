@@ -58,11 +58,12 @@ __device__ __forceinline__ void frame_axis(float lo, float hi, float* origin, ui
   *exponent = (uint32_t)(e + 127);
   *origin = lo - __uint_as_float(*exponent << 23);
 }
-__device__ __forceinline__ uint32_t plane(float x, float origin, uint32_t exponent, bool upper) {
-  const double q = ((double)x - (double)origin) / (double)__uint_as_float(exponent << 23);
-  const double r = upper ? ceil(q + 0.015625) : floor(q - 0.015625);
-  if (!(r >= 0.0)) return upper && !(r < 0.0) ? 255u : 0u;  // NaN: the whole frame
-  return (uint32_t)fmin(r, 255.0);
+// (x - origin and the scaling are exact or within 2e-5 of a unit.)
+__device__ __forceinline__ uint32_t plane(float x, float origin, float perUnit, bool upper) {
+  const float q = (x - origin) * perUnit;
+  const float r = upper ? ceilf(q + 0.015625f) : floorf(q - 0.015625f);
+  if (!(r >= 0.0f)) return upper && !(r < 0.0f) ? 255u : 0u;  // NaN: the whole frame
+  return (uint32_t)fminf(r, 255.0f);
 }
 
 static_assert(kLeafMax <= 8, "a warp's triangle queue has room for eight of each of 32 leaves");
@@ -92,27 +93,26 @@ __device__ void collapse(const WideBuild& B, uint32_t w) {
   }
   Box all = box[0];
   for (int i = 1; i < n; ++i) all = Box{vmin(all.lo, box[i].lo), vmax(all.hi, box[i].hi)};
-  // children to slots: the pair of child and free slot whose octant fits best, again and again
-  int slotOf[8], childAt[8];
-  for (int k = 0; k < 8; ++k) slotOf[k] = childAt[k] = -1;
+  // children to slots, the largest child first: the free slot whose octant fits its offset best
+  int childAt[8];
+  for (int k = 0; k < 8; ++k) childAt[k] = -1;
+  uint32_t placed = 0;
   for (int round = 0; round < n; ++round) {
-    float best = -INFINITY;
-    int bc = -1, bs = -1;
-    for (int c = 0; c < n; ++c) {
-      if (slotOf[c] >= 0) continue;
-      const V3 off = (box[c].lo + box[c].hi) - (all.lo + all.hi);
-      for (int k = 0; k < 8; ++k) {
-        if (childAt[k] >= 0) continue;
-        const float fit = (k & 1 ? off.x : -off.x) + (k & 2 ? off.y : -off.y) + (k & 4 ? off.z : -off.z);
-        if (bc < 0 || fit > best) {
-          best = fit;
-          bc = c;
-          bs = k;
-        }
+    int c = -1;
+    for (int i = 0; i < n; ++i)
+      if (!(placed >> i & 1u) && (c < 0 || area(box[i]) > area(box[c]))) c = i;
+    placed |= 1u << c;
+    const V3 off = (box[c].lo + box[c].hi) - (all.lo + all.hi);
+    int slot = -1;
+    float best = 0.0f;
+    for (int k = 0; k < 8; ++k) {
+      const float fit = (k & 1 ? off.x : -off.x) + (k & 2 ? off.y : -off.y) + (k & 4 ? off.z : -off.z);
+      if (childAt[k] < 0 && (slot < 0 || fit > best)) {
+        slot = k;
+        best = fit;
       }
     }
-    slotOf[bc] = bs;
-    childAt[bs] = bc;
+    childAt[slot] = c;
   }
   uint32_t inner = 0, leaf = 0;
   for (int k = 0; k < 8; ++k)
@@ -123,6 +123,7 @@ __device__ void collapse(const WideBuild& B, uint32_t w) {
   frame_axis(all.lo.x, all.hi.x, &px, &ex);
   frame_axis(all.lo.y, all.hi.y, &py, &ey);
   frame_axis(all.lo.z, all.hi.z, &pz, &ez);
+  const float ux = __uint_as_float((254u - ex) << 23), uy = __uint_as_float((254u - ey) << 23), uz = __uint_as_float((254u - ez) << 23);
   uint32_t q[6][2] = {};  // lo.x lo.y lo.z hi.x hi.y hi.z of the eight slots
   uint32_t child = firstChild, leafWord[8] = {}, instances = 0;
   for (int k = 0; k < 8; ++k) {
@@ -130,12 +131,12 @@ __device__ void collapse(const WideBuild& B, uint32_t w) {
     if (c < 0) continue;
     const Box& b = box[c];
     const int half = k >> 2, shift = 8 * (k & 3);
-    q[0][half] |= plane(b.lo.x, px, ex, false) << shift;
-    q[1][half] |= plane(b.lo.y, py, ey, false) << shift;
-    q[2][half] |= plane(b.lo.z, pz, ez, false) << shift;
-    q[3][half] |= plane(b.hi.x, px, ex, true) << shift;
-    q[4][half] |= plane(b.hi.y, py, ey, true) << shift;
-    q[5][half] |= plane(b.hi.z, pz, ez, true) << shift;
+    q[0][half] |= plane(b.lo.x, px, ux, false) << shift;
+    q[1][half] |= plane(b.lo.y, py, uy, false) << shift;
+    q[2][half] |= plane(b.lo.z, pz, uz, false) << shift;
+    q[3][half] |= plane(b.hi.x, px, ux, true) << shift;
+    q[4][half] |= plane(b.hi.y, py, uy, true) << shift;
+    q[5][half] |= plane(b.hi.z, pz, uz, true) << shift;
     if (ref[c] >= 0) {
       B.queue[child++] = (uint32_t)ref[c];
     } else {
