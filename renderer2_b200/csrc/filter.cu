@@ -672,6 +672,11 @@ __device__ __forceinline__ void write_record(const FilterLaunch& L, uint32_t vid
 // latency bound, and the extra warps hide more than the few spilled values of
 // the shading tail cost (measured on the 256^3 filter: 96 registers and 5
 // blocks 18.6 M voxels/s, 64 and 8 blocks 21.6 M).
+// Its warps are in different places of the kernel, so instruction fetch counts
+// as much as issue: the loops of one or a few turns (hit lengths, packing,
+// copies, iterations) are kept rolled, where the compiler's four-fold unrolling
+// cost more to fetch than it spared (256^3 filter 102.4 -> 94.9 ms, 24x77x24
+// tree 1.04 -> 1.00 ms, 48^3 of 400,000 triangles 2.09 -> 1.95 ms).
 // kEig: the build with the FP64 eigendecomposition tail (eigen output or
 // projection requested), kTex: with texture and opacity maps; the default
 // build carries none of their code.
@@ -709,6 +714,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
     int ncand, root = 0;
     if (entry.y != kNoList) {
       ncand = L.pool[entry.y];
+#pragma unroll 1
       for (int i = lane; i < ncand; i += 32) myCand[i] = L.pool[entry.y + 1 + i];
     } else {
       const float pad = padded_reach(ray_reach(L), center);  // every sample ray stays within it
@@ -722,6 +728,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
     }
     ++sampled;
     __syncwarp();
+#pragma unroll 1
     for (int i = lane; i < min(ncand, kCandStage); i += 32) {
       const int t = myCand[i];
       const float4 a = __ldg(&L.bvh.tris[3 * t]), b = __ldg(&L.bvh.tris[3 * t + 1]), c = __ldg(&L.bvh.tris[3 * t + 2]);
@@ -743,6 +750,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
     for (int k = 0; k < (kSums - kSumDiffuse) / 2; ++k) plain[k] = zero;
     uint32_t hits = 0;
 
+#pragma unroll 1
     for (uint32_t s = lane; s < L.spv; s += 32) {
       const U4 r0 = philox4x32_10(u4(s, 0u, L.lod, 0u), vid, L.seed);
       const U4 r1 = philox4x32_10(u4(s, 1u, L.lod, 0u), vid, L.seed);
@@ -818,6 +826,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
     // that every iteration of the density fit visits the hits only
     if (L.clip) {
       uint32_t packed = 0;
+#pragma unroll 1
       for (uint32_t base = 0; base < L.spv; base += 32) {
         const uint32_t s = base + lane;
         const float t = s < L.spv ? myTs[s] : -1.0f;
@@ -835,10 +844,12 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
     const float pMesh = (float)hits / (float)L.spv;
     float density = -logf(1.0f - pMesh) / (avgDist * L.sigma_t);
     const float nAlpha = L.alpha / L.sigma_t;
+#pragma unroll 1
     for (uint32_t it = 0; it < L.iters; ++it) {
       float pVol;
       if (L.clip) {
         CSum p = csum0();
+#pragma unroll 1
         for (uint32_t s = lane; s < hits; s += 32) cadd(p, expf(-density * L.sigma_t * myTs[s]));
         p = warp_csum(p);
         pVol = 1.0f - cvalue(p) / (float)hits;
