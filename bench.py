@@ -233,11 +233,7 @@ def filter_workload():
     return mesh, mat, prm, vs
 
 
-def _media_launches(tuning):
-    """Kernel launches per bounce of a media scene: resolve, then per queued round track + resolve (the
-    last one walking the rest), collide, events, shade, and the same rounds for the shadow rays, accum."""
-    r = tuning.get("media_rounds") or 2
-    return 6 + 4 * r
+MEDIA_LAUNCHES = 8  # per bounce of a media scene: extend, walk, collide, events, shade, shadow rays, walk, accum
 
 
 def _input_bytes(desc):
@@ -654,7 +650,7 @@ def bench_filter(args, world, local, grid=None, steps=None, warmup=None, e2e_run
                          "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                          "traffic": tr["bytes_per_unit"] * nvox if tr else None,
                          "kernel_ms": kms, "rays_per_s": rays / (kms / 1e3),
-                         "note": "36 B/voxel algorithmic; bound by issue (triangle tests, density fit) and L2 latency",
+                         "note": "36 B/voxel algorithmic; bound by issue and instruction fetch (triangle tests, Philox, density fit)",
                          "fp32": {"achieved": flops / (kms / 1e3) / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
                                   "frac": flops / (kms / 1e3) / 1e12 / fp32_peak,
                                   "peak_source": "nominal: 148 SMs x 128 FP32 lanes x 2 x 1.965 GHz",
@@ -662,6 +658,7 @@ def bench_filter(args, world, local, grid=None, steps=None, warmup=None, e2e_run
                                   "triangles_tested": n_tris,
                                   "formula": "24 per inner node visited + 30 per triangle tested + 40 per ray"}},
             "e2e": e2e,
+            # a lists and a sampling launch per part of the grid; one part counted
             "gpu_launches": 2 * steps, "_mesh": (mesh, mat, prm, vs), "_gpu_slab": (slab, gpu_slab)}
 
 
@@ -891,8 +888,8 @@ def bench_volume(args, world, local):
            "roofline": roofline, "latency": latency,
            "e2e": {"value": world * paths / (e2e_ms / 1e3), "unit": "paths/s", "h2d_bytes_per_step": int(h2d),
                    "d2h_bytes_per_step": int(npix * 12), "ms_per_step": e2e_ms},
-           # per wave: camera, finish; per bounce: _media_launches
-           "gpu_launches": (prm.spp // S) * (2 + _media_launches(tuning) * prm.max_depth) * args.steps}
+           # per wave: camera, finish; per bounce: MEDIA_LAUNCHES
+           "gpu_launches": (prm.spp // S) * (2 + MEDIA_LAUNCHES * prm.max_depth) * args.steps}
     return out, (desc, cam, prm)
 
 
@@ -996,8 +993,8 @@ def bench_forest(args, world, local, cfg=None, autotune=True):
                                                "kind": "port", "sample": f"{n_cpu} trees"},
                               "placement_s": place_s, "placement_attempts": c["attempts"]},
             "scene_build_ms": build_ms,
-            # per wave: camera, finish; per bounce: _media_launches
-            "gpu_launches": (prm.spp // S) * (2 + _media_launches(tuning) * prm.max_depth) * args.steps}
+            # per wave: camera, finish; per bounce: MEDIA_LAUNCHES
+            "gpu_launches": (prm.spp // S) * (2 + MEDIA_LAUNCHES * prm.max_depth) * args.steps}
 
 
 def bench_volume_batch(args, world, local):
@@ -1124,7 +1121,7 @@ def bench_volume_batch(args, world, local):
                                   f"over {args.steps} steps of {c['spp']} replays",
             "e2e": {"value": world * paths / (e2e_ms / 1e3), "unit": "paths/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(sum(npix) * 12), "ms_per_step": e2e_ms},
-            "gpu_launches": c["spp"] * c["scenes"] * (3 + _media_launches(tuned.as_dict()) * c["depth"]) * args.steps}
+            "gpu_launches": c["spp"] * c["scenes"] * (3 + MEDIA_LAUNCHES * c["depth"]) * args.steps}
 
 
 def serving_jobs(c=SERVE_CFG, seed=11):
