@@ -307,29 +307,20 @@ __device__ __forceinline__ void wide_rays(const BvhView& bvh, const WideView& wi
   bool has = false;   // the lane has a ray
   bool run = false;   // and nodes to visit for it
   int enter = -1;     // two-level: the instance to enter (or, -2, to leave) once its triangles are tested
+  bool queued = false;  // two-level: some may still wait
   bool more = true;   // warp-uniform: the queue may still hold items
   int drained = 0;    // rounds since the queue ran out
   int nl = 0, nt = 0; // warp-uniform: leaves and triangles that wait
   while (true) {
-    const unsigned running = __ballot_sync(0xffffffffu, run);
+    const unsigned running = __ballot_sync(0xffffffffu, run || (kInst && has && enter != -1 && !queued));
     if ((more && 32 - __popc(running) >= refill) || running == 0u || (!more && ++drained >= kWideDrain)) {
       drained = 0;
       if (nl + nt > 0) wide_leaves<kAnyHit, kAlpha>(bvh, wide, w, nl, nt, nl, true, lane);
+      queued = false;
       if (has) r.tmax = __uint_as_float((uint32_t)(w.key[lane] >> 32));
       if (kAnyHit && has && (uint32_t)w.key[lane] != kWideNoHit) run = false;
       if (has && !run) {
-        if (kInst && enter != -1 && !(kAnyHit && (uint32_t)w.key[lane] != kWideNoHit)) {
-          if (enter == -2) {
-            wide_set(r, w, lane, wo, wd, 0, 0u);
-            r.group.y = 0u;
-          } else {
-            const BvhInstance& in = bvh.inst[enter];
-            if (in.identity) wide_set(r, w, lane, wo, wd, in.vdelta, (uint32_t)in.wide);
-            else wide_set(r, w, lane, inst_point(in, wo), inst_vector(in, wd), in.vdelta, (uint32_t)in.wide);
-          }
-          enter = -1;
-          run = true;
-        } else {
+        if (!kInst || enter == -1 || (kAnyHit && (uint32_t)w.key[lane] != kWideNoHit)) {
           const unsigned long long key = w.key[lane];
           Hit h;
           h.t = __uint_as_float((uint32_t)(key >> 32));
@@ -366,6 +357,25 @@ __device__ __forceinline__ void wide_rays(const BvhView& bvh, const WideView& wi
         }
       } else if (want == 0xffffffffu) {
         break;
+      }
+      __syncwarp();
+    }
+    // Rays that enter an instance, or leave one without a leaf in the queue, need
+    // not wait for the queue to be emptied (144 instances of 20,480 triangles
+    // 19.2 -> 18.6 ms, 225 of 320 triangles at 605x252 3.85 -> 3.64 ms; looking
+    // for them sooner, at 4 or 8 such lanes, gained no more).
+    if (kInst) {
+      if (has && enter != -1 && !queued) {
+        if (enter == -2) {
+          wide_set(r, w, lane, wo, wd, 0, 0u);
+          r.group.y = 0u;
+        } else {
+          const BvhInstance& in = bvh.inst[enter];
+          if (in.identity) wide_set(r, w, lane, wo, wd, in.vdelta, (uint32_t)in.wide);
+          else wide_set(r, w, lane, inst_point(in, wo), inst_vector(in, wd), in.vdelta, (uint32_t)in.wide);
+        }
+        enter = -1;
+        run = true;
       }
       __syncwarp();
     }
@@ -428,6 +438,7 @@ __device__ __forceinline__ void wide_rays(const BvhView& bvh, const WideView& wi
         if (leaves) {
           w.leaves[nl + __popc(m & below)] = make_uint2((uint32_t)lane, word + __ffs(leaves) - 1u);
           leaves &= leaves - 1u;
+          queued = true;
         }
         nl += __popc(m);
         if (nl >= 32) {
