@@ -29,22 +29,6 @@ struct WideBuild {
   uint32_t* state;
 };
 
-struct Box {
-  V3 lo, hi;
-};
-__device__ __forceinline__ float area(const Box& b) {
-  const V3 e = b.hi - b.lo;
-  return e.x * e.y + e.y * e.z + e.z * e.x;
-}
-__device__ __forceinline__ void children_of(const BvhNode* nd, Box* b, int* ref) {
-  const float4 b0 = nd->b0, b1 = nd->b1, bz = nd->bz;
-  const int4 ch = nd->ch;
-  b[0] = Box{v3(b0.x, b0.z, bz.x), v3(b0.y, b0.w, bz.y)};
-  b[1] = Box{v3(b1.x, b1.z, bz.z), v3(b1.y, b1.w, bz.w)};
-  ref[0] = ch.x;
-  ref[1] = ch.y;
-}
-
 // One axis of a node's frame: the largest power of two 2^e in whose units the
 // extent is at most 252, and an origin one unit below the box, so that a
 // child's planes and 1/64 unit around them (far more than the traversal's
@@ -69,30 +53,11 @@ __device__ __forceinline__ uint32_t plane(float x, float origin, float perUnit, 
 static_assert(kLeafMax <= 8, "a warp's triangle queue has room for eight of each of 32 leaves");
 
 __device__ void collapse(const WideBuild& B, uint32_t w) {
-  Box box[9];
+  WideBox box[9];
   int ref[9];
-  children_of(&B.nodes[B.queue[w]], box, ref);
-  int n = ref[1] == R2_BVH_NONE ? 1 : 2;
-  while (n < 8) {
-    int open = -1;
-    float largest = -1.0f;
-    for (int i = 0; i < n; ++i)
-      if (ref[i] >= 0 && area(box[i]) > largest) {
-        open = i;
-        largest = area(box[i]);
-      }
-    if (open < 0) break;
-    Box b[2];
-    int r[2];
-    children_of(&B.nodes[ref[open]], b, r);
-    box[open] = b[0];
-    ref[open] = r[0];
-    box[n] = b[1];
-    ref[n] = r[1];
-    if (r[1] != R2_BVH_NONE) ++n;
-  }
-  Box all = box[0];
-  for (int i = 1; i < n; ++i) all = Box{vmin(all.lo, box[i].lo), vmax(all.hi, box[i].hi)};
+  const int n = wide_open(B.nodes, B.queue[w], box, ref);
+  WideBox all = box[0];
+  for (int i = 1; i < n; ++i) all = WideBox{vmin(all.lo, box[i].lo), vmax(all.hi, box[i].hi)};
   // children to slots, the largest child first: the free slot whose octant fits its offset best
   int childAt[8];
   for (int k = 0; k < 8; ++k) childAt[k] = -1;
@@ -100,7 +65,7 @@ __device__ void collapse(const WideBuild& B, uint32_t w) {
   for (int round = 0; round < n; ++round) {
     int c = -1;
     for (int i = 0; i < n; ++i)
-      if (!(placed >> i & 1u) && (c < 0 || area(box[i]) > area(box[c]))) c = i;
+      if (!(placed >> i & 1u) && (c < 0 || wide_area(box[i]) > wide_area(box[c]))) c = i;
     placed |= 1u << c;
     const V3 off = (box[c].lo + box[c].hi) - (all.lo + all.hi);
     int slot = -1;
@@ -129,7 +94,7 @@ __device__ void collapse(const WideBuild& B, uint32_t w) {
   for (int k = 0; k < 8; ++k) {
     const int c = childAt[k];
     if (c < 0) continue;
-    const Box& b = box[c];
+    const WideBox& b = box[c];
     const int half = k >> 2, shift = 8 * (k & 3);
     q[0][half] |= plane(b.lo.x, px, ux, false) << shift;
     q[1][half] |= plane(b.lo.y, py, uy, false) << shift;
@@ -210,10 +175,7 @@ __global__ void __launch_bounds__(64) k_wide_rest(WideBuild B) {
 
 void WideBvh::build(const BvhNode* nodes, const float4* tris, const uint32_t* roots, uint32_t nroots, uint32_t nleaves,
                     cudaStream_t s) {
-  // A node with fewer than eight children has leaves alone: of W nodes with L
-  // leaves below R roots, 7 L / 12 + R bounds W (L / 2 nodes of two leaves, an
-  // inner node per eight nodes).
-  const size_t cap = (size_t)nleaves * 7 / 12 + nroots + 8;
+  const size_t cap = wide_capacity(nleaves, nroots);
   reserve_together(mem_, part(nodes_, cap * kWideWords), part(queue_, cap), part(state_, kWideState));
   R2_CUDA(cudaMemsetAsync(state_.get(), 0, kWideState * sizeof(uint32_t), s));
   if (roots) R2_CUDA(cudaMemcpyAsync(queue_.get(), roots, nroots * sizeof(uint32_t), cudaMemcpyHostToDevice, s));

@@ -47,6 +47,56 @@ struct WideView {
   const uint4* nodes;
 };
 
+struct WideBox {
+  V3 lo, hi;
+};
+R2_HD float wide_area(const WideBox& b) {
+  const V3 e = b.hi - b.lo;
+  return e.x * e.y + e.y * e.z + e.z * e.x;
+}
+R2_HD void wide_children_of(const BvhNode* nd, WideBox* b, int* ref) {
+  const float4 b0 = nd->b0, b1 = nd->b1, bz = nd->bz;
+  const int4 ch = nd->ch;
+  b[0] = WideBox{v3(b0.x, b0.z, bz.x), v3(b0.y, b0.w, bz.y)};
+  b[1] = WideBox{v3(b1.x, b1.z, bz.z), v3(b1.y, b1.w, bz.w)};
+  ref[0] = ch.x;
+  ref[1] = ch.y;
+}
+
+// The children of the wide node over binary node `node`: box[0 .. n-1] and
+// ref[0 .. n-1] (room for nine each), n returned.  The inner child of largest
+// area is opened until there are eight or none is left; of areas that are not
+// numbers any is, so that the capacity below holds for every tree.
+R2_HD int wide_open(const BvhNode* nodes, uint32_t node, WideBox* box, int* ref) {
+  wide_children_of(&nodes[node], box, ref);
+  int n = ref[1] == R2_BVH_NONE ? 1 : 2;
+  while (n < 8) {
+    int open = -1;
+    float largest = 0.0f;
+    for (int i = 0; i < n; ++i)
+      if (ref[i] >= 0 && (open < 0 || wide_area(box[i]) > largest)) {
+        open = i;
+        largest = wide_area(box[i]);
+      }
+    if (open < 0) break;
+    WideBox b[2];
+    int r[2];
+    wide_children_of(&nodes[ref[open]], b, r);
+    box[open] = b[0];
+    ref[open] = r[0];
+    box[n] = b[1];
+    ref[n] = r[1];
+    if (r[1] != R2_BVH_NONE) ++n;
+  }
+  return n;
+}
+
+// Wide nodes that trees of nleaves leaves in all below nroots roots can take.
+// A node with fewer than eight children has leaves alone: of W nodes with L
+// leaves below R roots, 7 L / 12 + R bounds W (L / 2 nodes of two leaves, an
+// inner node per eight nodes).
+R2_HD size_t wide_capacity(uint32_t nleaves, uint32_t nroots) { return (size_t)nleaves * 7 / 12 + nroots + 8; }
+
 // Collapses binary BVHs into wide ones, keeping its buffers between builds.
 class WideBvh {
  public:

@@ -1,0 +1,140 @@
+// What the tests of the eight-wide BVH call below the library's C interface:
+// the collapse's choice of children over a host-built binary tree (no GPU), and
+// the closest hits of given rays through the wide tree and through the binary
+// one over the same build.  Compiled and loaded by wide_probe.py.
+#include <cstring>
+#include <vector>
+
+#include "bvh_build.cuh"
+#include "wide_bvh.cuh"
+
+using namespace r2;
+
+namespace {
+
+struct HostTree {
+  std::vector<BvhNode> nodes;
+  const float* boxes;  // 6 floats a leaf: lo, hi
+  uint32_t state;
+
+  uint32_t random() { return state = state * 1664525u + 1013904223u; }
+  // The subtree over leaves first .. first + n - 1; box: its bounds (fminf and fmaxf of its leaves', as the builders').
+  int add(uint32_t first, uint32_t n, int skew, WideBox* box) {
+    if (n == 1) {
+      const float* b = boxes + 6 * (size_t)first;
+      *box = WideBox{v3(b[0], b[1], b[2]), v3(b[3], b[4], b[5])};
+      return bvh_leaf_ref((int)first, 1);
+    }
+    const uint32_t left = skew == 0 ? n / 2 : 1 + (random() >> 8) % (n - 1);
+    const int me = (int)nodes.size();
+    nodes.push_back(BvhNode());
+    WideBox b[2];
+    const int l = add(first, left, skew, &b[0]), r = add(first + left, n - left, skew, &b[1]);
+    BvhNode& nd = nodes[me];
+    nd.b0 = make_float4(b[0].lo.x, b[0].hi.x, b[0].lo.y, b[0].hi.y);
+    nd.b1 = make_float4(b[1].lo.x, b[1].hi.x, b[1].lo.y, b[1].hi.y);
+    nd.bz = make_float4(b[0].lo.z, b[0].hi.z, b[1].lo.z, b[1].hi.z);
+    nd.ch = make_int4(l, r, 0, 0);
+    *box = WideBox{vmin(b[0].lo, b[1].lo), vmax(b[0].hi, b[1].hi)};
+    return me;
+  }
+};
+
+struct Ray {
+  float o[3], d[3], tmax;
+};
+
+__global__ void k_wide(BvhView bvh, WideView wide, const Ray* rays, uint32_t n, uint32_t* taken, unsigned int* bound,
+                       float4* closest, int* any) {
+  __shared__ WideWarp warps[4];
+  auto begin = [&](uint32_t k, V3* o, V3* d, float* tmax, uint32_t* item) {
+    *item = k;
+    *o = v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]);
+    *d = v3(rays[k].d[0], rays[k].d[1], rays[k].d[2]);
+    *tmax = rays[k].tmax;
+    return true;
+  };
+  auto put = [&](uint32_t k, V3, V3, const Hit& h) {
+    closest[k] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.tri));
+  };
+  auto seen = [&](uint32_t k, V3, V3, const Hit& h) { any[k] = h.tri >= 0; };
+  wide_rays<false, false, false>(bvh, wide, warps[threadIdx.x >> 5], n, &taken[0], 32, 16, bound, begin, put);
+  __syncwarp();
+  wide_rays<true, false, false>(bvh, wide, warps[threadIdx.x >> 5], n, &taken[1], 32, 16, bound, begin, seen);
+}
+
+__global__ void k_binary(BvhView bvh, const Ray* rays, uint32_t n, float4* closest) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const Hit h = bvh_trace<false>(bvh, v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]),
+                                   v3(rays[k].d[0], rays[k].d[1], rays[k].d[2]), rays[k].tmax);
+    closest[k] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.tri));
+  }
+}
+
+}  // namespace
+
+extern "C" {
+
+// Wide nodes of the collapse of a binary tree over the leaf boxes (skew: 0 halves, 1 splits anywhere); *capacity: what
+// the builder has room for.
+uint64_t probe_wide_nodes(const float* boxes, uint32_t nleaves, int skew, uint32_t seed, uint64_t* capacity) {
+  HostTree t;
+  t.boxes = boxes;
+  t.state = seed;
+  WideBox all;
+  t.add(0, nleaves, skew, &all);
+  *capacity = wide_capacity(nleaves, 1);
+  uint64_t count = 0;
+  std::vector<uint32_t> todo(1, 0u);
+  while (!todo.empty()) {
+    const uint32_t node = todo.back();
+    todo.pop_back();
+    ++count;
+    WideBox box[9];
+    int ref[9];
+    const int n = wide_open(t.nodes.data(), node, box, ref);
+    for (int i = 0; i < n; ++i)
+      if (ref[i] >= 0) todo.push_back((uint32_t)ref[i]);
+  }
+  return count;
+}
+
+// Closest hits (t, b1, b2, BVH-order triangle as int bits, t free without a hit) of n rays through the wide tree and
+// through the binary one, and whether the wide any-hit query sees one.  0 on success.
+int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t ntris, const float* rays, uint32_t n,
+                float* wideHits, float* binaryHits, int* any) {
+  try {
+    cudaStream_t s = nullptr;
+    DBuf<float> dpos;
+    DBuf<uint32_t> didx, taken(2);
+    DBuf<unsigned int> bound(1);
+    DBuf<Ray> drays;
+    DBuf<float4> a(n), b(n);
+    DBuf<int> dany(n);
+    dpos.upload(pos, 3 * (size_t)nverts, s);
+    didx.upload(idx, 3 * (size_t)ntris, s);
+    drays.upload(reinterpret_cast<const Ray*>(rays), n, s);
+    BvhBuilder builder;
+    DeviceBvh bvh;
+    builder.build(dpos.get(), didx.get(), ntris, &bvh, s);
+    WideBvh wide;
+    wide.build(bvh.nodes.get(), bvh.tris.get(), nullptr, 1, ntris, s);
+    R2_CUDA(cudaMemsetAsync(taken.get(), 0, 2 * sizeof(uint32_t), s));
+    R2_CUDA(cudaMemsetAsync(bound.get(), 0, sizeof(unsigned int), s));
+    k_wide<<<sm_count() * 4, 128, 0, s>>>(bvh.view(), wide.view(), drays.get(), n, taken.get(), bound.get(), a.get(),
+                                          dany.get());
+    k_binary<<<sm_count() * 8, 128, 0, s>>>(bvh.view(), drays.get(), n, b.get());
+    R2_CUDA(cudaGetLastError());
+    unsigned int ended = 0;
+    a.download(reinterpret_cast<float4*>(wideHits), n, s);
+    b.download(reinterpret_cast<float4*>(binaryHits), n, s);
+    dany.download(any, n, s);
+    bound.download(&ended, 1, s);
+    R2_CUDA(cudaStreamSynchronize(s));
+    return ended ? 1 : 0;
+  } catch (const Error& e) {
+    return 2;
+  }
+}
+
+}  // extern "C"
