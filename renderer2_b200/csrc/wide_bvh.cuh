@@ -180,10 +180,13 @@ __device__ __forceinline__ void wide_planes(float nearQ, float farQ, unsigned lo
   asm("mov.b64 {%0, %1}, %2;" : "=f"(*tn), "=f"(*tf) : "l"(q));
 }
 // The axis's scale and base: t = byte * 2^e / d + (origin - o) / d, for bytes
-// read as 2^23 + 256 * byte.
+// read as 2^23 + 256 * byte.  The scale is taken down from 2^23 times itself, so
+// that it is infinite where that product would be (a direction almost along
+// another axis): both planes are then no numbers and the axis culls nothing,
+// where an infinite base alone would put every child at the same infinity.
 __device__ __forceinline__ void wide_axis(float origin, float o, float invd, uint32_t exponent, unsigned long long* scale,
                                           unsigned long long* base) {
-  const float s = __uint_as_float(exponent << 23) * (1.0f / 256.0f) * invd;
+  const float s = __uint_as_float(exponent << 23) * 32768.0f * invd * (1.0f / 8388608.0f);
   const float b = fmaf(-8388608.0f, s, (origin - o) * invd);
   asm("mov.b64 %0, {%1, %1};" : "=l"(*scale) : "f"(s));
   asm("mov.b64 %0, {%1, %1};" : "=l"(*base) : "f"(b));
@@ -201,8 +204,9 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 
 // Slots of the children of a node whose boxes the ray enters before tmax.  The
 // far distance counts 4e-6 more, which exceeds the rounding of the distances
-// here and slab's factor.  A zero direction component makes its axis NaN,
-// which the minima and maxima ignore: the axis then culls nothing.  A child
+// here and slab's factor.  A direction component of zero, or so close to it that
+// wide_axis's scale overflows, makes its axis NaN, which the minima and maxima
+// ignore: the axis then culls nothing.  A child
 // is out when far * 1.000004 - near has its sign set.
 __device__ __forceinline__ uint32_t wide_hits(const WideRay& s, uint4 w0, uint4 w2, uint4 w3, uint4 w4) {
   unsigned long long sx, bx, sy, by, sz, bz;

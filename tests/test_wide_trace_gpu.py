@@ -1,0 +1,67 @@
+"""Rays through the eight-wide BVH against a test of every triangle: the closest hit's distance, barycentrics and
+triangle are equal bit for bit, and an any-hit query sees one exactly when there is one.  The same rays through the
+binary tree over the same build agree too."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import wide_probe  # noqa: E402
+
+
+def _soup(rng, n, size, at=(0.0, 0.0, 0.0)):
+    """Triangles of about `size` in a cube of edge 2."""
+    return rng.uniform(-1, 1, (n, 1, 3)) + size * rng.normal(size=(n, 3, 3)) + np.asarray(at)
+
+
+def _rays(rng, n, spread=1.5, at=(0.0, 0.0, 0.0), tmax=1e16):
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    return np.concatenate([rng.uniform(-spread, spread, (n, 3)) + np.asarray(at), d, np.full((n, 1), tmax)], 1)
+
+
+def _check(tris, rays, hits=True, binary_too=True):
+    wide, binary, every, seen = wide_probe.trace(tris, rays)
+    if hits:
+        assert (every["tri"] >= 0).mean() > 0.01
+    for got in (wide, binary)[:2 if binary_too else 1]:
+        differ = got != every
+        assert not differ.any(), (int(differ.sum()), got[differ][:4], every[differ][:4], np.asarray(rays)[differ][:4])
+    assert np.array_equal(seen, every["tri"] >= 0)
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 300, 20_000])
+@pytest.mark.parametrize("count", [1, 31, 40_000])
+def test_random_triangles(n, count):
+    rng = np.random.default_rng(n + count)
+    _check(_soup(rng, n, 0.3 if n < 300 else 0.05), _rays(rng, count), hits=n >= 300 and count > 1000)
+
+
+def test_coinciding_triangles_and_bounded_rays():
+    """Every triangle four times (equal distances: the lowest wins), and rays that end at, before and after a hit."""
+    rng = np.random.default_rng(3)
+    tris = np.tile(_soup(rng, 500, 0.1), (4, 1, 1))
+    rays = _rays(rng, 30_000)
+    _check(tris, rays)
+    t = wide_probe.trace(tris, rays)[2]["t"]
+    for k in (np.float32(1.0), np.nextafter(np.float32(1), np.float32(0)), np.float32(1.5)):
+        rays[:, 6] = np.where(t > 0, t * k, 1.0)
+        _check(tris, rays, hits=False)
+
+
+@pytest.mark.parametrize("small", [0.0, 1e-38, 1e-37, 1e-36, 1e-35, 1e-33, 1e-30, 1e-20], ids=str)
+@pytest.mark.parametrize("scale", [1.0, 1e4])
+def test_rays_almost_along_an_axis(small, scale):
+    """One or two components of the direction that are zero or close to it, of either sign."""
+    rng = np.random.default_rng(7)
+    tris = scale * _soup(rng, 4000, 0.1)
+    rays = _rays(rng, 20_000)
+    rays[:, :3] *= scale
+    sign = rng.choice([-1.0, 1.0], (20_000, 3))
+    keep = rng.integers(0, 3, 20_000)
+    both = rng.random(20_000) < 0.5
+    for axis in range(3):
+        tiny = (keep != axis) & (both | ((keep + 1) % 3 == axis))
+        rays[tiny, 3 + axis] = small * sign[tiny, axis]
+    _check(tris, rays)

@@ -71,6 +71,22 @@ __global__ void k_binary(BvhView bvh, const Ray* rays, uint32_t n, float4* close
   }
 }
 
+__global__ void k_all(BvhView bvh, const Ray* rays, uint32_t n, float4* closest) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const RayPre r = make_ray_pre(v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]),
+                                  v3(rays[k].d[0], rays[k].d[1], rays[k].d[2]));
+    Hit h;
+    h.t = rays[k].tmax;
+    h.b1 = h.b2 = 0.0f;
+    h.tri = 0x7FFFFFFF;
+    for (uint32_t t = 0; t < bvh.ntris; ++t) {
+      const float4 a = bvh.tris[3 * t], b = bvh.tris[3 * t + 1], c = bvh.tris[3 * t + 2];
+      tri_test(r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), (int)t, (int)t, &h);
+    }
+    closest[k] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.tri == 0x7FFFFFFF ? -1 : h.tri));
+  }
+}
+
 }  // namespace
 
 extern "C" {
@@ -99,17 +115,17 @@ uint64_t probe_wide_nodes(const float* boxes, uint32_t nleaves, int skew, uint32
   return count;
 }
 
-// Closest hits (t, b1, b2, BVH-order triangle as int bits, t free without a hit) of n rays through the wide tree and
-// through the binary one, and whether the wide any-hit query sees one.  0 on success.
+// Closest hits (t, b1, b2, BVH-order triangle as int bits, t free without a hit) of n rays through the wide tree,
+// through the binary one and among all triangles, and whether the wide any-hit query sees one.  0 on success.
 int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t ntris, const float* rays, uint32_t n,
-                float* wideHits, float* binaryHits, int* any) {
+                float* wideHits, float* binaryHits, float* allHits, int* any) {
   try {
     cudaStream_t s = nullptr;
     DBuf<float> dpos;
     DBuf<uint32_t> didx, taken(2);
     DBuf<unsigned int> bound(1);
     DBuf<Ray> drays;
-    DBuf<float4> a(n), b(n);
+    DBuf<float4> a(n), b(n), c(n);
     DBuf<int> dany(n);
     dpos.upload(pos, 3 * (size_t)nverts, s);
     didx.upload(idx, 3 * (size_t)ntris, s);
@@ -124,10 +140,12 @@ int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t
     k_wide<<<sm_count() * 4, 128, 0, s>>>(bvh.view(), wide.view(), drays.get(), n, taken.get(), bound.get(), a.get(),
                                           dany.get());
     k_binary<<<sm_count() * 8, 128, 0, s>>>(bvh.view(), drays.get(), n, b.get());
+    k_all<<<sm_count() * 8, 128, 0, s>>>(bvh.view(), drays.get(), n, c.get());
     R2_CUDA(cudaGetLastError());
     unsigned int ended = 0;
     a.download(reinterpret_cast<float4*>(wideHits), n, s);
     b.download(reinterpret_cast<float4*>(binaryHits), n, s);
+    c.download(reinterpret_cast<float4*>(allHits), n, s);
     dany.download(any, n, s);
     bound.download(&ended, 1, s);
     R2_CUDA(cudaStreamSynchronize(s));
