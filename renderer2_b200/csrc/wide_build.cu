@@ -29,20 +29,33 @@ struct WideBuild {
   uint32_t* state;
 };
 
-// One axis of a node's frame: the largest power of two 2^e in whose units the
-// extent is at most 252, and an origin one unit below the box, so that a
-// child's planes and 1/64 unit around them (far more than the traversal's
-// rounding in units) lie within 0 .. 255.
+// One axis of a node's frame: the smallest power of two 2^e in whose units the
+// box and one unit below it take at most 254, and an origin at least one unit
+// below the box, so that a child's planes and 1/64 unit around them (far more
+// than the traversal's rounding in units) lie within 0 .. 255.  Far from zero a
+// unit can be less than lo's unit in the last place: the origin is rounded down
+// and the unit grown until the box fits above it.  A box without extent keeps
+// the smallest unit and its own origin: the traversal's rounding is then all
+// relative to the distance.
 __device__ __forceinline__ void frame_axis(float lo, float hi, float* origin, uint32_t* exponent) {
   int e = 0;
   const float ext = hi - lo;
   frexpf(ext / 252.0f, &e);
   if (!(ext > 0.0f)) e = -126;
   e = isfinite(ext) ? max(-126, min(126, e)) : 126;
+  if (!(ext > 0.0f) || e >= 126) {
+    *exponent = (uint32_t)(e + 127);
+    *origin = lo - __uint_as_float(*exponent << 23);
+    return;
+  }
+  float from;
+  for (;; ++e) {
+    from = __fsub_rd(lo, __uint_as_float((uint32_t)(e + 127) << 23));
+    if (__fsub_ru(hi, from) * __uint_as_float((uint32_t)(127 - e) << 23) <= 254.0f || e == 126) break;
+  }
   *exponent = (uint32_t)(e + 127);
-  *origin = lo - __uint_as_float(*exponent << 23);
+  *origin = from;
 }
-// (x - origin and the scaling are exact or within 2e-5 of a unit.)
 __device__ __forceinline__ uint32_t plane(float x, float origin, float perUnit, bool upper) {
   const float q = (x - origin) * perUnit;
   const float r = upper ? ceilf(q + 0.015625f) : floorf(q - 0.015625f);

@@ -65,3 +65,24 @@ def test_rays_almost_along_an_axis(small, scale):
         tiny = (keep != axis) & (both | ((keep + 1) % 3 == axis))
         rays[tiny, 3 + axis] = small * sign[tiny, axis]
     _check(tris, rays)
+
+
+@pytest.mark.parametrize("at", [(1e3, -5e2, 2.5e2), (1e5, 1e5, -1e5), (3e6, 1e4, -2e6)], ids=["1e3", "1e5", "3e6"])
+@pytest.mark.parametrize("edge", [8, 60, 500], ids=str)
+def test_small_triangles_far_from_the_origin(at, edge):
+    """Cells of a grid of whole units in the last place, `edge` of them long, far from the origin: nodes of few units,
+    whose frames a float can hardly place, faces that share coordinates, and rays from nearby.  (The binary tree's own
+    test gives way by two units in the last place of the distance only and loses a few of these hits in a million.)"""
+    rng = np.random.default_rng(edge)
+    ulp = float(np.spacing(np.float32(max(abs(x) for x in at))))
+    base = np.round(np.asarray(at) / ulp) * ulp
+    cell = rng.integers(0, 12, (3000, 1, 3)) * edge
+    corner = rng.integers(0, 2, (3000, 3, 3)) * edge
+    tris = base + ulp * (cell + corner)
+    rays = _rays(rng, 200_000)
+    start = rng.integers(-2, 15, (200_000, 3)) * edge
+    target = rng.integers(0, 13, (200_000, 3)) * edge
+    rays[:, :3] = base + ulp * start
+    d = (target - start).astype(np.float64) + 0.01 * rng.normal(size=(200_000, 3))
+    rays[:, 3:6] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    _check(tris, rays, binary_too=False)
