@@ -81,3 +81,16 @@ def test_a_grid_in_parts_equals_the_whole():
     torch.cuda.synchronize()
     sc.close()
     assert torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("scale", [1e-14, 1e-12, 1e-10, 1e-6, 1e6, 1e10, 1e12], ids=str)
+def test_hits_match_the_oracle_at_any_scale(scale):
+    """Triangles whose edges' fourth powers leave the range of a float."""
+    mesh = _awkward(4)
+    m2w = np.array([scale, 0, 0, 0, scale, 0, 0, 0, scale, 0, 0, 0], np.float32)
+    mat = F.material(diffuse=(0.2, 0.5, 0.1), alpha=0.4)
+    prm = F.params(samples_per_voxel=40, iterations=3, seed=3)
+    g, gc, gw, st = _gpu_filter(mesh, mat, prm, scenes.voxel_size_for(mesh, 9) * scale, m2w)
+    ow, oc = _oracle(mesh, mat, prm, g, m2w)
+    assert ow[:, 17].sum() > 0
+    assert np.array_equal(gw[:, 17], ow[:, 17])

@@ -72,7 +72,7 @@ def test_rays_almost_along_an_axis(small, scale):
 def test_small_triangles_far_from_the_origin(at, edge):
     """Cells of a grid of whole units in the last place, `edge` of them long, far from the origin: nodes of few units,
     whose frames a float can hardly place, faces that share coordinates, and rays from nearby.  (The binary tree's own
-    test gives way by two units in the last place of the distance only and loses a few of these hits in a million.)"""
+    test gives way by two units in the last place of the distance only and loses a few of these hits in 200,000.)"""
     rng = np.random.default_rng(edge)
     ulp = float(np.spacing(np.float32(max(abs(x) for x in at))))
     base = np.round(np.asarray(at) / ulp) * ulp

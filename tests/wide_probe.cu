@@ -115,6 +115,29 @@ uint64_t probe_wide_nodes(const float* boxes, uint32_t nleaves, int skew, uint32
   return count;
 }
 
+// Buffers placed in one allocation by two users that ask for different parts of it in turn, as a builder does for
+// triangles (large) and for boxes (none of the first part, more of the others): how often a buffer moved after the
+// first turn of each.
+int probe_reserve_moves(uint32_t large, uint32_t more, int turns) {
+  try {
+    DBuf<uint8_t> mem;
+    DBuf<float4> boxes;
+    DBuf<uint64_t> keys;
+    int moves = 0;
+    for (int k = 0; k < turns; ++k) {
+      reserve_together(mem, part(boxes, large), part(keys, large));
+      const void *a = boxes.get(), *b = keys.get();
+      reserve_together(mem, part(boxes, 0), part(keys, more));
+      const void *c = boxes.get(), *d = keys.get();
+      if (k > 0) moves += (a != c) + (b != d);
+      if (boxes.size() < large || keys.size() < more) return -1;
+    }
+    return moves;
+  } catch (const Error&) {
+    return -2;
+  }
+}
+
 // Closest hits (t, b1, b2, BVH-order triangle as int bits, t free without a hit) of n rays through the wide tree,
 // through the binary one and among all triangles, and whether the wide any-hit query sees one.  0 on success.
 int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t ntris, const float* rays, uint32_t n,
