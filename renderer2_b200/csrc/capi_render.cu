@@ -186,7 +186,7 @@ r2_status r2_scene_wave_samples(r2_scene* scene, const r2_camera* camera, const 
   R2_API_BEGIN
   R2_REQUIRE(scene && camera && params && samples_out, R2_ERR_INVALID_ARGUMENT, "null argument");
   R2_REQUIRE(params->spp > 0, R2_ERR_INVALID_ARGUMENT, "spp must be positive");
-  *samples_out = scene->impl->wave_spp(camera->width * camera->height, params->spp);
+  *samples_out = scene->impl->wave_samples(camera->width * camera->height, params->spp);
   R2_API_END
 }
 

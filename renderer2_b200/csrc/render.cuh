@@ -88,8 +88,9 @@ constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a re
 // Paths per wave a frame's samples are grouped to.  A wave's later bounces hold
 // a few per cent of its paths, so larger waves keep the traversals' lanes and
 // the launches full: 64 samples of 1024x1024, 98.3 / 87.3 / 81.5 ms with 4M / 8M /
-// 16M paths (4 GB of state at 16M).  Served jobs share the device and keep
-// waves of kServeWavePaths; a frame whose 16M paths do not fit falls back to them.
+// 16M paths (3.6 GB of state at 16M, 5.8 with media; 0.9 and 1.5 at 4M).  They are
+// taken while memory is plenty (RenderContext::take_large); otherwise, and for
+// served jobs, which share the device, waves have kServeWavePaths.
 constexpr uint32_t kDefaultWavePaths = 1u << 24;
 constexpr uint32_t kServeWavePaths = 1u << 22;
 // media_rounds of a tuning, default and largest: accepted, without effect.

@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "asset_io.h"
 #include "host_math.h"
@@ -115,6 +116,7 @@ RenderContext::~RenderContext() {
     cudaStreamSynchronize(side.stream);
     cudaStreamDestroy(side.stream);
   }
+  release();
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -678,6 +680,38 @@ void RenderContext::ensure(uint32_t n, bool media) {
   }
 }
 
+// Bytes that the process's contexts hold beyond what small waves take.
+static std::atomic<size_t> g_largeWaveBytes{0};
+
+bool RenderContext::take_large(uint32_t n, uint32_t small, bool media) {
+  const uint32_t c = capacity_for(n);
+  if (c <= cap_ && (!media || c <= mediaCap_)) return true;
+  if (refused(n)) return false;
+  const size_t extra = bytes_for(n, media) - bytes_for(small, media);
+  size_t free = 0, total = 0;
+  bool room = cudaMemGetInfo(&free, &total) == cudaSuccess && extra <= free / 16;
+  if (room && extra > extra_) {
+    const size_t more = extra - extra_;
+    size_t held = g_largeWaveBytes.load();
+    do {
+      room = held + more <= total / 8;
+    } while (room && !g_largeWaveBytes.compare_exchange_weak(held, held + more));
+    if (room) extra_ = extra;
+  }
+  if (room) {
+    try {
+      ensure(n, media);
+      return true;
+    } catch (const Error& e) {
+      release();
+      if (e.code != R2_ERR_OUT_OF_MEMORY) throw;
+    }
+  }
+  cudaGetLastError();
+  refused_ = c;
+  return false;
+}
+
 size_t RenderContext::bytes_for(uint32_t n, bool media) {
   n = capacity_for(n);
   // per path: 5 float4 state + 3 x 2 float4 records + float4 throughput + 4 queue ids + 2 transmittances
@@ -689,6 +723,8 @@ size_t RenderContext::bytes_for(uint32_t n, bool media) {
 
 void RenderContext::release() {
   cap_ = mediaCap_ = 0;
+  g_largeWaveBytes -= extra_;
+  extra_ = 0;
   for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &swP_})
     b->release();
   for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &counts_, &sortBins_, &mc_, &pj_, &cl_}) b->release();
@@ -730,13 +766,29 @@ void RenderScene::check_params(const r2_camera& c, const r2_render_params& p, co
   R2_REQUIRE((p.flags & ~R2_RENDER_BRICK_GRID) == 0, R2_ERR_INVALID_ARGUMENT, "unknown render flags");
 }
 
-uint32_t RenderScene::wave_spp(uint32_t npix, uint32_t spp, uint32_t maxWavePaths) const {
-  uint64_t target = tuning_.wave_paths ? tuning_.wave_paths : kDefaultWavePaths;
-  if (maxWavePaths && maxWavePaths < target) target = maxWavePaths;
+// The largest divisor of spp whose wave has at most `paths` paths (at least one sample).
+static uint32_t wave_spp_of(uint32_t paths, uint32_t npix, uint32_t spp) {
   uint32_t best = 1;
   for (uint32_t k = 2; k <= spp; ++k)
-    if (spp % k == 0 && (uint64_t)k * npix <= target && (uint64_t)k * npix < (1ull << 31)) best = k;
+    if (spp % k == 0 && (uint64_t)k * npix <= paths && (uint64_t)k * npix < (1ull << 31)) best = k;
   return best;
+}
+
+uint32_t RenderScene::wave_spp(uint32_t npix, uint32_t spp, uint32_t maxWavePaths) const {
+  const uint32_t target = tuning_.wave_paths ? tuning_.wave_paths : kDefaultWavePaths;
+  return wave_spp_of(maxWavePaths ? std::min(target, maxWavePaths) : target, npix, spp);
+}
+
+uint32_t RenderScene::wave_samples(uint32_t npix, uint32_t spp) const {
+  const uint32_t S = wave_spp(npix, spp), small = wave_spp(npix, spp, serve_wave_paths());
+  return S != small && ctx_.refused(npix * S) ? small : S;
+}
+
+uint32_t RenderScene::take_waves(uint32_t npix, uint32_t spp) {
+  const uint32_t S = wave_spp(npix, spp), small = wave_spp(npix, spp, serve_wave_paths());
+  if (S != small && ctx_.take_large(npix * S, npix * small, !media_.empty())) return S;
+  ctx_.ensure(npix * small, !media_.empty());
+  return small;
 }
 
 RenderLaunch RenderScene::make_launch(const RenderContext& ctx, const r2_camera& c, const r2_render_params& p,
@@ -773,17 +825,7 @@ void RenderScene::render(const r2_camera& c, const r2_render_params& p, float* d
   RenderContext& ctx = ctx_;
   if (!s) s = ctx.stream;
   const uint32_t npix = c.width * c.height;
-  uint32_t S = wave_spp(npix, p.spp);
-  const uint32_t small = wave_spp(npix, p.spp, serve_wave_paths());
-  try {
-    ctx.ensure(npix * S, !media_.empty());
-  } catch (const Error& e) {  // not enough memory for large waves
-    if (e.code != R2_ERR_OUT_OF_MEMORY || small == S) throw;
-    cudaGetLastError();
-    ctx.release();
-    S = small;
-    ctx.ensure(npix * S, !media_.empty());
-  }
+  const uint32_t S = take_waves(npix, p.spp);
   RenderLaunch L = make_launch(ctx, c, p, d_frame, S);
   R2_CUDA(cudaMemsetAsync(ctx.bound.get(), 0, sizeof(unsigned int), s));
   const int nblocks = wave_blocks(npix * S);
@@ -883,6 +925,7 @@ void RenderScene::set_tuning(const r2_render_tuning& t) {
              "tuning out of range (track_steps <= 1024, trav_refill <= 32, wave_paths < 2^31, media_rounds <= 32, "
              "track_blocks <= 64, track_limit <= 2^20, top_nodes <= 256, sort_rays <= 1)");
   tuning_ = t;
+  ctx_.forget_refusal();
 }
 
 r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_params& p) {
@@ -917,7 +960,14 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
   };
   r2_render_tuning cur{kDefaultTrackSteps, kDefaultTravVisits, kDefaultTravRefill, kDefaultWavePaths,
                        kDefaultMediaRounds, 0, saved.track_limit, 0, 0};  // the step bound is kept, never tuned
+  // waves larger than small ones only where their memory is to be had, as for a frame by default
+  const uint32_t small = wave_spp_of(kServeWavePaths, npix, p.spp);
+  auto room = [&](uint32_t wavePaths) {
+    const uint32_t S = wave_spp_of(wavePaths, npix, p.spp);
+    return S <= small || ctx.take_large(npix * S, npix * small, !media_.empty());
+  };
   try {
+    if (!room(cur.wave_paths)) cur.wave_paths = kServeWavePaths;
     R2_CUDA(cudaMemsetAsync(ctx.bound.get(), 0, sizeof(unsigned int), s));
     time_wave(cur);  // warm-up
     float curT = time_wave(cur);
@@ -930,7 +980,7 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
           tuning_ = t;
           const uint32_t S = wave_spp(npix, p.spp);
           tuning_ = cur;
-          if (S == wave_spp(npix, p.spp)) continue;
+          if (S == wave_spp(npix, p.spp) || !room(cand[i])) continue;
         }
         const float ms = time_wave(t);
         if (ms < curT * 0.98f) {

@@ -41,7 +41,15 @@ class RenderContext {
   // Buffers for at least npix paths (media: the walks' state too),
   // grown in steps so that renders of varying size reallocate rarely.
   void ensure(uint32_t npix, bool media);
-  // Gives the path buffers back (after an ensure that ran out of memory).
+  // ensure(npix) for a wave that is larger than it need be (small paths), as
+  // long as memory is plenty: what it takes beyond the small wave must be at
+  // most a sixteenth of the memory that is free and, over all contexts of the
+  // process, an eighth of the device.  False, with nothing taken, when it is
+  // not; the size is then refused without another look until forget_refusal.
+  bool take_large(uint32_t npix, uint32_t small, bool media);
+  bool refused(uint32_t npix) const { return refused_ && capacity_for(npix) >= refused_; }
+  void forget_refusal() { refused_ = 0; }
+  // Gives the path buffers back.
   void release();
   void fill(PathState* st) const;
   // Device bytes a render of npix paths needs (buffers as ensure grows them + frame).
@@ -60,6 +68,8 @@ class RenderContext {
 
  private:
   uint32_t cap_ = 0, mediaCap_ = 0;
+  uint32_t refused_ = 0;  // least capacity that take_large refused (0: none)
+  size_t extra_ = 0;      // this context's part of the bytes beyond small waves
   DBuf<uint8_t> mem_, mediaMem_;  // the path buffers, in one allocation each
   DBuf<float4> rayO_, rayD_, T_, L_, hit_, shO_, shD_, shPre_, shT_;
   DBuf<uint32_t> q0_, q1_, qh_, qs_, counts_, sortBins_;
@@ -131,6 +141,9 @@ class RenderScene {
   // within the tuning's paths per wave, or maxWavePaths if smaller and nonzero
   // (at least one sample).
   uint32_t wave_spp(uint32_t npix, uint32_t spp, uint32_t maxWavePaths = 0) const;
+  // Samples per wave of the scene's own frames: wave_spp's, or those of waves of
+  // kServeWavePaths where the default large ones were refused for their memory.
+  uint32_t wave_samples(uint32_t npix, uint32_t spp) const;
   // The cap on served jobs' waves: none when the tuning sets the paths per wave.
   uint32_t serve_wave_paths() const { return tuning_.wave_paths ? 0u : kServeWavePaths; }
   // Launch tuning (0 fields: the defaults) and the autotuner that sets it.
@@ -146,6 +159,8 @@ class RenderScene {
  private:
   RenderLaunch make_launch(const RenderContext& ctx, const r2_camera& c, const r2_render_params& p, float* d_frame,
                            uint32_t waveSpp);
+  // wave_samples of a frame on the scene's context, its buffers taken.
+  uint32_t take_waves(uint32_t npix, uint32_t spp);
   static void check_params(const r2_camera& c, const r2_render_params& p, const float* d_frame);
   RenderContext ctx_;
   bool committed_ = false;

@@ -1,13 +1,77 @@
-"""Device memory that scenes keep: buffers that stay where they are between builds."""
+"""Device memory that scenes keep: buffers that stay where they are between builds, and the state of large waves, which a
+frame takes only while it is a small part of what is free and of the device."""
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import wide_probe  # noqa: E402
+from renderer2_b200 import raytracer as R  # noqa: E402
+from renderer2_b200 import render_scenes as RS  # noqa: E402
+
+GB = 1 << 30
 
 
 @pytest.mark.parametrize("large,more", [(1000, 10), (1000, 1000), (1000, 5000)])
 def test_buffers_of_one_allocation_stay_in_place(large, more):
     """A builder that builds triangles and boxes by turns allocates in the first turn alone."""
     assert wide_probe.lib().probe_reserve_moves(large, more, 4) == 0
+
+
+def _scene():
+    desc, _ = RS.icosphere_grid_scene()
+    return RS.build_scene(desc), R.camera(1024, 1024, 45.0, (0, 0, 24), (0, 0, 0), (0, 1, 0)), R.params(16, 4, 1)
+
+
+def _render(sc, cam, prm):
+    frame = torch.empty((cam.height, cam.width, 3), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    sc.render_device(cam, prm, frame.data_ptr())
+    torch.cuda.synchronize()
+    return frame, before - torch.cuda.mem_get_info()[0]
+
+
+def test_large_waves_leave_a_nearly_full_device_alone():
+    """16M paths take 3.6 GB; with 20 GB free a frame keeps to waves of 4M (0.9 GB), frame after frame, and the tuner
+    too.  The frame is the same bit for bit."""
+    sc, cam, prm = _scene()
+    want, large = _render(sc, cam, prm)
+    assert large > 2 * GB and sc.wave_samples(cam, prm) == 16
+    sc.close()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - 20 * GB, dtype=torch.uint8, device="cuda")
+    try:
+        sc, cam, prm = _scene()
+        got, small = _render(sc, cam, prm)
+        assert small < 2 * GB and torch.equal(got, want)
+        assert sc.wave_samples(cam, prm) == 4
+        again, more = _render(sc, cam, prm)
+        assert more <= 0 and torch.equal(again, want)
+        before = torch.cuda.mem_get_info()[0]
+        sc.autotune(cam, prm)
+        tuned, _ = _render(sc, cam, prm)
+        assert before - torch.cuda.mem_get_info()[0] < GB and torch.equal(tuned, want)
+        sc.close()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+
+
+def test_scenes_together_are_bounded():
+    """However many scenes are rendered, their large waves take no more than an eighth of the device beyond what waves
+    of 4M paths take, and a scene that is closed gives its share back."""
+    total = torch.cuda.mem_get_info()[1]
+    scenes, grew = [], []
+    for _ in range(12):
+        sc, cam, prm = _scene()
+        grew.append(_render(sc, cam, prm)[1])
+        scenes.append(sc)
+    extra = sum(max(0, g - 1.1 * GB) for g in grew)
+    assert max(grew) > 2 * GB and grew[-1] < 2 * GB and extra <= total / 8
+    for sc in scenes:
+        sc.close()
+    sc, cam, prm = _scene()
+    assert _render(sc, cam, prm)[1] > 2 * GB
+    sc.close()
