@@ -55,7 +55,12 @@ class DBuf {
   void alloc(size_t n) {
     release();
     if (n == 0) return;
-    R2_CUDA(cudaMalloc((void**)&p_, n * sizeof(T)));
+    const cudaError_t e = cudaMalloc((void**)&p_, n * sizeof(T));
+    if (e != cudaSuccess) {
+      p_ = nullptr;
+      cudaGetLastError();  // reported here, not by the next launch as well
+    }
+    R2_CUDA(e);
     n_ = n;
   }
   // Grow-only reallocation (contents are not preserved).

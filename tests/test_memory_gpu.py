@@ -75,3 +75,23 @@ def test_scenes_together_are_bounded():
     sc, cam, prm = _scene()
     assert _render(sc, cam, prm)[1] > 2 * GB
     sc.close()
+
+
+def test_a_failed_allocation_fails_one_call():
+    """A frame whose smallest wave does not fit is refused for its memory; the next call is not."""
+    from renderer2_b200 import _native as N
+    sc, cam, prm = _scene()
+    small = R.camera(64, 64, 45.0, (0, 0, 24), (0, 0, 0), (0, 1, 0))
+    want, _ = _render(sc, small, prm)
+    huge = R.camera(20000, 20000, 45.0, (0, 0, 24), (0, 0, 0), (0, 1, 0))  # 400M paths at one sample: 90 GB
+    held = torch.empty(torch.cuda.mem_get_info()[0] - 20 * GB, dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(N.R2Error) as e:
+            sc.render_device(huge, R.params(1, 2, 0), held.data_ptr())
+        assert e.value.name == "R2_ERR_OUT_OF_MEMORY"
+        got, _ = _render(sc, small, prm)
+        assert torch.equal(got, want)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+        sc.close()
