@@ -34,28 +34,23 @@ struct WideBuild {
 // below the box, so that a child's planes and 1/64 unit around them (far more
 // than the traversal's rounding in units) lie within 0 .. 255.  Far from zero a
 // unit can be less than lo's unit in the last place: the origin is rounded down
-// and the unit grown until the box fits above it.  A box without extent keeps
-// the smallest unit and its own origin: the traversal's rounding is then all
-// relative to the distance.
+// and the unit grown until the box fits above it; a box without extent counts as
+// one of about a unit in the last place.  Units stay between 2^-42 and 2^23 (see
+// wide_rcp); a box of more than 2e9 or an infinite one gets an infinite unit, whose planes are no numbers: the axis then culls nothing.
 __device__ __forceinline__ void frame_axis(float lo, float hi, float* origin, uint32_t* exponent) {
   int e = 0;
-  const float ext = hi - lo;
+  const float ext = fmaxf(hi - lo, 1.2e-7f * fmaxf(fabsf(lo), fabsf(hi)));
   frexpf(ext / 252.0f, &e);
-  if (!(ext > 0.0f)) e = -126;
-  e = isfinite(ext) ? max(-126, min(126, e)) : 126;
-  if (!(ext > 0.0f) || e >= 126) {
-    *exponent = (uint32_t)(e + 127);
-    *origin = lo - __uint_as_float(*exponent << 23);
-    return;
-  }
-  float from;
-  for (;; ++e) {
+  if (!(ext > 0.0f)) e = -42;
+  float from = lo;
+  for (e = max(e, -42); isfinite(ext) && e <= 23; ++e) {
     from = __fsub_rd(lo, __uint_as_float((uint32_t)(e + 127) << 23));
-    if (__fsub_ru(hi, from) * __uint_as_float((uint32_t)(127 - e) << 23) <= 254.0f || e == 126) break;
+    if (__fsub_ru(hi, from) * __uint_as_float((uint32_t)(127 - e) << 23) <= 254.0f) break;
   }
-  *exponent = (uint32_t)(e + 127);
+  *exponent = isfinite(ext) && e <= 23 ? (uint32_t)(e + 127) : 255u;
   *origin = from;
 }
+// (x - origin and the scaling are exact or within 2e-5 of a unit.)
 __device__ __forceinline__ uint32_t plane(float x, float origin, float perUnit, bool upper) {
   const float q = (x - origin) * perUnit;
   const float r = upper ? ceilf(q + 0.015625f) : floorf(q - 0.015625f);

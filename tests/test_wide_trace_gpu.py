@@ -22,7 +22,7 @@ def _rays(rng, n, spread=1.5, at=(0.0, 0.0, 0.0), tmax=1e16):
 
 
 def _check(tris, rays, hits=True, binary_too=True):
-    wide, binary, every, seen = wide_probe.trace(tris, rays)
+    wide, binary, every, seen, _ = wide_probe.trace(tris, rays)
     if hits:
         assert (every["tri"] >= 0).mean() > 0.01
     for got in (wide, binary)[:2 if binary_too else 1]:
@@ -51,7 +51,7 @@ def test_coinciding_triangles_and_bounded_rays():
 
 
 @pytest.mark.parametrize("small", [0.0, 1e-38, 1e-37, 1e-36, 1e-35, 1e-33, 1e-30, 1e-20], ids=str)
-@pytest.mark.parametrize("scale", [1.0, 1e4])
+@pytest.mark.parametrize("scale", [1e-11, 1e-8, 1.0, 1e4, 1e8, 1e10], ids=str)
 def test_rays_almost_along_an_axis(small, scale):
     """One or two components of the direction that are zero or close to it, of either sign."""
     rng = np.random.default_rng(7)
@@ -86,3 +86,23 @@ def test_small_triangles_far_from_the_origin(at, edge):
     d = (target - start).astype(np.float64) + 0.01 * rng.normal(size=(200_000, 3))
     rays[:, 3:6] = d / np.linalg.norm(d, axis=1, keepdims=True)
     _check(tris, rays, binary_too=False)
+
+
+@pytest.mark.parametrize("zero", [0.0, -0.0, 1e-38, -1e-30, 1e-19], ids=str)
+@pytest.mark.parametrize("flat", [False, True], ids=["soup", "flat"])
+def test_axis_parallel_rays_visit_no_more_nodes(zero, flat):
+    """A ray within a plane of constant x, y or z passes the boxes that a ray almost within it does, and no more than a
+    fifth besides."""
+    rng = np.random.default_rng(11)
+    tris = _soup(rng, 20_000, 0.02)
+    if flat:
+        tris[:, :, 1] = np.round(tris[:, :1, 1] * 20) / 20
+    rays = _rays(rng, 5000, spread=1.0)
+    axis = rng.integers(0, 3, 5000)
+    rays[np.arange(5000), 3 + axis] = zero
+    near = rays.copy()
+    near[np.arange(5000), 3 + axis] = 1e-7
+    _check(tris, rays)
+    along, almost = wide_probe.trace(tris, rays)[4], wide_probe.trace(tris, near)[4]
+    print(along.mean(), almost.mean(), (along / almost).max())
+    assert along.sum() <= 1.2 * almost.sum()

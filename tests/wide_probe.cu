@@ -87,6 +87,32 @@ __global__ void k_all(BvhView bvh, const Ray* rays, uint32_t n, float4* closest)
   }
 }
 
+// Wide nodes whose boxes each ray enters before its tmax.
+__global__ void k_visits(WideView wide, const Ray* rays, uint32_t n, uint32_t* visits) {
+  __shared__ WideWarp warps[4];
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    WideRay r;
+    wide_set(r, warps[threadIdx.x >> 5], threadIdx.x & 31, v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]),
+             v3(rays[k].d[0], rays[k].d[1], rays[k].d[2]), 0, 0u);
+    r.tmax = rays[k].tmax;
+    uint2 stack[R2_BVH_STACK];  // first child, inner children to visit and, above them, all
+    int sp = 0;
+    stack[sp++] = make_uint2(0u, 0x0101u);
+    uint32_t count = 0;
+    while (sp > 0) {
+      const uint32_t hits = stack[sp - 1].y & 0xFFu, slot = __ffs(hits) - 1u;
+      const uint32_t node = stack[sp - 1].x + __popc((stack[sp - 1].y >> 8) & ((1u << slot) - 1u));
+      stack[sp - 1].y &= ~(1u << slot);
+      if (!(stack[sp - 1].y & 0xFFu)) --sp;
+      const uint4* nd = wide.nodes + kWideWords * (size_t)node;
+      const uint32_t inner = nd[0].w >> 24, in = wide_hits(r, nd[0], nd[2], nd[3], nd[4]) & inner;
+      ++count;
+      if (in) stack[sp++] = make_uint2(nd[1].x, inner << 8 | in);
+    }
+    visits[k] = count;
+  }
+}
+
 }  // namespace
 
 extern "C" {
@@ -139,9 +165,10 @@ int probe_reserve_moves(uint32_t large, uint32_t more, int turns) {
 }
 
 // Closest hits (t, b1, b2, BVH-order triangle as int bits, t free without a hit) of n rays through the wide tree,
-// through the binary one and among all triangles, and whether the wide any-hit query sees one.  0 on success.
+// through the binary one and among all triangles, whether the wide
+// any-hit query sees one, and the wide nodes whose boxes the ray enters.  0 on success.
 int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t ntris, const float* rays, uint32_t n,
-                float* wideHits, float* binaryHits, float* allHits, int* any) {
+                float* wideHits, float* binaryHits, float* allHits, int* any, uint32_t* visits) {
   try {
     cudaStream_t s = nullptr;
     DBuf<float> dpos;
@@ -150,6 +177,7 @@ int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t
     DBuf<Ray> drays;
     DBuf<float4> a(n), b(n), c(n);
     DBuf<int> dany(n);
+    DBuf<uint32_t> dvisits(n);
     dpos.upload(pos, 3 * (size_t)nverts, s);
     didx.upload(idx, 3 * (size_t)ntris, s);
     drays.upload(reinterpret_cast<const Ray*>(rays), n, s);
@@ -164,12 +192,14 @@ int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t
                                           dany.get());
     k_binary<<<sm_count() * 8, 128, 0, s>>>(bvh.view(), drays.get(), n, b.get());
     k_all<<<sm_count() * 8, 128, 0, s>>>(bvh.view(), drays.get(), n, c.get());
+    k_visits<<<sm_count() * 8, 128, 0, s>>>(wide.view(), drays.get(), n, dvisits.get());
     R2_CUDA(cudaGetLastError());
     unsigned int ended = 0;
     a.download(reinterpret_cast<float4*>(wideHits), n, s);
     b.download(reinterpret_cast<float4*>(binaryHits), n, s);
     c.download(reinterpret_cast<float4*>(allHits), n, s);
     dany.download(any, n, s);
+    dvisits.download(visits, n, s);
     bound.download(&ended, 1, s);
     R2_CUDA(cudaStreamSynchronize(s));
     return ended ? 1 : 0;

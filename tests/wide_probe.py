@@ -25,7 +25,7 @@ def lib():
         _lib = C.CDLL(LIB)
         _lib.probe_wide_nodes.restype = C.c_uint64
         _lib.probe_wide_nodes.argtypes = [C.c_void_p, C.c_uint32, C.c_int, C.c_uint32, C.c_void_p]
-        _lib.probe_trace.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32] + [C.c_void_p] * 4
+        _lib.probe_trace.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32] + [C.c_void_p] * 5
     return _lib
 
 
@@ -39,16 +39,18 @@ def wide_nodes(boxes, skew, seed=1):
 
 def trace(tris, rays):
     """Hits of the rays, an (n, 7) array of origin, direction and tmax, among (m, 3, 3) triangles: records (t, b1, b2,
-    triangle) of the wide tree, of the binary one and of a test of every triangle, and whether the wide any-hit query found one."""
+    triangle) of the wide tree, of the binary one and of a test of every triangle, whether the wide any-hit query found
+    one, and the wide nodes whose boxes the ray enters."""
     pos = np.ascontiguousarray(tris, np.float32).reshape(-1, 3)
     idx = np.arange(pos.shape[0], dtype=np.uint32)
     rays = np.ascontiguousarray(rays, np.float32)
     n = rays.shape[0]
     rec = np.dtype([("t", "<f4"), ("b1", "<f4"), ("b2", "<f4"), ("tri", "<i4")])
-    a, b, c, seen = np.empty(n, rec), np.empty(n, rec), np.empty(n, rec), np.empty(n, np.int32)
+    a, b, c, seen, visits = (np.empty(n, t) for t in (rec, rec, rec, np.int32, np.uint32))
     status = lib().probe_trace(pos.ctypes.data, pos.shape[0], idx.ctypes.data, idx.size // 3, rays.ctypes.data, n,
-                               a.ctypes.data, b.ctypes.data, c.ctypes.data, seen.ctypes.data)
+                               a.ctypes.data, b.ctypes.data, c.ctypes.data, seen.ctypes.data,
+                               visits.ctypes.data)
     assert status == 0, status
     for h in (a, b, c):
         h["t"][h["tri"] < 0] = 0.0
-    return a, b, c, seen != 0
+    return a, b, c, seen != 0, visits
