@@ -50,8 +50,8 @@ FILTER_BYTES_PER_VOXEL = 36.0
 # hierarchy 1, bottom-up 1, emission 1, shading gather 1
 FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # no measured FP32 figure on this pool
 # media scenes:
-#   extend phase (k_walk, k_collide): queue id 4 + ray in/out 64 + throughput in/out 32 + hit record 16 = 116 B per segment
-#   shadow phase (k_shadow_surfaces, k_walk): record origin 16 + direction 16 + tmax/medium 8 + queue id 4 + transmittance 4 = 48 B per slot
+#   extend phase (k_find, k_track, k_walk, k_collide): queue id 4 + ray in/out 64 + throughput in/out 32 + hit record 16 = 116 B per segment
+#   shadow phase (k_shadow_surfaces, k_find, k_track, k_walk): record origin 16 + direction 16 + tmax/medium 8 + queue id 4 + transmittance 4 = 48 B per slot
 #   k_shade<true>: hit 16 + ray 32 + throughput 16 + radiance 16 + 2 records x 64 + continuation 48 = 256 B per segment
 VOLUME_EXTEND_BYTES_PER_SEGMENT = 116.0
 SHADOW_MEDIA_BYTES_PER_SLOT = 48.0
@@ -233,7 +233,13 @@ def filter_workload():
     return mesh, mat, prm, vs
 
 
-MEDIA_LAUNCHES = 8  # per bounce of a media scene: extend, walk, collide, events, shade, shadow rays, walk, accum
+
+
+def media_launches(tuning: dict, wave_paths: int) -> int:
+    """Kernels per bounce of a media scene: extend, walk, collide, events, shade, shadow rays, walk, accum, and per
+    queued round (waves of 2^18 paths and more) find and track of paths and of shadow rays."""
+    return 8 + (4 * (tuning["media_rounds"] or 1) if wave_paths >= 1 << 18 else 0)
+
 
 
 def _input_bytes(desc):
@@ -888,8 +894,8 @@ def bench_volume(args, world, local):
            "roofline": roofline, "latency": latency,
            "e2e": {"value": world * paths / (e2e_ms / 1e3), "unit": "paths/s", "h2d_bytes_per_step": int(h2d),
                    "d2h_bytes_per_step": int(npix * 12), "ms_per_step": e2e_ms},
-           # per wave: camera, finish; per bounce: MEDIA_LAUNCHES
-           "gpu_launches": (prm.spp // S) * (2 + MEDIA_LAUNCHES * prm.max_depth) * args.steps}
+           # per wave: camera, finish; per bounce: media_launches
+           "gpu_launches": (prm.spp // S) * (2 + media_launches(tuning, npix * S) * prm.max_depth) * args.steps}
     return out, (desc, cam, prm)
 
 
@@ -993,8 +999,8 @@ def bench_forest(args, world, local, cfg=None, autotune=True):
                                                "kind": "port", "sample": f"{n_cpu} trees"},
                               "placement_s": place_s, "placement_attempts": c["attempts"]},
             "scene_build_ms": build_ms,
-            # per wave: camera, finish; per bounce: MEDIA_LAUNCHES
-            "gpu_launches": (prm.spp // S) * (2 + MEDIA_LAUNCHES * prm.max_depth) * args.steps}
+            # per wave: camera, finish; per bounce: media_launches
+            "gpu_launches": (prm.spp // S) * (2 + media_launches(tuning, npix * S) * prm.max_depth) * args.steps}
 
 
 def bench_volume_batch(args, world, local):
@@ -1121,7 +1127,8 @@ def bench_volume_batch(args, world, local):
                                   f"over {args.steps} steps of {c['spp']} replays",
             "e2e": {"value": world * paths / (e2e_ms / 1e3), "unit": "paths/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(sum(npix) * 12), "ms_per_step": e2e_ms},
-            "gpu_launches": c["spp"] * c["scenes"] * (3 + MEDIA_LAUNCHES * c["depth"]) * args.steps}
+            "gpu_launches": c["spp"] * c["scenes"] * args.steps *
+            (3 + media_launches(batch_tuning.as_dict(), npix[0]) * c["depth"])}
 
 
 def serving_jobs(c=SERVE_CFG, seed=11):

@@ -294,8 +294,8 @@ typedef struct r2_render_tuning {
   uint32_t trav_refill; /* idle lanes of a warp (1..32) at which it ends finished rays and takes new ones */
   uint32_t wave_paths;  /* paths per wave: a wave renders the largest divisor of spp samples of every
                            pixel that keeps width*height*samples within it (at least one sample) */
-  uint32_t media_rounds; /* at most 32; without effect since a path's medium boundaries are walked in
-                            one persistent kernel */
+  uint32_t media_rounds; /* media: queued rounds of medium boundaries (1..32) in bounces of many paths, before
+                            the remaining boundaries are walked in one persistent kernel */
   uint32_t track_blocks; /* media: blocks per SM of the persistent trackers (at most the resident
                             blocks; 0: all of them) */
   uint32_t track_limit; /* media: bound on the steps of one tracking loop (delta / ratio tracking of

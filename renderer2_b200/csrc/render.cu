@@ -38,7 +38,7 @@ constexpr uint32_t kPurposeMedium = 0x1000u;   // + pass-through index within th
 constexpr uint32_t kPurposeScatter = 0x100u;   // phase-function and light draws at a collision
 constexpr uint32_t kPurposeShadowTr = 0x200u;  // + shadow slot (0 light, 1 BSDF)
 constexpr int kMaxPassThrough = 4096;          // medium boundaries crossed within one bounce
-constexpr int kMaxShadowSegments = 4096;       // medium boundaries along one shadow ray (per round)
+constexpr int kMaxShadowSegments = 4096;       // medium boundaries along one shadow ray between queued rounds
 
 __device__ __forceinline__ float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 // Sample index of the wave: a kernel parameter, or the device counter of a
@@ -510,12 +510,12 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) 
 // A persistent kernel (k_walk) gives each lane a path and alternates, warp by
 // warp, between finding the next boundaries (resolve_path, up to the path's
 // first segment that needs tracking) and stepping along the segments; a lane
-// whose path is done takes the next one.  So lanes wait neither for the warp's
-// longest path nor, between segments, for a launch, as they did when rounds of
-// queued segments alternated between two kernels (1,200 trees, delta tracking,
-// 36.4 -> 24.1 ms; a 128^3 crown through its brick grid 9.0 -> 7.5 ms).  In the
-// forest most rounds still run with few lanes: paths are few and differ much
-// in length.  Making the box search resumable too was no faster (26.6 ms), nor
+// whose path is done takes the next one.  Where paths are few, that spares the
+// launches between segments (1,200 trees at 640x360, delta tracking, 4 samples
+// 36.4 -> 24.1 ms; a 128^3 crown through its brick grid at 960x540, 8 samples, one
+// seed 9.0 -> 7.5 ms).  Where they are many, its lanes wait for one another's
+// phases, and queued rounds (k_find, k_track) come first: see kRoundPaths.
+// Making the box search resumable too was no faster (26.6 ms), nor
 // were caps on registers for 6 or 8 blocks an SM.  Every segment draws from
 // its own stream (purpose kPurposeMedium + j, j = medium boundaries met in the
 // bounce), so the order of the work changes no result.
@@ -1023,6 +1023,13 @@ __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_shadow_surfaces(RenderL
 }
 
 // ------------------------------------------------------------------ media: shadow transmittance
+// The ray of a shadow walk's segment from p0 towards p1 (CRay::spawnRay).
+__device__ __forceinline__ void shadow_segment(V3 p0, V3 p1, V3* off, V3* dir, float* tl) {
+  *off = offset_ray_origin(p0, normalize(p1 - p0));
+  *tl = length(p1 - *off);
+  *dir = (p1 - p0) / *tl;
+}
+
 // CDeviceScene::intersectTr as direct() uses it: 0 when the walk ends on a
 // surface (materials do not emit), else the product of the media's
 // ratio-tracking estimates.  A surface anywhere on the ray ends the walk there,
@@ -1038,6 +1045,7 @@ __device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot
   const float4 o4 = L.st.shO[slot], d4 = L.st.shD[slot];
   const float2 x = L.st.shX[slot];
   const V3 o = xyz(o4), d = xyz(d4);
+  const V3 p1 = o + d * x.x;
   V3 p0;
   int cur;
   float tr;
@@ -1047,19 +1055,20 @@ __device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot
     cur = __float_as_int(x.y);
     tr = 1.0f;
     idx = 0;
-  } else {
+  } else {  // past the tracked segment
     const float4 w = L.st.swP[slot];
-    const int2 m = L.st.swM[slot];
-    p0 = xyz(w);
+    V3 off, dir;
+    float tl;
+    shadow_segment(xyz(w), p1, &off, &dir, &tl);
+    p0 = off + dir * L.st.swT[slot];
+    cur = -1;
     tr = w.w;
-    cur = m.x;
-    idx = (uint32_t)m.y;
+    idx = (uint32_t)L.st.swM[slot].y;
   }
-  const V3 p1 = o + d * x.x;
   for (; *segments < kMaxShadowSegments; ++*segments) {
-    const V3 off = offset_ray_origin(p0, normalize(p1 - p0));
-    const float tl = length(p1 - off);
-    const V3 dir = (p1 - p0) / tl;
+    V3 off, dir;
+    float tl;
+    shadow_segment(p0, p1, &off, &dir, &tl);
     float best;
     int hitM = media_first(S, off, dir, tl, &best);
     if (hitM >= 0 && !(best < tl)) hitM = -1;
@@ -1069,8 +1078,9 @@ __device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot
     }
     if (cur >= 0 && hitM == cur) {
       *out = Segment{off, dir, best, cur, idx};
-      L.st.swP[slot] = f4(off + dir * best, tr);
-      L.st.swM[slot] = make_int2(-1, (int)idx);
+      L.st.swP[slot] = f4(p0, tr);
+      L.st.swM[slot] = make_int2(cur, (int)idx);
+      L.st.swT[slot] = best;
       ++*segments;
       return true;
     }
@@ -1082,11 +1092,126 @@ __device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot
   return false;
 }
 
+// Queued rounds.  Where a bounce has many paths (or events), their next segments
+// are found by one kernel, each lane its own, and tracked by another whose lanes
+// take the next segment of the queue as soon as their own ends; paths that go on
+// are found their next segment in the following round, and after the last round
+// k_walk takes them to their end.  k_track holds tentative collisions as k_walk does.
+__device__ __forceinline__ bool in_rounds(const RenderLaunch& L, uint32_t live) {
+  return L.mediaRounds > 0 && live >= kRoundPaths;
+}
+
+template <bool kSample>
+__global__ void __launch_bounds__(128) k_find(RenderLaunch L, int round) {
+  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce + (kSample ? 0 : kShadowCounters);
+  const uint32_t live = kSample ? *(volatile uint32_t*)&L.st.counts[L.bounce] : event_count(L);
+  if (!in_rounds(L, live)) return;
+  const uint32_t n = round ? *(volatile uint32_t*)&mc[3 * round - 1] : (kSample ? live : 2 * live);
+  const uint32_t* list = round ? (kSample ? L.st.pq[1] : L.st.sq[1]) : path_queue(L, L.bounce);
+  uint32_t* queue = kSample ? L.st.pq[0] : L.st.sq[0];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t owner = kSample || round ? list[i] : i;
+    if (!kSample && round == 0 && L.st.shTr[owner] == 0.0f) continue;  // no ray, or behind a surface
+    Segment seg;
+    int segments = 0;
+    if (kSample ? resolve_path(L, owner, round == 0, &seg) : shadow_walk(L, owner, round == 0, &seg, &segments)) {
+      if (kSample) {
+        L.st.evA[owner] = f4(seg.o, seg.tmax);
+        L.st.evB[owner] = f4(seg.d, __int_as_float(seg.med));
+      }
+      queue[warp_reserve(&mc[3 * round])] = owner;
+    }
+  }
+}
+
+template <bool kDDA, bool kSample>
+__global__ void __launch_bounds__(128) k_track(RenderLaunch L, int round) {
+  uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce + (kSample ? 0 : kShadowCounters);
+  const uint32_t njobs = *(volatile uint32_t*)&mc[3 * round];
+  uint32_t* taken = &mc[3 * round + 1];
+  const uint32_t* queue = kSample ? L.st.pq[0] : L.st.sq[0];
+  uint32_t* next = kSample ? L.st.pq[1] : L.st.sq[1];
+  const int lane = threadIdx.x & 31;
+  TrackState s;
+  uint32_t owner = 0;
+  int med = 0;
+  bool active = false, drained = false, pending = false;
+  const auto end = [&](int st) {
+    active = false;
+    if (kSample && st == kTrackCollide) finish_collide(L, owner, med, s);
+    else if (kSample ? finish_pass(L, owner, st) : finish_tr(L, owner, st, s)) next[warp_reserve(&mc[3 * round + 2])] = owner;
+  };
+  for (;;) {
+    const bool need = !active && !drained;
+    const unsigned want = __ballot_sync(0xffffffffu, need);
+    if (want) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(taken, (uint32_t)__popc(want));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base + (uint32_t)__popc(want) >= njobs) drained = true;  // warp-uniform
+      const uint32_t k = base + (uint32_t)__popc(want & ((1u << lane) - 1u));
+      if (need && k < njobs) {
+        owner = queue[k];
+        Ray r;
+        if (kSample) {
+          const float4 a = L.st.evA[owner], b = L.st.evB[owner];
+          r = make_ray(xyz(a), xyz(b), a.w);
+          med = __float_as_int(b.w);
+          s.rng = rng_stream(path_pixel(L, owner), L.seed, path_sample(L, owner), L.bounce,
+                             kPurposeMedium + L.st.pj[owner]);
+        } else {
+          const float4 o4 = L.st.shO[owner], d4 = L.st.shD[owner];
+          const int2 m = L.st.swM[owner];
+          V3 off, dir;
+          float tl;
+          shadow_segment(xyz(L.st.swP[owner]), xyz(o4) + xyz(d4) * L.st.shX[owner].x, &off, &dir, &tl);
+          r = make_ray(off, dir, L.st.swT[owner]);
+          med = m.x;
+          const uint32_t op = event_path(L, owner >> 1);
+          s.rng = rng_resume(path_pixel(L, op), L.seed, path_sample(L, op), L.bounce, kPurposeShadowTr + (owner & 1u),
+                             (uint32_t)m.y);
+        }
+        const int st = track_init<kDDA, kSample>(L.scene.media[med], r, &s, (int)L.trackLimit);
+        if (st == kTrackRunning) active = true;
+        else end(st);
+      }
+    }
+    if (!__any_sync(0xffffffffu, active)) {
+      if (drained) break;
+      continue;
+    }
+    if (kDDA) {
+      for (uint32_t k = 0; k < L.trackSteps; ++k) {
+        if (!__any_sync(0xffffffffu, active)) break;
+        int st = kTrackRunning;
+        if (active && !pending) {
+          st = track_dda_advance<kSample>(L.scene.media[med], s);
+          if (st == kTrackPending) {
+            pending = true;
+            st = kTrackRunning;
+          }
+        }
+        const unsigned held = __ballot_sync(0xffffffffu, pending);
+        const unsigned running = __ballot_sync(0xffffffffu, active && st == kTrackRunning);
+        if (held && 2 * __popc(held) >= __popc(running) && pending) {
+          st = track_dda_collide<kSample>(L.scene.media[med], s);
+          pending = false;
+        }
+        if (active && st != kTrackRunning) end(st);
+      }
+    } else {
+      for (uint32_t k = 0; k < L.trackSteps && active; ++k) {
+        const int st = track_step<kDDA, kSample>(L.scene.media[med], s);
+        if (st != kTrackRunning) end(st);
+      }
+    }
+  }
+}
+
 // Lanes at a boundary that make a warp look for their next one: the search is
-// long, so it waits for company unless no lane is tracking.  4 / 8 / 16: a 256^3
-// foliage medium at 1920x1080, 8 samples 140.0 / 136.6 / 149.3 ms, 1,200 trees at
-// 640x360 19.8 / 19.7 / 19.5 ms.  (The two-kernel rounds took 128.1 ms of the first
-// in waves of 16M paths, 196.0 ms in waves of 4M.)
+// long, so it waits for company unless no lane is tracking.  4 / 8 / 16 without queued
+// rounds: a 256^3 foliage medium at 1920x1080, 8 samples 140.0 / 136.6 / 149.3 ms,
+// 1,200 trees at 640x360 19.8 / 19.7 / 19.5 ms.
 constexpr int kResolveLanes = 8;
 
 // The bounce's paths (kSample) or shadow rays through the media.  With the
@@ -1099,8 +1224,12 @@ template <bool kDDA, bool kSample>
 __global__ void __launch_bounds__(128) k_walk(RenderLaunch L) {
   uint32_t* mc = L.st.mc + kCountersPerBounce * L.bounce;
   uint32_t* taken = &mc[kSample ? kPathCounter : kShadowCounter];
-  const uint32_t n = kSample ? *(volatile uint32_t*)&L.st.counts[L.bounce] : 2 * event_count(L);
-  const uint32_t* list = path_queue(L, L.bounce);
+  const uint32_t live = kSample ? *(volatile uint32_t*)&L.st.counts[L.bounce] : event_count(L);
+  // all of them, or what the last queued round left
+  const bool rest = in_rounds(L, live);
+  const uint32_t n = rest ? *(volatile uint32_t*)&mc[(kSample ? 0 : kShadowCounters) + 3 * L.mediaRounds - 1]
+                          : (kSample ? live : 2 * live);
+  const uint32_t* list = rest ? (kSample ? L.st.pq[1] : L.st.sq[1]) : path_queue(L, L.bounce);
   const int lane = threadIdx.x & 31;
   enum { kIdle, kResolve, kTracking, kEnded };
   int mode = kIdle;
@@ -1127,11 +1256,11 @@ __global__ void __launch_bounds__(128) k_walk(RenderLaunch L) {
         if (base + (uint32_t)__popc(want) >= n) drained = true;  // warp-uniform
         const uint32_t k = base + (uint32_t)__popc(want & ((1u << lane) - 1u));
         if (mode == kIdle && k < n) {
-          owner = kSample ? list[k] : k;
+          owner = kSample || rest ? list[k] : k;
           // shadow records without a ray, or behind a surface, are done
-          if (kSample || L.st.shTr[owner] != 0.0f) {
+          if (kSample || rest || L.st.shTr[owner] != 0.0f) {
             mode = kResolve;
-            fresh = true;
+            fresh = !rest;
             segments = 0;
           }
         }
@@ -1237,11 +1366,16 @@ int resident_blocks(K kernel, int threads, size_t smem = 0) {
   return std::max(1, n) * sm_count();
 }
 
-int g_trackBlocks[4] = {0, 0, 0, 0};  // resident blocks of k_walk<dda, sample>, by dda + 2 sample
+using RenderKernel = void (*)(RenderLaunch);
+// Resident blocks of k_walk<dda, sample> and k_track<dda, sample>, by dda + 2 sample.
+int g_walkBlocks[4] = {0, 0, 0, 0}, g_trackBlocks[4] = {0, 0, 0, 0};
+const RenderKernel kWalkVariants[4] = {k_walk<false, false>, k_walk<true, false>, k_walk<false, true>, k_walk<true, true>};
+using RoundKernel = void (*)(RenderLaunch, int);
+const RoundKernel kTrackVariants[4] = {k_track<false, false>, k_track<true, false>, k_track<false, true>,
+                                       k_track<true, true>};
 
 // The surface traversal kernels by variant: alpha + 2 * two-level; 4: a scene
 // without triangles.
-using RenderKernel = void (*)(RenderLaunch);
 const RenderKernel kExtendVariants[5] = {k_extend<true, false, false>, k_extend<true, true, false>,
                                          k_extend<true, false, true>, k_extend<true, true, true>,
                                          k_extend<false, false, false>};
@@ -1276,29 +1410,29 @@ int trav_blocks(int which, int variant) {
 }
 
 void query_track_blocks() {
-  if (g_trackBlocks[0] != 0) return;
-  g_trackBlocks[1] = resident_blocks(k_walk<true, false>, 128);
-  g_trackBlocks[2] = resident_blocks(k_walk<false, true>, 128);
-  g_trackBlocks[3] = resident_blocks(k_walk<true, true>, 128);
-  g_trackBlocks[0] = resident_blocks(k_walk<false, false>, 128);
+  if (g_walkBlocks[0] != 0) return;
+  for (int i = 3; i >= 0; --i) {
+    g_trackBlocks[i] = resident_blocks(kTrackVariants[i], 128);
+    g_walkBlocks[i] = resident_blocks(kWalkVariants[i], 128);
+  }
 }
 
 __global__ void k_advance_sample(uint32_t* sample, uint32_t n) { *sample += n; }
 
-void launch_walk(const RenderLaunch& L, bool sample, cudaStream_t s) {
-  query_track_blocks();
+// A bounce's paths (sample) or shadow rays through the media.
+void launch_media(const RenderLaunch& L, bool sample, int nblocks, cudaStream_t s) {
   const int which = (L.dda ? 1 : 0) + (sample ? 2 : 0);
   // all resident blocks, or L.trackBlocks per SM (fewer warps per SM can
-  // reuse L1 better: a tuning choice)
-  int b[4];
-  for (int i = 0; i < 4; ++i)
-    b[i] = L.trackBlocks ? std::max(1, std::min(g_trackBlocks[i], (int)L.trackBlocks * sm_count())) : g_trackBlocks[i];
-  switch (which) {
-    case 0: k_walk<false, false><<<b[0], 128, 0, s>>>(L); break;
-    case 1: k_walk<true, false><<<b[1], 128, 0, s>>>(L); break;
-    case 2: k_walk<false, true><<<b[2], 128, 0, s>>>(L); break;
-    default: k_walk<true, true><<<b[3], 128, 0, s>>>(L); break;
+  // raise the L1 hit rate of the grid lookups)
+  const auto blocks = [&](int resident) {
+    return L.trackBlocks ? std::max(1, std::min(resident, (int)L.trackBlocks * sm_count())) : resident;
+  };
+  for (int round = 0; round < (int)L.mediaRounds; ++round) {
+    if (sample) k_find<true><<<nblocks * 2, 128, 0, s>>>(L, round);
+    else k_find<false><<<nblocks * 2, 128, 0, s>>>(L, round);
+    kTrackVariants[which]<<<blocks(g_trackBlocks[which]), 128, 0, s>>>(L, round);
   }
+  kWalkVariants[which]<<<blocks(g_walkBlocks[which]), 128, 0, s>>>(L);
 }
 
 }  // namespace
@@ -1308,6 +1442,8 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
   if (L.trackSteps == 0) L.trackSteps = kDefaultTrackSteps;
   if (L.travVisits == 0) L.travVisits = kDefaultTravVisits;
   if (L.travRefill == 0) L.travRefill = kDefaultTravRefill;
+  if (L.mediaRounds == 0) L.mediaRounds = kDefaultMediaRounds;
+  if (L.wavePaths < 2 * kRoundPaths) L.mediaRounds = 0;
   query_track_blocks();
   const bool media = L.scene.nmedia > 0;
   int ev = 0, last[2] = {-1, -1};
@@ -1329,7 +1465,7 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
     L.bounce = b;
     if (media) {
       kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv)), kTraceWarps * 32, 0, s>>>(L);
-      launch_walk(L, true, s);
+      launch_media(L, true, nblocks, s);
       if (L.dda) k_collide<true><<<nblocks * 2, 128, 0, s>>>(L);
       else k_collide<false><<<nblocks * 2, 128, 0, s>>>(L);
       k_events<<<nblocks, 256, 0, s>>>(L);
@@ -1355,7 +1491,7 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
     R2_CUDA(cudaStreamWaitEvent(side.stream, side.fork, 0));
     mark(-1, true);
     kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, side.stream>>>(L);
-    if (media) launch_walk(L, false, side.stream);
+    if (media) launch_media(L, false, nblocks, side.stream);
     mark(3, true);
     k_accum<<<nblocks, 256, 0, side.stream>>>(L);
     mark(4, true);

@@ -74,8 +74,11 @@ struct PathState {
   uint32_t* mc;     // per-bounce media counters
   uint32_t* pj;     // per path: medium boundaries met in the bounce up to the segment it tracks
   uint32_t* cl;     // paths whose segment ended in a collision
-  float4* swP;      // shadow walk: next origin, transmittance so far
-  int2* swM;        // shadow walk: current medium, draw index of the slot's stream
+  float4* swP;      // shadow walk: origin of the segment it tracks, transmittance before it
+  int2* swM;        // shadow walk: medium of the segment, draw index of the slot's stream
+  float* swT;       // shadow walk: length of the segment
+  uint32_t* pq[2];  // queued rounds: paths with a segment to track, paths that go on after one
+  uint32_t* sq[2];  // the same of shadow slots
 };
 
 // Most wide BVH nodes the surface traversals stage in shared memory (20 KB per block).
@@ -88,16 +91,29 @@ constexpr uint32_t kDefaultTravRefill = 16;  // finished lanes that trigger a re
 // Paths per wave a frame's samples are grouped to.  A wave's later bounces hold
 // a few per cent of its paths, so larger waves keep the traversals' lanes and
 // the launches full: 64 samples of 1024x1024, 98.3 / 87.3 / 81.5 ms with 4M / 8M /
-// 16M paths (3.6 GB of state at 16M, 5.8 with media; 0.9 and 1.5 at 4M).  They are
+// 16M paths (3.6 GB of state at 16M, 6.3 with media; 0.9 and 1.6 at 4M).  They are
 // taken while memory is plenty (RenderContext::take_large); otherwise, and for
 // served jobs, which share the device, waves have kServeWavePaths.
 constexpr uint32_t kDefaultWavePaths = 1u << 24;
 constexpr uint32_t kServeWavePaths = 1u << 22;
-// media_rounds of a tuning, default and largest: accepted, without effect.
-constexpr uint32_t kDefaultMediaRounds = 2, kMaxMediaRounds = 32;
-// Media counters of a bounce (PathState::mc): paths and shadow slots taken by
-// k_walk, entries of the collision list.
-enum { kPathCounter = 0, kShadowCounter = 1, kCollideCounter = 2, kCountersPerBounce = 4 };
+// Queued rounds of medium boundaries (media_rounds of a tuning) in bounces of at
+// least kRoundPaths paths (shadow rays: events), of waves of at least twice as
+// many; k_walk alone takes the others, and what the rounds leave.  Frames with
+// rounds in bounces of 2^17 and more / of 2^18 / without: 256^3 foliage at 1920x1080,
+// 16 samples 228 / 227 / 278 ms; 24,000 trees, 4 samples 133 / 133 / 144; eight
+// 1080p volumes in one graph 560 / 567 / 707; 1,200 trees at 640x360, 4 samples
+// 19.1 / 19.7 / 19.9.  In waves below 2^18 paths the launches cost more than they
+// bring: 820x114, 2 samples 4.04 ms against 3.56, 191x439, 3 samples 7.9 against 7.2.
+// One round or two or four: 227 / 228 / 230 ms of the volume, 133 / 129 / 130 of the
+// trees, and in waves of 4M paths 314 / 327 of the volume.
+constexpr uint32_t kDefaultMediaRounds = 1, kMaxMediaRounds = 32;
+constexpr uint32_t kRoundPaths = 1u << 17;
+// Media counters of a bounce (PathState::mc): [3r] segments queued in round r,
+// [3r + 1] segments taken, [3r + 2] paths that go on, for paths and, from
+// kShadowCounters on, shadow slots; then paths and slots taken by k_walk, entries of
+// the collision list.
+constexpr int kShadowCounters = 3 * kMaxMediaRounds;
+enum { kPathCounter = 2 * kShadowCounters, kShadowCounter, kCollideCounter, kCountersPerBounce = kPathCounter + 4 };
 
 // PathState::counts layout: [0, 64) live paths per bounce, then two counters
 // per bounce (extension rays taken, shadow records taken), then the surface
@@ -136,6 +152,7 @@ struct RenderLaunch {
   uint32_t travVisits;  // BVH node steps a lane takes between refill checks of the surface kernels (tuning, >= 1)
   uint32_t travRefill;  // finished lanes of a warp that trigger a refill (tuning, 1..32)
   uint32_t trackBlocks; // persistent tracker blocks per SM (tuning; 0: every resident block)
+  uint32_t mediaRounds; // queued rounds of a bounce's medium boundaries (tuning; 0: the default)
   uint32_t trackLimit;  // steps of one tracking loop after which the path ends (1..kMaxTrackingSteps)
   uint32_t sortRays;    // surface scenes: reorder each bounce's rays by a coherence key before k_extend
   unsigned long long* stats;  // nullable: [0] path segments traced, [1] shadow rays traced

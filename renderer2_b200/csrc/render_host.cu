@@ -675,7 +675,7 @@ void RenderContext::ensure(uint32_t n, bool media) {
     const size_t m = n, m2 = 2 * m;
     reserve_together(mediaMem_, part(shX_, m2), part(evA_, m), part(evB_, m), part(evC_, m), part(evD_, m),
                      part(mc_, (size_t)kCountersPerBounce * 64), part(pj_, m), part(cl_, m), part(swP_, m2),
-                     part(swM_, m2));
+                     part(swM_, m2), part(swT_, m2), part(pq0_, m), part(pq1_, m), part(sq0_, m2), part(sq1_, m2));
     mediaCap_ = n;
   }
 }
@@ -716,8 +716,8 @@ size_t RenderContext::bytes_for(uint32_t n, bool media) {
   n = capacity_for(n);
   // per path: 5 float4 state + 3 x 2 float4 records + float4 throughput + 4 queue ids + 2 transmittances
   size_t b = (size_t)n * (5 * 16 + 6 * 16 + 16 + 16 + 8) + kCountsSize * 4;
-  // media: shadow tmax/medium, events (3 float4 + float2), two words and the walk state
-  if (media) b += (size_t)n * (16 + 48 + 8 + 8 + 32 + 16) + 16 * 64 * 4;
+  // media: shadow tmax/medium, events (3 float4 + float2), two words, the walk state and the rounds' queues
+  if (media) b += (size_t)n * (16 + 48 + 8 + 8 + 32 + 16 + 8 + 24) + (size_t)kCountersPerBounce * 64 * 4;
   return b + (size_t)n * 12;  // frame
 }
 
@@ -727,8 +727,11 @@ void RenderContext::release() {
   extra_ = 0;
   for (DBuf<float4>* b : {&rayO_, &rayD_, &T_, &L_, &hit_, &shO_, &shD_, &shPre_, &shT_, &evA_, &evB_, &evC_, &swP_})
     b->release();
-  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &counts_, &sortBins_, &mc_, &pj_, &cl_}) b->release();
+  for (DBuf<uint32_t>* b : {&q0_, &q1_, &qh_, &qs_, &counts_, &sortBins_, &mc_, &pj_, &cl_, &pq0_, &pq1_, &sq0_,
+                            &sq1_})
+    b->release();
   shTr_.release();
+  swT_.release();
   shX_.release();
   evD_.release();
   swM_.release();
@@ -746,7 +749,8 @@ void RenderContext::fill(PathState* st) const {
     st->shX = shX_.get();
     st->evA = evA_.get(); st->evB = evB_.get(); st->evC = evC_.get(); st->evD = evD_.get();
     st->mc = mc_.get(); st->pj = pj_.get(); st->cl = cl_.get();
-    st->swP = swP_.get(); st->swM = swM_.get();
+    st->swP = swP_.get(); st->swM = swM_.get(); st->swT = swT_.get();
+    st->pq[0] = pq0_.get(); st->pq[1] = pq1_.get(); st->sq[0] = sq0_.get(); st->sq[1] = sq1_.get();
   }
 }
 
@@ -809,6 +813,7 @@ RenderLaunch RenderScene::make_launch(const RenderContext& ctx, const r2_camera&
   L.trackSteps = tuning_.track_steps;
   L.travVisits = tuning_.trav_visits;
   L.travRefill = tuning_.trav_refill;
+  L.mediaRounds = tuning_.media_rounds;
   L.trackBlocks = tuning_.track_blocks;
   L.trackLimit = tuning_.track_limit ? tuning_.track_limit : (uint32_t)kMaxTrackingSteps;
   L.sortRays = media_.empty() && view_.hasTris && tuning_.sort_rays ? 1u : 0u;
@@ -993,6 +998,7 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
     static const uint32_t refills[] = {4, 8, 12, 24};
     static const uint32_t visits[] = {8, 16, 64, 256};
     static const uint32_t steps[] = {2, 4, 16, 32};
+    static const uint32_t rounds[] = {2, 4, 8};
     static const uint32_t trackBlocks[] = {2, 3, 4, 6};
     static const uint32_t sortRays[] = {1};
     sweep(&r2_render_tuning::wave_paths, wavePaths, 4);
@@ -1001,6 +1007,7 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
       sweep(&r2_render_tuning::trav_visits, visits, 4);
       sweep(&r2_render_tuning::sort_rays, sortRays, 1);
     } else {
+      sweep(&r2_render_tuning::media_rounds, rounds, 3);
       sweep(&r2_render_tuning::track_steps, steps, 4);
       sweep(&r2_render_tuning::track_blocks, trackBlocks, 4);
     }

@@ -76,9 +76,10 @@ class RenderContext {
   DBuf<float> shTr_;
   DBuf<float2> shX_, evD_;
   DBuf<float4> evA_, evB_, evC_;
-  DBuf<uint32_t> mc_, pj_, cl_;
+  DBuf<uint32_t> mc_, pj_, cl_, pq0_, pq1_, sq0_, sq1_;
   DBuf<float4> swP_;
   DBuf<int2> swM_;
+  DBuf<float> swT_;
 };
 
 class RenderScene {
