@@ -421,9 +421,10 @@ r2_status r2_scene_get_tuning(r2_scene* scene, r2_render_tuning* tuning);
  * scene's tuning (stats_out[4..7] of r2_render_device time one such wave). */
 r2_status r2_scene_wave_samples(r2_scene* scene, const r2_camera* camera, const r2_render_params* params,
                                 uint32_t* samples_out);
-/* Autotuner: times one wave of this frame for each candidate value of one
- * setting at a time (scenes without media: refill lanes, then visits; with
- * media: tracking steps), keeps a candidate that is faster by more than 2 %,
+/* Autotuner: times waves of this frame's first samples, the same samples for
+ * every setting, for each candidate value of one setting at a time (the paths
+ * per wave; scenes without media: refill lanes, visits, ray order; with media:
+ * queued rounds, tracking steps, tracker blocks), keeps a candidate that is faster by more than 2 %,
  * and stores the result as the scene's tuning (also written to tuning_out,
  * nullable).  Commits the scene if needed; waits. */
 r2_status r2_scene_autotune(r2_scene* scene, const r2_camera* camera, const r2_render_params* params,

@@ -108,6 +108,23 @@ constexpr uint32_t kServeWavePaths = 1u << 22;
 // trees, and in waves of 4M paths 314 / 327 of the volume.
 constexpr uint32_t kDefaultMediaRounds = 1, kMaxMediaRounds = 32;
 constexpr uint32_t kRoundPaths = 1u << 17;
+// What the tuner tries of each setting: the default among them (the current value
+// is not timed against itself), and the waves of served jobs.
+constexpr uint32_t kTuneWavePaths[] = {1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24};
+constexpr uint32_t kTuneTravRefill[] = {4, 8, 12, 16, 24}, kTuneTravVisits[] = {8, 16, 32, 64, 256};
+constexpr uint32_t kTuneTrackSteps[] = {2, 4, 8, 16, 32}, kTuneMediaRounds[] = {1, 2, 4, 8};
+constexpr uint32_t kTuneTrackBlocks[] = {0, 2, 3, 4, 6}, kTuneSortRays[] = {0, 1};
+template <size_t N>
+constexpr bool tunes(const uint32_t (&values)[N], uint32_t value) {
+  for (uint32_t v : values)
+    if (v == value) return true;
+  return false;
+}
+static_assert(tunes(kTuneWavePaths, kDefaultWavePaths) && tunes(kTuneWavePaths, kServeWavePaths) &&
+                  tunes(kTuneTravRefill, kDefaultTravRefill) && tunes(kTuneTravVisits, kDefaultTravVisits) &&
+                  tunes(kTuneTrackSteps, kDefaultTrackSteps) && tunes(kTuneMediaRounds, kDefaultMediaRounds),
+              "a default left the tuner's lists when it changed");
+
 // Media counters of a bounce (PathState::mc): [3r] segments queued in round r,
 // [3r + 1] segments taken, [3r + 2] paths that go on, for paths and, from
 // kShadowCounters on, shadow slots; then paths and slots taken by k_walk, entries of

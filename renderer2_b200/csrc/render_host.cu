@@ -944,24 +944,28 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
   cudaStream_t s = ctx.stream;
   prepare_render_launches();
   const r2_render_tuning saved = tuning_;
-  // milliseconds per path of the frame's first wave under tuning t, the faster of two runs
-  auto time_wave = [&](const r2_render_tuning& t) {
+  // milliseconds per path of the frame's first samples under tuning t, the faster of two runs.  As many samples for
+  // waves of every size as the largest wave has: one sample can lack the few slow paths that set a wave's time.
+  uint32_t span = 1;
+  auto time_waves = [&](const r2_render_tuning& t) {
     tuning_ = t;
-    const uint32_t S = wave_spp(npix, p.spp);
+    const uint32_t S = wave_spp(npix, p.spp), waves = (span + S - 1) / S;
     RenderLaunch L = prepare(ctx, c, p, frame.get(), S);
     L.sampleDev = nullptr;
-    L.sample = 0;
     float best = 1e30f;
     for (int rep = 0; rep < 2; ++rep) {
       R2_CUDA(cudaEventRecord(ctx.ev0, s));
-      launch_render_wave(L, wave_blocks(npix * S), s, ctx.side);
+      for (uint32_t w = 0; w < waves; ++w) {
+        L.sample = w * S;
+        launch_render_wave(L, wave_blocks(npix * S), s, ctx.side);
+      }
       R2_CUDA(cudaEventRecord(ctx.ev1, s));
       R2_CUDA(cudaEventSynchronize(ctx.ev1));
       float ms = 0.0f;
       R2_CUDA(cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1));
       best = std::min(best, ms);
     }
-    return best / ((float)S * (float)npix);
+    return best / ((float)(S * waves) * (float)npix);
   };
   r2_render_tuning cur{kDefaultTrackSteps, kDefaultTravVisits, kDefaultTravRefill, kDefaultWavePaths,
                        kDefaultMediaRounds, 0, saved.track_limit, 0, 0};  // the step bound is kept, never tuned
@@ -974,42 +978,36 @@ r2_render_tuning RenderScene::autotune(const r2_camera& c, const r2_render_param
   try {
     if (!room(cur.wave_paths)) cur.wave_paths = kServeWavePaths;
     R2_CUDA(cudaMemsetAsync(ctx.bound.get(), 0, sizeof(unsigned int), s));
-    time_wave(cur);  // warm-up
-    float curT = time_wave(cur);
-    auto sweep = [&](uint32_t r2_render_tuning::*field, const uint32_t* cand, int n) {
+    for (uint32_t paths : kTuneWavePaths)
+      if (room(paths)) span = std::max(span, wave_spp_of(paths, npix, p.spp));
+    time_waves(cur);  // warm-up
+    float curT = time_waves(cur);
+    auto sweep = [&](uint32_t r2_render_tuning::*field, const auto& cand) {
       const r2_render_tuning base = cur;
-      for (int i = 0; i < n; ++i) {
+      for (uint32_t value : cand) {
+        if (value == base.*field) continue;
         r2_render_tuning t = base;
-        t.*field = cand[i];
+        t.*field = value;
         if (field == &r2_render_tuning::wave_paths) {  // skip settings that give the same waves
-          tuning_ = t;
-          const uint32_t S = wave_spp(npix, p.spp);
-          tuning_ = cur;
-          if (S == wave_spp(npix, p.spp) || !room(cand[i])) continue;
+          const uint32_t S = wave_spp_of(value, npix, p.spp);
+          if (S == wave_spp_of(cur.wave_paths, npix, p.spp) || !room(value)) continue;
         }
-        const float ms = time_wave(t);
+        const float ms = time_waves(t);
         if (ms < curT * 0.98f) {
           cur = t;
           curT = ms;
         }
       }
     };
-    static const uint32_t wavePaths[] = {1u << 20, 1u << 21, 1u << 23, 1u << 24};
-    static const uint32_t refills[] = {4, 8, 12, 24};
-    static const uint32_t visits[] = {8, 16, 64, 256};
-    static const uint32_t steps[] = {2, 4, 16, 32};
-    static const uint32_t rounds[] = {2, 4, 8};
-    static const uint32_t trackBlocks[] = {2, 3, 4, 6};
-    static const uint32_t sortRays[] = {1};
-    sweep(&r2_render_tuning::wave_paths, wavePaths, 4);
+    sweep(&r2_render_tuning::wave_paths, kTuneWavePaths);
     if (media_.empty()) {  // the persistent surface traversals run in scenes without media
-      sweep(&r2_render_tuning::trav_refill, refills, 4);
-      sweep(&r2_render_tuning::trav_visits, visits, 4);
-      sweep(&r2_render_tuning::sort_rays, sortRays, 1);
+      sweep(&r2_render_tuning::trav_refill, kTuneTravRefill);
+      sweep(&r2_render_tuning::trav_visits, kTuneTravVisits);
+      sweep(&r2_render_tuning::sort_rays, kTuneSortRays);
     } else {
-      sweep(&r2_render_tuning::media_rounds, rounds, 3);
-      sweep(&r2_render_tuning::track_steps, steps, 4);
-      sweep(&r2_render_tuning::track_blocks, trackBlocks, 4);
+      sweep(&r2_render_tuning::media_rounds, kTuneMediaRounds);
+      sweep(&r2_render_tuning::track_steps, kTuneTrackSteps);
+      sweep(&r2_render_tuning::track_blocks, kTuneTrackBlocks);
     }
   } catch (...) {
     tuning_ = saved;

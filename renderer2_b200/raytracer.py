@@ -214,7 +214,7 @@ class Scene:
         return n.value
 
     def autotune(self, cam: Camera, prm: RenderParams) -> Tuning:
-        """Times one wave of this frame per candidate setting and keeps the fastest (see r2_scene_autotune)."""
+        """Times waves of this frame per candidate setting and keeps the fastest (see r2_scene_autotune)."""
         t = Tuning()
         N.check(N.lib.r2_scene_autotune(self.handle, C.byref(cam), C.byref(prm), C.byref(t)))
         return t
