@@ -9,6 +9,9 @@
 
 namespace r2 {
 
+// Words of a filter job's work space.
+static size_t filter_work(size_t nvox) { return std::max(nvox, kFilterMinWork); }
+
 // Bytes of a buffer grown to a power of two (DBuf::reserve_grow).
 static size_t grow_bytes(size_t n) {
   size_t c = 1;
@@ -100,7 +103,7 @@ uint64_t Server::submit(std::unique_ptr<ServerJob> job) {
     const size_t nvox = (size_t)j->grid.num_voxels[0] * j->grid.num_voxels[1] * j->grid.num_voxels[2];
     R2_REQUIRE(nvox > 0 && nvox < (1ull << 32), R2_ERR_INVALID_ARGUMENT, "bad filter grid");
     j->outBytes = nvox * sizeof(r2_voxel);
-    j->bytes = grow_bytes(nvox * sizeof(r2_voxel)) + grow_bytes(nvox * 4) + 64;
+    j->bytes = grow_bytes(nvox * sizeof(r2_voxel)) + grow_bytes(filter_work(nvox) * 4) + 64;
   }
   R2_REQUIRE(j->bytes <= budget_, R2_ERR_ADMISSION_REJECTED, "job needs more device memory than the HBM budget");
   uint64_t id;
@@ -157,7 +160,7 @@ bool Server::start(Slot& s, ServerJob* j) {
     } else {
       const size_t nvox = (size_t)j->grid.num_voxels[0] * j->grid.num_voxels[1] * j->grid.num_voxels[2];
       s.vox.reserve_grow(nvox);
-      s.work.reserve_grow(std::max(nvox, kFilterMinWork));
+      s.work.reserve_grow(filter_work(nvox));
       s.counters.reserve(kFilterCounters);
       j->fscene->run(j->grid, j->fp, j->lod, s.vox.get(), nullptr, nullptr, st, nullptr, s.work.get(),
                      s.work.size(), s.counters.get());

@@ -95,3 +95,26 @@ def test_a_failed_allocation_fails_one_call():
         del held
         torch.cuda.empty_cache()
         sc.close()
+
+
+def test_a_filter_job_is_admitted_with_the_work_space_it_takes():
+    """A job of few voxels takes 256 KB to work in: a budget without room for that does not admit it."""
+    from renderer2_b200 import _native as N
+    from renderer2_b200 import filter as F
+    from renderer2_b200 import scenes
+    from renderer2_b200 import serving as S
+    mesh = scenes.icosphere(2, 0.05, 1)
+    sc = F.FilterScene(mesh, F.material())
+    g = sc.grid(scenes.voxel_size_for(mesh, 8))
+    nvox = int(np.prod(np.array(g.num_voxels[:], np.int64)))
+    out = 32 * (1 << (nvox - 1).bit_length())
+    for budget, fits in ((out + (1 << 18) + 64, True), (out + (1 << 17), False)):
+        srv = S.Server(1, budget)
+        if fits:
+            srv.wait(srv.submit_filter(sc, g, F.params(samples_per_voxel=8, iterations=2)))
+        else:
+            with pytest.raises(N.R2Error) as e:
+                srv.submit_filter(sc, g, F.params(samples_per_voxel=8, iterations=2))
+            assert e.value.name == "R2_ERR_ADMISSION_REJECTED"
+        srv.close()
+    sc.close()
