@@ -237,7 +237,7 @@ R2_HD bool trace_all_have_leaf(bool mine) {
 }
 
 // Visits about maxVisits nodes and triangles; true when the query has
-// finished (closest hit in (0, tmax], kAnyHit: the first hit found) with
+// finished (closest hit in (0, tmax]) with
 // s.best.tri the BVH-order index, -1 on a miss.  Speculative while-while
 // traversal (Aila and Laine, "Understanding the Efficiency of Ray Traversal on
 // GPUs", HPG 2009): inner nodes are visited until every lane of the warp has
@@ -254,7 +254,7 @@ R2_HD bool trace_all_have_leaf(bool mine) {
 // leaf of the instance has been tested.  The stack then holds the top-level
 // path, the marker and the instance's path: the builder bounds the sum of the
 // two heights plus two by R2_BVH_STACK.
-template <bool kAnyHit, bool kCount = false, bool kAlpha = false, bool kInst = false>
+template <bool kCount = false, bool kAlpha = false, bool kInst = false>
 R2_HD bool trace_advance(const BvhView& bvh, TraceState& s, int* stack, float* stackT, int maxVisits) {
   int budget = maxVisits;
   while (budget > 0) {
@@ -347,11 +347,6 @@ R2_HD bool trace_advance(const BvhView& bvh, TraceState& s, int* stack, float* s
         if (tri_test<kAlpha>(s.r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), tri,
                              kInst ? tri + s.vdelta : tri, &s.best, &bvh.alpha)) {
           s.found = 1;
-          if (kAnyHit) {
-            s.leaf = 0;
-            s.cur = kTraceDone;
-            return true;
-          }
         }
       }
       s.leaf = 0;
@@ -368,33 +363,26 @@ R2_HD bool trace_advance(const BvhView& bvh, TraceState& s, int* stack, float* s
   return false;
 }
 
-// The whole query at once; the counting instantiation adds the inner nodes
-// visited and the triangles tested to *nodes and *tris.
-template <bool kAnyHit, bool kCount = false>
-R2_HD Hit bvh_trace(const BvhView& bvh, V3 o, V3 d, float tmax, uint32_t* nodes = nullptr,
-                    uint32_t* tris = nullptr, int root = 0) {
+// The whole query at once.
+R2_HD Hit bvh_trace(const BvhView& bvh, V3 o, V3 d, float tmax) {
   TraceState s;
-  trace_begin(s, o, d, tmax, root);
+  trace_begin(s, o, d, tmax);
   int stack[R2_BVH_STACK];
   float stackT[R2_BVH_STACK];
   if (bvh.inst) {
     if (bvh.alpha.alphaTex) {
-      while (!trace_advance<kAnyHit, kCount, true, true>(bvh, s, stack, stackT, 1 << 30)) {
+      while (!trace_advance<false, true, true>(bvh, s, stack, stackT, 1 << 30)) {
       }
     } else {
-      while (!trace_advance<kAnyHit, kCount, false, true>(bvh, s, stack, stackT, 1 << 30)) {
+      while (!trace_advance<false, false, true>(bvh, s, stack, stackT, 1 << 30)) {
       }
     }
   } else if (bvh.alpha.alphaTex) {
-    while (!trace_advance<kAnyHit, kCount, true>(bvh, s, stack, stackT, 1 << 30)) {
+    while (!trace_advance<false, true>(bvh, s, stack, stackT, 1 << 30)) {
     }
   } else {
-    while (!trace_advance<kAnyHit, kCount, false>(bvh, s, stack, stackT, 1 << 30)) {
+    while (!trace_advance(bvh, s, stack, stackT, 1 << 30)) {
     }
-  }
-  if (kCount) {
-    *nodes += s.nodes;
-    *tris += s.tris;
   }
   return s.best;
 }

@@ -630,7 +630,7 @@ __device__ Hit trace_bvh(const BvhView& bvh, V3 o, V3 d, float tmax, int root, u
   trace_begin(s, o, d, tmax, root);
   int stack[R2_BVH_STACK];
   float stackT[R2_BVH_STACK];
-  while (!trace_advance<false, kCount, kAlpha>(bvh, s, stack, stackT, 1 << 30)) {
+  while (!trace_advance<kCount, kAlpha>(bvh, s, stack, stackT, 1 << 30)) {
   }
   if (kCount) {
     *nodes += s.nodes;
@@ -639,8 +639,10 @@ __device__ Hit trace_bvh(const BvhView& bvh, V3 o, V3 d, float tmax, int root, u
   return s.best;
 }
 
-// Writes a voxel's record w (the wide layout, in shared memory): its 32-byte
-// payload (encode_voxel, a field per lane; tmp: 8 words of shared memory), the
+// Writes a voxel's record w (the wide layout, in shared memory: [0] density,
+// [1..6] Sxx Syy Szz Sxy Sxz Syz, [7..9] diffuse, [10..12] specular, [13..15] normal,
+// [16] ior): its 32-byte payload (SFilteredDataCompact(const SFilteredData&),
+// filtered_data.hpp:91-107, a field per lane; tmp: 8 words of shared memory), the
 // wide record and the FP16 payload.
 __device__ __forceinline__ void write_record(const FilterLaunch& L, uint32_t vid, const float* w, uint32_t* tmp,
                                              int lane) {

@@ -87,33 +87,6 @@ R2_HD uint8_t to_u8(float v) {
   return (uint8_t)v;
 }
 
-// SFilteredDataCompact(const SFilteredData&) (filtered_data.hpp:91-107) from
-// the wide record: [0] density, [1..6] Sxx Syy Szz Sxy Sxz Syz, [7..9] diffuse,
-// [10..12] specular, [13..15] normal, [16] ior.
-R2_HD r2_voxel encode_voxel(const float* w) {
-  const float M16 = 65535.0f, M8 = 255.0f;
-  r2_voxel v;
-  v.density = w[0];
-  float sxx = w[1], syy = w[2], szz = w[3], sxy = w[4], sxz = w[5], syz = w[6];
-  v.sigma_x = to_u16(clampf(M16 * sqrtf(sxx), 0.0f, M16));
-  v.sigma_y = to_u16(clampf(M16 * sqrtf(syy), 0.0f, M16));
-  v.sigma_z = to_u16(clampf(M16 * sqrtf(szz), 0.0f, M16));
-  v.r_xy = to_u16(clampf(M16 * 0.5f * (sxy / sqrtf(sxx * syy) + 1.0f), 0.0f, M16));
-  v.r_xz = to_u16(clampf(M16 * 0.5f * (sxz / sqrtf(sxx * szz) + 1.0f), 0.0f, M16));
-  v.r_yz = to_u16(clampf(M16 * 0.5f * (syz / sqrtf(syy * szz) + 1.0f), 0.0f, M16));
-  for (int k = 0; k < 3; ++k) {
-    v.diffuse[k] = to_u8(clampf(M8 * w[7 + k], 0.0f, M8));
-    v.specular[k] = to_u8(clampf(M8 * w[10 + k], 0.0f, M8));
-  }
-  V3 n = normalize(v3(w[13], w[14], w[15]));  // SFilteredData::n()
-  v.normal[0] = to_u16(clampf(M16 * 0.5f * (n.x + 1.0f), 0.0f, M16));
-  v.normal[1] = to_u16(clampf(M16 * 0.5f * (n.y + 1.0f), 0.0f, M16));
-  v.normal[2] = to_u16(clampf(M16 * 0.5f * (n.z + 1.0f), 0.0f, M16));
-  v.ior = f32_to_f16_bits(w[16]);
-  v.pad = 0;
-  return v;
-}
-
 // Eigendecomposition of the symmetric 3x3 matrix S (xx yy zz xy xz yz) in
 // double precision by cyclic Jacobi rotations (Jacobi 1846; Golub and Van
 // Loan, Matrix Computations, 4th ed., section 8.5): S = V diag(w) V^T with

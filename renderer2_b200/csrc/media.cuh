@@ -362,156 +362,6 @@ R2_HD void fill_event(MediumEvent* ev, const Ray& w, const FData& fd) {
 
 R2_HD float inv_majorant(const MediumView& m) { return 1.0f / (m.filterRenderRatio / m.invMaxDensity); }
 
-// CNVDBMedium::sampleInternal (delta tracking against the global majorant),
-// model-space ray; *err is set when `limit` steps are reached.
-R2_HD V3 medium_sample_internal(const MediumView& m, const Ray& rayModel, RngStream& rng, MediumEvent* ev, int* err,
-                                int limit) {
-  Ray ray = ray_transform2(rayModel, m.modelToIndex);
-  const float invMax = inv_majorant(m);
-  if (!(invMax < INFINITY)) return v3(1.0f);  // empty grid: no collision possible
-  float t = 0.0f;
-  for (int it = 0; it < limit; ++it) {
-    t -= log_r2(1.0f - rng.next()) * invMax / m.sigmaT;
-    if (t >= ray.tmax) return v3(1.0f);
-    const V3 pt = ray.o + ray.d * t;
-    if (m.filterRenderRatio * medium_density(m, pt) * invMax > rng.next()) {
-      const FData fd = medium_filtered(m, pt);
-      ray.tmax = t;
-      const Ray w = ray_transform2(ray, m.indexToModel);
-      fill_event(ev, w, fd);
-      return scatter_albedo(m, fd, w.d);
-    }
-  }
-  *err = 1;
-  return v3(0.0f);
-}
-
-// CNVDBMedium::sampleDDA (brick-grid majorants; mip starts at 3, +0.25 per
-// step, -2 after a tentative collision).
-R2_HD V3 medium_sample_dda(const MediumView& m, const Ray& rayModel, RngStream& rng, MediumEvent* ev, int* err,
-                           int limit) {
-  Ray iray = ray_transform2(rayModel, m.unitToScaled);
-  const V3 ri = v3(1.0f / iray.d.x, 1.0f / iray.d.y, 1.0f / iray.d.z);
-  float t = 0.0f;
-  float tau = -log_r2(1.0f - rng.next());
-  float mip = 3.0f;
-  for (int it = 0; it < limit; ++it) {
-    if (!(t < iray.tmax)) return v3(1.0f);
-    const V3 curr = iray.o + iray.d * t;
-    const int mi = (int)roundf(mip);
-    const float majorant = m.filterRenderRatio * brick_majorant(m, curr, mi);
-    const float dt = step_dda(curr, ri, mi);
-    const float prevT = t;
-    t += dt / m.sigmaT;
-    if (t == prevT) return v3(1.0f);
-    tau -= majorant * dt;
-    mip = fminf(mip + 0.25f, 3.0f);
-    if (tau > 0.0f) continue;
-    t += tau / (majorant * m.sigmaT);
-    if (t >= iray.tmax) return v3(1.0f);
-    const float jx = rng.next();
-    const float jy = rng.next();
-    const float jz = rng.next();
-    const float d = brick_density(m, iray.o + iray.d * t + v3(jx, jy, jz) - v3(0.5f));
-    if (rng.next() * majorant < d * m.filterRenderRatio) {
-      iray.tmax = t;
-      const V3 ip = iray.o + iray.d * t;
-      const V3 pos = v3((ip.x - (float)m.ibbMin[0]) / (float)m.size[0], (ip.y - (float)m.ibbMin[1]) / (float)m.size[1],
-                        (ip.z - (float)m.ibbMin[2]) / (float)m.size[2]);
-      const FData fd = medium_filtered(m, pos);
-      const Ray w = ray_transform2(iray, m.scaledToModel);
-      fill_event(ev, w, fd);
-      return scatter_albedo(m, fd, w.d);
-    }
-    tau = -log_r2(1.0f - rng.next());
-    mip = fmaxf(0.0f, mip - 2.0f);
-  }
-  *err = 1;
-  return v3(0.0f);
-}
-
-// CNVDBMedium::trInternal (ratio tracking with Russian roulette).
-R2_HD float medium_tr_internal(const MediumView& m, const Ray& rayModel, RngStream& rng, int* err, int limit) {
-  const Ray ray = ray_transform2(rayModel, m.modelToIndex);
-  const float invMax = inv_majorant(m);
-  if (!(invMax < INFINITY)) return 1.0f;
-  float tr = 1.0f, t = 0.0f;
-  for (int it = 0; it < limit; ++it) {
-    t -= log_r2(1.0f - rng.next()) * invMax / m.sigmaT;
-    if (t >= ray.tmax) return tr;
-    const float d = medium_density(m, ray.o + ray.d * t);
-    tr *= 1.0f - fmaxf(0.0f, m.filterRenderRatio * d * invMax);
-    if (tr < 1.0f) {
-      const float p = 1.0f - tr;
-      if (rng.next() < p) return 0.0f;
-      tr /= 1.0f - p;
-    }
-  }
-  *err = 1;
-  return 0.0f;
-}
-
-// CNVDBMedium::trDDA.
-R2_HD float medium_tr_dda(const MediumView& m, const Ray& rayModel, RngStream& rng, int* err, int limit) {
-  const Ray iray = ray_transform2(rayModel, m.unitToScaled);
-  const V3 ri = v3(1.0f / iray.d.x, 1.0f / iray.d.y, 1.0f / iray.d.z);
-  float tr = 1.0f, t = 0.0f;
-  const float volMajorant = 1.0f / inv_majorant(m);
-  float tau = -log_r2(1.0f - rng.next());
-  float mip = 3.0f;
-  for (int it = 0; it < limit; ++it) {
-    if (!(t < iray.tmax)) return tr;
-    const V3 curr = iray.o + iray.d * t;
-    const int mi = (int)roundf(mip);
-    const float majorant = m.filterRenderRatio * brick_majorant(m, curr, mi);
-    const float dt = step_dda(curr, ri, mi);
-    const float prevT = t;
-    t += dt / m.sigmaT;
-    if (t == prevT) return tr;
-    tau -= majorant * dt;
-    mip = fminf(mip + 0.25f, 3.0f);
-    if (tau > 0.0f) continue;
-    t += tau / (majorant * m.sigmaT);
-    if (t >= iray.tmax) return tr;
-    const float jx = rng.next();
-    const float jy = rng.next();
-    const float jz = rng.next();
-    const float d = brick_density(m, iray.o + iray.d * t + v3(jx, jy, jz) - v3(0.5f));
-    if (rng.next() * majorant < d * m.filterRenderRatio) {
-      tr *= fmaxf(0.0f, 1.0f - volMajorant / majorant);
-      if (tr < 0.1f) {
-        const float prob = 1.0f - tr;
-        if (rng.next() < prob) return 0.0f;
-        tr /= 1.0f - prob;
-      }
-    }
-    tau = -log_r2(1.0f - rng.next());
-    mip = fmaxf(0.0f, mip - 2.0f);
-  }
-  *err = 1;
-  return 0.0f;
-}
-
-// CMediumInstance::sample: world-space ray; returns the albedo weight (1 when
-// the ray passes) and, on a collision, the event in world space.
-R2_HD V3 instance_sample(const MediumView& m, const Ray& rayWorld, bool dda, RngStream& rng, MediumEvent* ev, int* err,
-                         int limit) {
-  const Ray rm = ray_transform2(rayWorld, m.worldToModel);
-  ev->hit = 0;
-  const V3 a = dda ? medium_sample_dda(m, rm, rng, ev, err, limit) : medium_sample_internal(m, rm, rng, ev, err, limit);
-  if (ev->hit) {
-    ev->pos = xform_point(m.modelToWorld, ev->pos);
-    ev->normal = normalize(xform_vector(m.modelToWorld, ev->normal));
-  }
-  return a;
-}
-
-// CMediumInstance::tr.
-R2_HD float instance_tr(const MediumView& m, const Ray& rayWorld, bool dda, RngStream& rng, int* err, int limit) {
-  const Ray rm = ray_transform2(rayWorld, m.worldToModel);
-  return dda ? medium_tr_dda(m, rm, rng, err, limit) : medium_tr_internal(m, rm, rng, err, limit);
-}
-
 // CNVDBMedium::moveToVoxelBorder (model space): the origin moves to just
 // before the exit of its voxel.
 R2_HD Ray medium_move_to_voxel_border(const MediumView& m, const Ray& rayModel) {

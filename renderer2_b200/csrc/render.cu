@@ -216,7 +216,7 @@ __device__ __forceinline__ float4 surface_closest_after(const SceneView& S, V3 o
 __device__ __forceinline__ float4 surface_closest(const SceneView& S, V3 o, V3 d, float tmax) {
   Hit h;
   h.tri = -1;
-  if (S.hasTris) h = bvh_trace<false>(S.bvh, o, d, tmax);
+  if (S.hasTris) h = bvh_trace(S.bvh, o, d, tmax);
   return surface_closest_after(S, o, d, tmax, h);
 }
 

@@ -314,7 +314,7 @@ void RenderScene::rebuild(cudaStream_t s) {
   builder_.build(dPos_.get(), dIdx_.get(), nt, &bvh_, s);
   bvhNodes_ = bvh_.nnodes;
   bvhHeight_ = bvh_.height;
-  wide_.build(bvh_.nodes.get(), bvh_.tris.get(), nullptr, 1, nt, s);
+  wide_.build(bvh_.nodes.get(), nullptr, 1, nt, s);
   buildLaunches_ = builder_.launches() + WideBvh::kLaunches + 1;
   k_gather_shading<<<(nt + 255) / 256, 256, 0, s>>>(bvh_.order.get(), nt, dIdx_.get(), dNrm_.get(), dTriMatIn_.get(),
                                                     anyUV_ ? dUV_.get() : nullptr, dTriAlphaIn_.get(), triN_.get(),
@@ -495,7 +495,7 @@ void RenderScene::build_two_level(cudaStream_t s) {
     launches += 2;
   }
   R2_CUDA(cudaGetLastError());
-  wide_.build(gNodes_.get(), gTris_.get(), roots.data(), (uint32_t)roots.size(), (uint32_t)(totalTris + ninst), s);
+  wide_.build(gNodes_.get(), roots.data(), (uint32_t)roots.size(), (uint32_t)(totalTris + ninst), s);
   launches += WideBvh::kLaunches;
   view_.wide = wide_.view();
   const BvhAlpha alpha = view_.bvh.alpha;

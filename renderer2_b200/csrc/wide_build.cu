@@ -23,7 +23,6 @@ enum { kWideNodes = 0, kWideDone = 1, kWideRange = 2, kWideState = kWideRange + 
 
 struct WideBuild {
   const BvhNode* nodes;
-  const float4* tris;
   uint4* out;
   uint32_t* queue;
   uint32_t* state;
@@ -181,14 +180,14 @@ __global__ void __launch_bounds__(64) k_wide_rest(WideBuild B) {
 
 }  // namespace
 
-void WideBvh::build(const BvhNode* nodes, const float4* tris, const uint32_t* roots, uint32_t nroots, uint32_t nleaves,
+void WideBvh::build(const BvhNode* nodes, const uint32_t* roots, uint32_t nroots, uint32_t nleaves,
                     cudaStream_t s) {
   const size_t cap = wide_capacity(nleaves, nroots);
   reserve_together(mem_, part(nodes_, cap * kWideWords), part(queue_, cap), part(state_, kWideState));
   R2_CUDA(cudaMemsetAsync(state_.get(), 0, kWideState * sizeof(uint32_t), s));
   if (roots) R2_CUDA(cudaMemcpyAsync(queue_.get(), roots, nroots * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   else R2_CUDA(cudaMemsetAsync(queue_.get(), 0, sizeof(uint32_t), s));
-  const WideBuild B = {nodes, tris, nodes_.get(), queue_.get(), state_.get()};
+  const WideBuild B = {nodes, nodes_.get(), queue_.get(), state_.get()};
   k_wide_top<<<1, kTopThreads, 0, s>>>(B, nroots);
   const int blocks = sm_count() * 4;
   for (int level = 0; level < kLevels; ++level) k_wide_level<<<blocks, 64, 0, s>>>(B, level);

@@ -101,10 +101,9 @@ R2_HD size_t wide_capacity(uint32_t nleaves, uint32_t nroots) { return (size_t)n
 class WideBvh {
  public:
   // nodes: binary nodes, trees below roots[0 .. nroots-1] (host; null: one
-  // root, node 0) with at most nleaves leaves in all; tris: their triangles.
+  // root, node 0) with at most nleaves leaves in all.
   // Wide node i < nroots is the root of tree i.  Asynchronous on s.
-  void build(const BvhNode* nodes, const float4* tris, const uint32_t* roots, uint32_t nroots, uint32_t nleaves,
-             cudaStream_t s);
+  void build(const BvhNode* nodes, const uint32_t* roots, uint32_t nroots, uint32_t nleaves, cudaStream_t s);
   WideView view() const { return WideView{nodes_.get()}; }
   static constexpr int kLaunches = 5;  // kernels of a build
 

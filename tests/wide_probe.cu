@@ -65,7 +65,7 @@ __global__ void k_wide(BvhView bvh, WideView wide, const Ray* rays, uint32_t n, 
 
 __global__ void k_binary(BvhView bvh, const Ray* rays, uint32_t n, float4* closest) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const Hit h = bvh_trace<false>(bvh, v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]),
+    const Hit h = bvh_trace(bvh, v3(rays[k].o[0], rays[k].o[1], rays[k].o[2]),
                                    v3(rays[k].d[0], rays[k].d[1], rays[k].d[2]), rays[k].tmax);
     closest[k] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.tri));
   }
@@ -185,7 +185,7 @@ int probe_trace(const float* pos, uint32_t nverts, const uint32_t* idx, uint32_t
     DeviceBvh bvh;
     builder.build(dpos.get(), didx.get(), ntris, &bvh, s);
     WideBvh wide;
-    wide.build(bvh.nodes.get(), bvh.tris.get(), nullptr, 1, ntris, s);
+    wide.build(bvh.nodes.get(), nullptr, 1, ntris, s);
     R2_CUDA(cudaMemsetAsync(taken.get(), 0, 2 * sizeof(uint32_t), s));
     R2_CUDA(cudaMemsetAsync(bound.get(), 0, sizeof(unsigned int), s));
     k_wide<<<sm_count() * 4, 128, 0, s>>>(bvh.view(), wide.view(), drays.get(), n, taken.get(), bound.get(), a.get(),
