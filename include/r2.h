@@ -179,8 +179,9 @@ r2_status r2_filter_scene_grid(const r2_filter_scene* scene, float voxel_size,
 /* Filter one LOD into device memory.  d_out: nx*ny*nz r2_voxel; d_wide
  * (nullable): 20 floats per voxel; d_fp16 (nullable): 8 halves per voxel
  * (density, Sxx, Syy, Szz, Sxy, Sxz, Syz, 0).  stream: cudaStream_t or NULL.
- * stats_out (nullable, host): [0]=voxels, [1]=voxels with candidate geometry,
- * [2]=device milliseconds of the filter's kernels. */
+ * stats_out (nullable, host): [0]=voxels, [1]=voxels with a triangle
+ * within reach of their rays (by a ball about the voxel, so a few of them have none
+ * that a ray could hit), [2]=device milliseconds of the filter's kernels. */
 r2_status r2_filter_scene_run(r2_filter_scene* scene, const r2_filter_grid* grid,
                               const r2_filter_params* params, r2_voxel* d_out, float* d_wide,
                               uint16_t* d_fp16, void* stream, double* stats_out);
@@ -400,11 +401,12 @@ r2_status r2_scene_set_vertices(r2_scene* scene, const float* positions, const f
 /* Renders one frame into device memory d_rgb (width*height*3 floats).
  * stats_out (nullable, 8 doubles): [0] paths, [1] milliseconds of the frame on
  * the stream, [2] path segments traced, [3] shadow rays traced, [4..7]
- * milliseconds of the extend / shade / shadow / accumulate kernels (a bounce's
- * shadow rays overlap the next one's extension) of one (the middle) wave, which renders r2_scene_wave_samples samples of every
- * pixel.  With stats_out the call waits for the frame and returns
+ * milliseconds of the extend / shade / shadow / accumulate stages of one (the
+ * middle) wave, which renders r2_scene_wave_samples samples of every pixel (a
+ * bounce's shadow rays overlap the next one's extension, so these two contain
+ * each other's work).  With stats_out the call waits for the frame and returns
  * R2_ERR_DEVICE_TIMEOUT (frame still written) if a loop bound ended any path:
- * 2^20 tracking steps, 64 medium boundaries within a bounce, 256 along a
+ * 2^20 tracking steps, 4096 medium boundaries within a bounce or along a
  * shadow ray (the reference's loops have no bound). */
 r2_status r2_render_device(r2_scene* scene, const r2_camera* camera, const r2_render_params* params, float* d_rgb,
                            void* stream, double* stats_out);

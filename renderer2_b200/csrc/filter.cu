@@ -25,7 +25,7 @@
 // walked the BVH by itself, a node at a time, inside the sampling kernel and
 // tested the triangles whose boxes overlap the ball's box (8.5 per ray over
 // 12.0M voxels); with the ball test, the lists and the smaller kernel (4.6 per
-// ray over 6.5M voxels) it takes 103 ms, 16 of them for the lists.
+// ray over 6.5M voxels) it takes 95 ms, 16 of them for the lists.
 #include "filter.cuh"
 #include "filter_math.h"
 #include "texture_shade.cuh"

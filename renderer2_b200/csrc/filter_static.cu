@@ -11,7 +11,8 @@
 // (BVH, shading data) is created beforehand, when allocation is allowed.
 //
 // The scratch is kStaticMaxVoxels words (4 MiB) and the counters; a grid of
-// that many voxels is worked off in six parts.  Every GPU that loads the library keeps it until the process ends.
+// that many voxels is worked off in seven parts.  Every GPU that loads the
+// library keeps it until the process ends.
 // Larger grids are rejected with R2_ERR_UNSUPPORTED.  All calls share the one
 // array: calls that overlap on the GPU (different streams, or different host
 // threads without ordering) race on it and must not be issued concurrently.

@@ -4,20 +4,25 @@
 // running CPathIntegrator::Li (raytracer/include/integrators/path_integrator_impl.hpp:120-247)
 // with direct() (23-118) once per spp launch (raytracer/raytracer.cu:161-210).
 //
-// Here one wave is one sample of every pixel.  Per bounce:
-//   k_extend  closest hit of every live path (BVH + analytic shapes, and in
-//             scenes with media the medium boxes: entering / traversing a
-//             medium runs delta tracking, and material-less medium hits are
-//             passed through inside the kernel without counting a bounce,
-//             exactly like the reference's `--bounces; continue`);
-//   k_shade   miss / surface or medium-collision shading: next-event
+// Here one wave is a number of samples of every pixel.  Per bounce:
+//   k_extend  closest surface hit of every live path (wide BVH, analytic shapes);
+//   k_find, k_track, k_walk  (media) the path through the medium boxes up to that
+//             hit: delta tracking along its segments, in queued rounds where
+//             paths are many and by a persistent kernel; material-less medium
+//             hits are passed through without counting a bounce, exactly like
+//             the reference's `--bounces; continue`;
+//   k_collide, k_events  (media) the collisions' events, and the bounce's list of
+//             surface hits and collisions;
+//   k_shade   surface or medium-collision shading: next-event
 //             estimation from the environment map and the BSDF- or
 //             phase-sampled MIS ray become two shadow records; the
 //             continuation ray, Russian roulette and the push of the surviving
 //             path into the next queue (warp ballot + popc);
-//   k_shadow  transmittance of every shadow record (any-hit against surfaces,
-//             then ratio tracking through the media boxes along the ray);
+//   k_shadow_surfaces  any-hit of every shadow record against surfaces; then
+//             (media) k_find, k_track, k_walk: ratio tracking through the boxes;
 //   k_accum   L += (L_light * tr + L_bsdf * tr) * T for the bounce.
+// The shadow rays and their accumulation run on a second stream, beside the next
+// bounce's extension.
 // All kernels are grid-stride over a live count read on the device, so a
 // wave is a fixed launch sequence (graph-capturable, no host round trips).
 // Random numbers: Philox4x32-10 keyed by (pixel, seed), counter (sample,
@@ -473,7 +478,7 @@ __device__ __forceinline__ float extend_tmax(const RenderLaunch& L, uint32_t p) 
 }
 
 // One instantiation per traversal variant (no triangles; alpha test, two
-// levels, shared top nodes), each with its own register allocation.
+// levels), each with its own register allocation.
 template <bool kTris, bool kAlpha, bool kInst>
 __global__ void __launch_bounds__(kTraceWarps * 32, 8) k_extend(RenderLaunch L) {
   const uint32_t n = *(volatile uint32_t*)&L.st.counts[L.bounce];

@@ -81,7 +81,7 @@ struct PathState {
   uint32_t* sq[2];  // the same of shadow slots
 };
 
-// Most wide BVH nodes the surface traversals stage in shared memory (20 KB per block).
+// top_nodes of a tuning, largest: accepted, without effect.
 constexpr uint32_t kMaxTopNodes = 256;
 // Launch tuning defaults (RenderLaunch::trackSteps, travVisits, travRefill);
 // no result depends on them.
