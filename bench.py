@@ -1035,7 +1035,7 @@ def bench_volume_batch(args, world, local):
     # blocks per branch can pay where one scene alone wants them all): set-up, untimed
     best = None
     for blocks in (tuned.track_blocks, 4, 3):
-        t = R.tuning(*tuned.as_tuple()[:5], blocks)
+        t = R.tuning(*tuned.as_tuple()[:4], 0, blocks)  # the batch's own number of media rounds
         for sc in scs:
             sc.set_tuning(t)
         b = R.RenderBatch(scs, cams, prms, [f.data_ptr() for f in frames])
@@ -1128,7 +1128,8 @@ def bench_volume_batch(args, world, local):
             "e2e": {"value": world * paths / (e2e_ms / 1e3), "unit": "paths/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(sum(npix) * 12), "ms_per_step": e2e_ms},
             "gpu_launches": c["spp"] * c["scenes"] * args.steps *
-            (3 + media_launches(batch_tuning.as_dict(), npix[0]) * c["depth"])}
+            (3 + media_launches(dict(batch_tuning.as_dict(), media_rounds=batch_tuning.media_rounds or 2), npix[0]) *
+             c["depth"])}
 
 
 def serving_jobs(c=SERVE_CFG, seed=11):

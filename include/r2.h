@@ -296,7 +296,8 @@ typedef struct r2_render_tuning {
   uint32_t wave_paths;  /* paths per wave: a wave renders the largest divisor of spp samples of every
                            pixel that keeps width*height*samples within it (at least one sample) */
   uint32_t media_rounds; /* media: queued rounds of medium boundaries (1..32) in bounces of many paths, before
-                            the remaining boundaries are walked in one persistent kernel */
+                            the remaining boundaries are walked in one persistent kernel (default 1, in a batch of
+                            several frames 2) */
   uint32_t track_blocks; /* media: blocks per SM of the persistent trackers (at most the resident
                             blocks; 0: all of them) */
   uint32_t track_limit; /* media: bound on the steps of one tracking loop (delta / ratio tracking of

@@ -105,8 +105,13 @@ constexpr uint32_t kServeWavePaths = 1u << 22;
 // 19.1 / 19.7 / 19.9.  In waves below 2^18 paths the launches cost more than they
 // bring: 820x114, 2 samples 4.04 ms against 3.56, 191x439, 3 samples 7.9 against 7.2.
 // One round or two or four: 227 / 228 / 230 ms of the volume, 133 / 129 / 130 of the
-// trees, and in waves of 4M paths 314 / 327 of the volume.
-constexpr uint32_t kDefaultMediaRounds = 1, kMaxMediaRounds = 32;
+// trees, in waves of 4M paths 314 / 327 of the volume, 128^3 foliage at 960x540, 8
+// samples 6.3 / 6.7.  In a batch a scene's waves are of one sample and run beside the
+// others': two rounds, and each scene's shadow rays on its own stream after its
+// paths.  Sixteen 1080p volumes, 4 samples, 4 tracker blocks an SM: 1082 ms with one
+// round and the second stream, 1046 without the stream, 1033 with two rounds, 1004
+// with two and without.
+constexpr uint32_t kDefaultMediaRounds = 1, kBatchMediaRounds = 2, kMaxMediaRounds = 32;
 constexpr uint32_t kRoundPaths = 1u << 17;
 // What the tuner tries of each setting: the default among them (the current value
 // is not timed against itself), and the waves of served jobs.

@@ -1057,7 +1057,11 @@ RenderBatch::RenderBatch(const std::vector<RenderScene*>& scenes, const std::vec
     for (size_t i = 0; i < n; ++i) {
       cudaStream_t b = ctx_[i]->stream;
       R2_CUDA(cudaStreamWaitEvent(b, evs[n], 0));
-      launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, ctx_[i]->side);
+      // the other frames fill the GPU beside a bounce's shadow rays (kBatchMediaRounds)
+      WaveSide side = ctx_[i]->side;
+      if (n > 1) side.stream = b;
+      if (n > 1 && Ls[i].mediaRounds == 0) Ls[i].mediaRounds = kBatchMediaRounds;
+      launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, side);
       R2_CUDA(cudaEventRecord(evs[i], b));
       R2_CUDA(cudaStreamWaitEvent(cap, evs[i], 0));
     }
