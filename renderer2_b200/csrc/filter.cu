@@ -29,6 +29,7 @@
 #include "filter.cuh"
 #include "filter_math.h"
 #include "texture_shade.cuh"
+#include "tri_ball.h"
 
 namespace r2 {
 namespace {
@@ -114,57 +115,9 @@ __device__ __forceinline__ bool box_overlap(float lox, float hix, float loy, flo
   return !(lox > qhi.x || hix < qlo.x || loy > qhi.y || hiy < qlo.y || loz > qhi.z || hiz < qlo.z);
 }
 
-// Tests of one triangle against balls of radius r whose centres lie within
-// `around` of c0.  near() is false only when the ball cannot touch the
-// triangle: it is out of reach of the plane, or of all three edges while its
-// centre projects outside the triangle.  The radius grows by 2e-6 of the
-// vertices' distances, more than the rounding of the products; the plane and
-// the side tests give way by the rounding of their cross products, so a sliver
-// whose normal is only rounding is left to its edges, and a NaN rejects
-// nothing.
-struct TriBall {
-  V3 p0, p1, AB, BC, AC, n, m0, m1, m2;  // vertices, edges, normal, the edges' outward normals
-  float i0, i1, i2;                      // 1 / squared edge lengths (0 for an edge without length)
-  float rr, plane, side;                 // squared padded radius; bounds of the plane and the side tests
-};
-__device__ __forceinline__ TriBall tri_ball(V3 p0, V3 p1, V3 p2, V3 c0, float around, float r) {
-  TriBall t;
-  t.p0 = p0;
-  t.p1 = p1;
-  t.AB = p1 - p0;
-  t.BC = p2 - p1;
-  t.AC = p2 - p0;
-  const V3 a = vabs(p0 - c0), b = vabs(p1 - c0), c = vabs(p2 - c0);
-  const float far = fmaxf(fmaxf(a.x + a.y + a.z, b.x + b.y + b.z), c.x + c.y + c.z) + around;
-  const float rp = r + 2e-6f * far;
-  t.rr = rp * rp;
-  const float e0 = dot(t.AB, t.AB), e1 = dot(t.BC, t.BC), e2 = dot(t.AC, t.AC);
-  t.i0 = e0 > 1e-30f ? __frcp_rn(e0) : 0.0f;
-  t.i1 = e1 > 1e-30f ? __frcp_rn(e1) : 0.0f;
-  t.i2 = e2 > 1e-30f ? __frcp_rn(e2) : 0.0f;
-  t.n = cross(t.AB, t.AC);
-  t.m0 = cross(t.AB, t.n);
-  t.m1 = cross(t.BC, t.n);
-  t.m2 = cross(t.n, t.AC);
-  const float area = e0 + e1 + e2;  // more than |AB| |AC|
-  t.plane = rp * sqrtf(dot(t.n, t.n)) + 2e-6f * (far + rp) * area;
-  t.side = 4e-6f * far * area * sqrtf(area);
-  return t;
-}
-__device__ __forceinline__ float edge_dist2(V3 a, V3 e, float inv) {  // of the origin from the edge a + [0, 1] e
-  const V3 q = a + e * clampf(-dot(a, e) * inv, 0.0f, 1.0f);
-  return dot(q, q);
-}
-__device__ __forceinline__ bool tri_near(const TriBall& t, V3 c) {
-  const V3 A = t.p0 - c, B = t.p1 - c;
-  const float d2 = fminf(fminf(edge_dist2(A, t.AB, t.i0), edge_dist2(B, t.BC, t.i1)), edge_dist2(A, t.AC, t.i2));
-  // the centre lies outside an edge where its outward normal points back to the edge's vertex
-  const float out = fminf(fminf(dot(A, t.m0), dot(B, t.m1)), dot(A, t.m2));
-  return !(fabsf(dot(A, t.n)) > t.plane) && (!(d2 > t.rr) || !(out < -t.side));
-}
-__device__ __forceinline__ TriBall load_tri_ball(const BvhView& bvh, int t, V3 c0, float around, float r) {
-  const float4 a = __ldg(&bvh.tris[3 * t]), b = __ldg(&bvh.tris[3 * t + 1]), c = __ldg(&bvh.tris[3 * t + 2]);
-  return tri_ball(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), c0, around, r);
+__device__ __forceinline__ TriBall load_tri_ball(const FilterLaunch& L, int t, V3 c0, float around, float r) {
+  const float4 a = __ldg(&L.bvh.tris[3 * t]), b = __ldg(&L.bvh.tris[3 * t + 1]), c = __ldg(&L.bvh.tris[3 * t + 2]);
+  return tri_ball(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), c0, around, r, L.ballScale);
 }
 
 // Does any triangle box overlap the query box?
@@ -229,7 +182,7 @@ __device__ int bvh_local_root(const BvhView& bvh, V3 qlo, V3 qhi) {
 // that can touch the ball: appended to list, the lanes' first triangles, then
 // their second ones, and so on.  Returns the list's new length, or -1 when it
 // would pass kCandMax.
-__device__ __forceinline__ int near_triangles(const BvhView& bvh, const int* refs, int n, V3 qlo, V3 qhi, V3 center,
+__device__ __forceinline__ int near_triangles(const FilterLaunch& L, const int* refs, int n, V3 qlo, V3 qhi, V3 center,
                                               float r, int* list, int len, int lane) {
   const int ref = lane < n ? refs[lane] : 0;
   const int first = bvh_leaf_first(ref), count = lane < n ? bvh_leaf_count(ref) : 0;
@@ -237,11 +190,12 @@ __device__ __forceinline__ int near_triangles(const BvhView& bvh, const int* ref
     bool near = false;
     if (k < count) {
       const int t = first + k;
-      const float4 a = __ldg(&bvh.tris[3 * t]), b = __ldg(&bvh.tris[3 * t + 1]), c = __ldg(&bvh.tris[3 * t + 2]);
+      const float4 a = __ldg(&L.bvh.tris[3 * t]), b = __ldg(&L.bvh.tris[3 * t + 1]), c = __ldg(&L.bvh.tris[3 * t + 2]);
       near = box_overlap(fminf(fminf(a.x, b.x), c.x), fmaxf(fmaxf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y),
                          fmaxf(fmaxf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z), fmaxf(fmaxf(a.z, b.z), c.z), qlo,
                          qhi) &&
-             tri_near(tri_ball(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), center, 0.0f, r), center);
+             tri_near(tri_ball(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), center, 0.0f, r, L.ballScale),
+                      center);
     }
     const unsigned m = __ballot_sync(0xFFFFFFFFu, near);
     const int added = __popc(m);
@@ -262,7 +216,7 @@ __device__ __forceinline__ int near_triangles(const BvhView& bvh, const int* ref
 // fetches (the tree's depth) and not 100.  scratch: kWalkInts ints.  Returns
 // the number of candidates, or -1 when there are more than kCandMax or the
 // stack is full.  nodes: inner nodes visited by this lane (the counting build).
-__device__ int gather_candidates(const BvhView& bvh, V3 qlo, V3 qhi, V3 center, float r, int* list, int* scratch,
+__device__ int gather_candidates(const FilterLaunch& L, V3 qlo, V3 qhi, V3 center, float r, int* list, int* scratch,
                                  int lane, uint32_t* nodes) {
   int* stack = scratch;
   int* leaves = scratch + kWalkStack;
@@ -276,7 +230,7 @@ __device__ int gather_candidates(const BvhView& bvh, V3 qlo, V3 qhi, V3 center, 
     int c0 = R2_BVH_NONE, c1 = R2_BVH_NONE;
     if (lane < take) {
       ++*nodes;
-      const BvhNode* nd = &bvh.nodes[stack[sp + lane]];
+      const BvhNode* nd = &L.bvh.nodes[stack[sp + lane]];
       const float4 b0 = __ldg(&nd->b0), b1 = __ldg(&nd->b1), bz = __ldg(&nd->bz);
       const int4 ch = __ldg(&nd->ch);
       if (box_overlap(b0.x, b0.y, b0.z, b0.w, bz.x, bz.y, qlo, qhi)) c0 = ch.x;
@@ -298,7 +252,7 @@ __device__ int gather_candidates(const BvhView& bvh, V3 qlo, V3 qhi, V3 center, 
     while (nleaf >= 32 || (sp == 0 && nleaf > 0)) {
       const int n = min(nleaf, 32);
       nleaf -= n;
-      len = near_triangles(bvh, leaves + nleaf, n, qlo, qhi, center, r, list, len, lane);
+      len = near_triangles(L, leaves + nleaf, n, qlo, qhi, center, r, list, len, lane);
       if (len < 0) return -1;
     }
   }
@@ -494,7 +448,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32) k_filter_lists(FilterLaunch
   for (uint32_t w = blockIdx.x * kSampleWarps + warp; w < nbricks; w += gridDim.x * kSampleWarps) {
     const Brick k = brick_at(L, kAll ? L.brickFirst + w : L.bricks[w]);
     uint32_t walked = 0;
-    const int n = gather_candidates(L.bvh, k.center - v3(k.r), k.center + v3(k.r), k.center, k.r, cand, sScratch[warp],
+    const int n = gather_candidates(L, k.center - v3(k.r), k.center + v3(k.r), k.center, k.r, cand, sScratch[warp],
                                     lane, &walked);
     __syncwarp();
     int x, y, z;
@@ -504,7 +458,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32) k_filter_lists(FilterLaunch
     for (int base = 0; base < n; base += 32) {
       const bool valid = base + lane < n;
       const float r = padded_reach(reach, k.center) + 1e-5f * L.brickOffset * 2.0f;  // any of its voxels' padded reach
-      const TriBall t = load_tri_ball(L.bvh, cand[valid ? base + lane : base], k.center, 2.0f * k.r, r);
+      const TriBall t = load_tri_ball(L, cand[valid ? base + lane : base], k.center, 2.0f * k.r, r);
       for (int v = 0; v < 8; ++v) {
         int vx, vy, vz;
         const bool in = brick_voxel(L, k, v, &vx, &vy, &vz);
@@ -720,7 +674,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32, 8) k_filter_sample(FilterLa
       for (int i = lane; i < ncand; i += 32) myCand[i] = L.pool[entry.y + 1 + i];
     } else {
       const float pad = padded_reach(ray_reach(L), center);  // every sample ray stays within it
-      ncand = gather_candidates(L.bvh, center - v3(pad), center + v3(pad), center, pad, myCand,
+      ncand = gather_candidates(L, center - v3(pad), center + v3(pad), center, pad, myCand,
                                 reinterpret_cast<int*>(myV), lane, &cNodes);
       if (ncand < 0) root = bvh_local_root(L.bvh, center - v3(pad), center + v3(pad));
     }

@@ -35,6 +35,7 @@ struct FilterLaunch {
   // list in the pool, from both ends) and the counters.
   uint32_t brickFirst, brickCount;
   float brickOffset;         // from a brick's centre to its farthest voxel centre
+  float ballScale;           // of the triangle tests (tri_ball.h)
   uint32_t* bricks;
   uint2* entries;
   int* pool;                 // candidate lists: their length, then triangles

@@ -7,6 +7,7 @@
 
 #include "filter.cuh"
 #include "filter_host.h"
+#include "tri_ball.h"
 #include "filter_math.h"
 #include "host_math.h"
 
@@ -274,6 +275,7 @@ void FilterScene::run(const r2_filter_grid& g, const r2_filter_params& p, uint32
            hz = xform_vector(L.indexToWorld, v3(0.0f, 0.0f, 0.5f));
   L.brickOffset = std::max(std::max(length(hx + hy + hz), length(hx + hy - hz)),
                            std::max(length(hx - hy + hz), length(hy + hz - hx)));
+  L.ballScale = ball_scale(length(L.voxelSize));
   // The grid in parts of bricks whose lists fit the work space: of W words,
   // W / 6 voxels at most, two words each for their entries (first: they are
   // 8-byte aligned), one per brick, and what is left for candidate lists.

@@ -1,11 +1,12 @@
-// What the tests of the eight-wide BVH call below the library's C interface:
-// the collapse's choice of children over a host-built binary tree (no GPU), and
+// What tests call below the library's C interface: the filter's test of a
+// triangle against a ball (no GPU); of the eight-wide BVH the collapse's choice of children over a host-built binary tree (no GPU), and
 // the closest hits of given rays through the wide tree and through the binary
 // one over the same build.  Compiled and loaded by wide_probe.py.
 #include <cstring>
 #include <vector>
 
 #include "bvh_build.cuh"
+#include "tri_ball.h"
 #include "wide_bvh.cuh"
 
 using namespace r2;
@@ -116,6 +117,19 @@ __global__ void k_visits(WideView wide, const Ray* rays, uint32_t n, uint32_t* v
 }  // namespace
 
 extern "C" {
+
+// near[k]: whether tri_near keeps triangle k (9 floats) for a ball of radius r[k] about c[3k..], whose test was set up
+// for centres within around[k] of c0[3k..], among voxels of the given size.
+void probe_tri_near(const float* tris, const float* c0, const float* around, const float* c, const float* r, float voxel,
+                    uint32_t n, int* near) {
+  const float scale = ball_scale(voxel);
+  const auto at = [](const float* p) { return v3(p[0], p[1], p[2]); };
+  for (uint32_t k = 0; k < n; ++k) {
+    const float* t = tris + 9 * (size_t)k;
+    near[k] = tri_near(tri_ball(at(t), at(t + 3), at(t + 6), at(c0 + 3 * (size_t)k), around[k], r[k], scale),
+                       at(c + 3 * (size_t)k));
+  }
+}
 
 // Wide nodes of the collapse of a binary tree over the leaf boxes (skew: 0 halves, 1 splits anywhere); *capacity: what
 // the builder has room for.

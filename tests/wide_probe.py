@@ -25,6 +25,8 @@ def lib():
         _lib = C.CDLL(LIB)
         _lib.probe_wide_nodes.restype = C.c_uint64
         _lib.probe_wide_nodes.argtypes = [C.c_void_p, C.c_uint32, C.c_int, C.c_uint32, C.c_void_p]
+        _lib.probe_tri_near.argtypes = [C.c_void_p] * 5 + [C.c_float, C.c_uint32, C.c_void_p]
+        _lib.probe_tri_near.restype = None
         _lib.probe_trace.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32] + [C.c_void_p] * 5
     return _lib
 
@@ -54,3 +56,12 @@ def trace(tris, rays):
     for h in (a, b, c):
         h["t"][h["tri"] < 0] = 0.0
     return a, b, c, seen != 0, visits
+
+
+def tri_near(tris, c0, around, c, r, voxel):
+    """Whether the filter keeps each (n, 3, 3) triangle for the ball of radius r about c (test set up for centres within
+    `around` of c0), among voxels of the given size."""
+    a = [np.ascontiguousarray(x, np.float32) for x in (tris, c0, around, c, r)]
+    near = np.empty(a[0].shape[0], np.int32)
+    lib().probe_tri_near(*(x.ctypes.data for x in a), float(voxel), near.size, near.ctypes.data)
+    return near != 0
