@@ -118,3 +118,19 @@ def test_a_filter_job_is_admitted_with_the_work_space_it_takes():
             assert e.value.name == "R2_ERR_ADMISSION_REJECTED"
         srv.close()
     sc.close()
+
+
+def test_a_served_frame_keeps_to_the_budget():
+    """A scene tuned to large waves is served in waves of 4M paths where the budget has no room for them, with the same
+    frame."""
+    from renderer2_b200 import serving as S
+    sc, cam, prm = _scene()
+    want = _render(sc, cam, prm)[0].cpu().numpy()
+    sc.set_tuning(R.tuning(wave_paths=1 << 24))
+    assert S.Server.render_bytes(sc, cam, prm) > 2 * GB
+    srv = S.Server(1, 2 * GB)
+    job = srv.submit_render(sc, cam, prm)
+    srv.wait(job)
+    srv.close()
+    sc.close()
+    assert np.array_equal(job.out, want)
