@@ -524,7 +524,8 @@ def bench_render(args, world, local):
                 "alg_bytes_per_launch": alg / launches, "avg_launch_ms": kms / launches,
                 "samples_per_wave": S,
                 "note": "per-launch figures averaged over the bounces of the timed middle wave; "
-                        "traversal is L2/issue bound, see rays_per_s",
+                        "traversal is issue bound, see rays_per_s; a bounce's shadow rays overlap the next one's "
+                        "extension, so the times of these two stages contain each other's work",
                 "rays_per_s": (seg + shadow) / (st[1] / 1e3), "kernel_ms_per_wave": ms_wave}
     # end to end through the C ABI with host buffers, every step: the frame's world-space vertices and normals
     # copied from pinned host memory (r2_scene_set_vertices), the BVH rebuilt (r2_scene_rebuild), the frame
@@ -680,7 +681,8 @@ def surface_roofline(st, S, spp, launches):
     achieved = alg / (kms / 1e3) / 1e9
     return {"bound": "hbm", "kernel": "k_extend" if dom_ext else "k_shadow_surfaces", "achieved": achieved,
             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": kind,
-            "alg_bytes_per_launch": alg / launches, "avg_launch_ms": kms / launches, "samples_per_wave": S}
+            "alg_bytes_per_launch": alg / launches, "avg_launch_ms": kms / launches, "samples_per_wave": S,
+            "note": "shadow and extend stages overlap, so their times contain each other's work"}
 
 
 def bench_small(args, world, local):
@@ -820,7 +822,8 @@ def media_roofline(st, S, spp, depth):
             "frac": achieved / peak, "peak_source": peak_kind,
             "traffic": tr["bytes_per_unit"] * per_unit[1] / depth if tr else None,
             "alg_bytes_per_launch": alg / depth, "avg_launch_ms": kms / depth,
-            "note": "delta/ratio tracking is latency bound on dependent grid lookups",
+            "note": "delta/ratio tracking is latency bound on dependent grid lookups; shadow and extend stages overlap, "
+                    "so their times contain each other's work",
             "kernel_ms_per_wave": ms_wave}
 
 
