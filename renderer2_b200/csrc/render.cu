@@ -1466,6 +1466,7 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
   k_camera<<<nblocks, 256, 0, s>>>(L);
   mark(0);
   const int tv = trav_variant(L);
+  bool forked = false;
   for (uint32_t b = 0; b < L.maxDepth; ++b) {
     L.bounce = b;
     if (media) {
@@ -1485,25 +1486,30 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
       kExtendVariants[tv]<<<std::min(nblocks * 2, trav_blocks(0, tv)), kTraceWarps * 32, 0, s>>>(L);
     }
     mark(1);
-    if (b > 0) {  // the last bounce's shadow records are free
+    if (forked) {  // the last bounce's shadow records are free
       R2_CUDA(cudaStreamWaitEvent(s, side.join, 0));
       mark(-1);
     }
     kShadeVariants[(media ? 4 : 0) + shade_variant(L)]<<<nblocks * 2, 128, 0, s>>>(L);
     mark(2);
-    // the bounce's shadow rays beside the next bounce's extension
-    R2_CUDA(cudaEventRecord(side.fork, s));
-    R2_CUDA(cudaStreamWaitEvent(side.stream, side.fork, 0));
-    mark(-1, true);
-    kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, side.stream>>>(L);
-    if (media) launch_media(L, false, nblocks, side.stream);
-    mark(3, true);
-    k_accum<<<nblocks, 256, 0, side.stream>>>(L);
-    mark(4, true);
-    R2_CUDA(cudaEventRecord(side.join, side.stream));
+    forked = b < side.bounces;
+    const cudaStream_t ss = forked ? side.stream : s;
+    if (forked) {  // the bounce's shadow rays beside the next bounce's extension
+      R2_CUDA(cudaEventRecord(side.fork, s));
+      R2_CUDA(cudaStreamWaitEvent(side.stream, side.fork, 0));
+      mark(-1, true);
+    }
+    kShadowVariants[tv]<<<std::min(nblocks * 2, trav_blocks(1, tv)), kTraceWarps * 32, 0, ss>>>(L);
+    if (media) launch_media(L, false, nblocks, ss);
+    mark(3, forked);
+    k_accum<<<nblocks, 256, 0, ss>>>(L);
+    mark(4, forked);
+    if (forked) R2_CUDA(cudaEventRecord(side.join, side.stream));
   }
-  R2_CUDA(cudaStreamWaitEvent(s, side.join, 0));
-  mark(-1);
+  if (forked) {
+    R2_CUDA(cudaStreamWaitEvent(s, side.join, 0));
+    mark(-1);
+  }
   k_finish<<<nblocks, 256, 0, s>>>(L);
   mark(5);
   if (L.sampleDev) k_advance_sample<<<1, 1, 0, s>>>(L.sampleDev, L.waveSpp);

@@ -200,7 +200,16 @@ struct WaveTimer {
 struct WaveSide {
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  uint32_t bounces = 64;  // of which the shadow rays go to it; the others' stay on the wave's own stream
 };
+// Bounces of a served job's captured wave that fork to it, in waves of at least so
+// many paths: every fork costs in the graph's instantiation and launch.  Without
+// forks / in the first 2 / 4 / 8 / 16 bounces, eight jobs on four slots, ms (one
+// stream and the binary tree before: in brackets): 64x64, 4 samples, 50 bounces
+// 9.2 / 8.4 / 10.2 / 13.0 / 18.5 (12.2; 46.6 with all bounces forked); 256x256, 1 sample
+// 4.5 / 5.6 / 7.3 / 9.6 / 9.3 (5.5); 512x512, 4 samples, 50 bounces 26.9 / 26.1 / 25.2 /
+// 24.1 / 24.5 (34.6); 1280x720, 32 samples 329 / 322 / 314 / 304 / 304 (428).
+constexpr uint32_t kCapturedForks = 8, kCapturedForkPaths = 1u << 18;
 
 // One wave (L.waveSpp consecutive samples of every pixel) on s and side, which
 // rejoins s before the wave ends.  With L.sampleDev the last launch advances

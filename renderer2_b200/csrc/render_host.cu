@@ -898,7 +898,9 @@ void RenderScene::render_graph(RenderContext& ctx, const r2_camera& c, const r2_
   } guard{cap};
   R2_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   try {
-    launch_render_wave(L, wave_blocks(npix * S), cap, ctx.side);
+    WaveSide side = ctx.side;
+    side.bounces = npix * S >= kCapturedForkPaths ? kCapturedForks : 0;
+    launch_render_wave(L, wave_blocks(npix * S), cap, side);
   } catch (...) {
     cudaGraph_t g = nullptr;
     cudaStreamEndCapture(cap, &g);
@@ -1059,7 +1061,7 @@ RenderBatch::RenderBatch(const std::vector<RenderScene*>& scenes, const std::vec
       R2_CUDA(cudaStreamWaitEvent(b, evs[n], 0));
       // the other frames fill the GPU beside a bounce's shadow rays (kBatchMediaRounds)
       WaveSide side = ctx_[i]->side;
-      if (n > 1) side.stream = b;
+      if (n > 1) side.bounces = 0;
       if (n > 1 && Ls[i].mediaRounds == 0) Ls[i].mediaRounds = kBatchMediaRounds;
       launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, side);
       R2_CUDA(cudaEventRecord(evs[i], b));
