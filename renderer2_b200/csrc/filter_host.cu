@@ -74,16 +74,16 @@ static int grid_for(uint32_t n) {
   return (int)std::max<uint32_t>(1u, std::min<uint32_t>((n + 255) / 256, (uint32_t)sm_count() * 16));
 }
 
-// Words of the scene's own work space: the scratch of its BVH build where that
-// has four per voxel; else 24 per voxel up to 16 MiB, so that the lists of a
-// small dense grid fit (the 48^3 grid of 400,000 triangles needs 22 a voxel),
-// then at least two per voxel (a quarter of the output; the 256^3 grid of 1M
-// triangles uses 1.8) up to kMaxWork: larger grids are filtered in parts.
 constexpr size_t kMaxWork = (size_t)1 << 24;
-static size_t work_words(size_t nvox, size_t have) {
-  if (have >= std::min(std::max(4 * nvox, kFilterMinWork), kMaxWork)) return have;
+size_t filter_work_words(size_t nvox) {
   const size_t small = std::min<size_t>(24 * nvox, (size_t)1 << 22);
   return std::min<size_t>(std::max(std::max<size_t>(2 * nvox, small), kFilterMinWork), kMaxWork);
+}
+
+// Words of the scene's own work space: the scratch of its BVH build where that
+// has four per voxel.
+static size_t work_words(size_t nvox, size_t have) {
+  return have >= std::min(std::max(4 * nvox, kFilterMinWork), kMaxWork) ? have : filter_work_words(nvox);
 }
 
 // SAABB::transform (include/intersect/aabb.hpp:9-13): only the min and max

@@ -11,6 +11,11 @@ r2_filter_grid setup_grid(V3 minWorld, V3 maxWorld, const M43& worldToModel, flo
 void world_aabb(V3 mlo, V3 mhi, const M43& modelToWorld, V3* wlo, V3* whi);
 
 constexpr size_t kFilterMinWork = 1u << 16;  // least words of a work space
+// Words that let most grids run in one part: 24 per voxel up to 16 MiB, so that
+// the lists of a small dense grid fit (the 48^3 grid of 400,000 triangles needs 22
+// a voxel), then at least two per voxel (a quarter of the output; the 256^3 grid of
+// 1M triangles uses 1.8) up to 64 MiB: larger grids are filtered in parts.
+size_t filter_work_words(size_t nvox);
 
 class FilterScene {
  public:

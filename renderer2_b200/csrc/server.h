@@ -42,6 +42,7 @@ struct ServerJob {
   r2_filter_params fp;
   uint32_t lod = 0;
   r2_voxel* voxOut = nullptr;
+  size_t workWords = 0;
   // accounting
   size_t bytes = 0;        // device memory the job holds while admitted
   size_t outBytes = 0;

@@ -134,3 +134,24 @@ def test_a_served_frame_keeps_to_the_budget():
     srv.close()
     sc.close()
     assert np.array_equal(job.out, want)
+
+
+@pytest.mark.parametrize("spare", [1 << 30, 1 << 18], ids=["room", "tight"])
+def test_a_served_filter_equals_a_direct_one(spare):
+    """With the work space that suits the grid, and with the least, where the grid takes several parts."""
+    from renderer2_b200 import _native as N
+    from renderer2_b200 import filter as F
+    from renderer2_b200 import scenes
+    from renderer2_b200 import serving as S
+    mesh = scenes.foliage(8000, 6, 0.7, 5)
+    sc = F.FilterScene(mesh, F.material())
+    g, prm = sc.grid(scenes.voxel_size_for(mesh, 37)), F.params(samples_per_voxel=32, iterations=3)
+    nvox = int(np.prod(np.array(g.num_voxels[:], np.int64)))
+    want = torch.empty(nvox * 32, dtype=torch.uint8, device="cuda")
+    sc.run(g, prm, want.data_ptr())
+    srv = S.Server(1, 32 * (1 << (nvox - 1).bit_length()) + spare + 64)
+    job = srv.submit_filter(sc, g, prm)
+    srv.wait(job)
+    srv.close()
+    sc.close()
+    assert np.array_equal(job.out.view(np.uint8), want.cpu().numpy()) and job.out.dtype == N.VOXEL_DTYPE
