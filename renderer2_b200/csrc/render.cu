@@ -1103,7 +1103,7 @@ __device__ __forceinline__ bool shadow_walk(const RenderLaunch& L, uint32_t slot
 // are found their next segment in the following round, and after the last round
 // k_walk takes them to their end.  k_track holds tentative collisions as k_walk does.
 __device__ __forceinline__ bool in_rounds(const RenderLaunch& L, uint32_t live) {
-  return L.mediaRounds > 0 && live >= kRoundPaths;
+  return L.mediaRounds > 0 && live >= L.roundPaths;
 }
 
 template <bool kSample>
@@ -1448,7 +1448,8 @@ void launch_render_wave(const RenderLaunch& L0, int nblocks, cudaStream_t s, con
   if (L.travVisits == 0) L.travVisits = kDefaultTravVisits;
   if (L.travRefill == 0) L.travRefill = kDefaultTravRefill;
   if (L.mediaRounds == 0) L.mediaRounds = kDefaultMediaRounds;
-  if (L.wavePaths < 2 * kRoundPaths) L.mediaRounds = 0;
+  if (L.roundPaths == 0) L.roundPaths = kRoundPaths;
+  if (L.wavePaths < 2 * L.roundPaths) L.mediaRounds = 0;
   query_track_blocks();
   const bool media = L.scene.nmedia > 0;
   int ev = 0, last[2] = {-1, -1};

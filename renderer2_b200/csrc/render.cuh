@@ -106,12 +106,17 @@ constexpr uint32_t kServeWavePaths = 1u << 22;
 // bring: 820x114, 2 samples 4.04 ms against 3.56, 191x439, 3 samples 7.9 against 7.2.
 // One round or two or four: 227 / 228 / 230 ms of the volume, 133 / 129 / 130 of the
 // trees, in waves of 4M paths 314 / 327 of the volume, 128^3 foliage at 960x540, 8
-// samples 6.3 / 6.7.  In a batch a scene's waves are of one sample and run beside the
-// others': two rounds, and each scene's shadow rays on its own stream after its
-// paths.  Sixteen 1080p volumes, 4 samples, 4 tracker blocks an SM: 1082 ms with one
-// round and the second stream, 1046 without the stream, 1033 with two rounds, 1004
-// with two and without.
+// samples 6.3 / 6.7.  In a batch of n
+// frames a wave is of one sample and runs beside the others': two rounds, from
+// 2 / n of the paths on, and the second stream for shadow rays only where the waves
+// have no more than kBatchForkPaths in all.  Sixteen 1080p volumes, 4 samples, 4
+// tracker blocks an SM: 1082 ms with one round and the second stream, 1046 without
+// the stream, 1033 with two rounds, 1004 with two and without.  Twelve volumes at
+// 640x360, 8 samples: 266 ms, 317 with rounds from kRoundPaths on (264 with rounds in
+// every bounce, inline ends and no second stream); two at 160x90 5.6 ms, 7.5 without the
+// second stream.
 constexpr uint32_t kDefaultMediaRounds = 1, kBatchMediaRounds = 2, kMaxMediaRounds = 32;
+constexpr size_t kBatchForkPaths = (size_t)1 << 24;
 constexpr uint32_t kRoundPaths = 1u << 17;
 // What the tuner tries of each setting: the default among them (the current value
 // is not timed against itself), and the waves of served jobs.
@@ -175,6 +180,7 @@ struct RenderLaunch {
   uint32_t travRefill;  // finished lanes of a warp that trigger a refill (tuning, 1..32)
   uint32_t trackBlocks; // persistent tracker blocks per SM (tuning; 0: every resident block)
   uint32_t mediaRounds; // queued rounds of a bounce's medium boundaries (tuning; 0: the default)
+  uint32_t roundPaths;  // paths of a bounce from which they are used (0: kRoundPaths)
   uint32_t trackLimit;  // steps of one tracking loop after which the path ends (1..kMaxTrackingSteps)
   uint32_t sortRays;    // surface scenes: reorder each bounce's rays by a coherence key before k_extend
   unsigned long long* stats;  // nullable: [0] path segments traced, [1] shadow rays traced

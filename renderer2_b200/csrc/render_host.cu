@@ -1035,6 +1035,8 @@ RenderBatch::RenderBatch(const std::vector<RenderScene*>& scenes, const std::vec
     frames_.push_back(frames[i]);
     npix_.push_back((size_t)cams[i].width * cams[i].height);
   }
+  size_t total = 0;  // paths of the batch's waves
+  for (size_t pixels : npix_) total += pixels;
   prepare_render_launches();  // occupancy queries stay outside the capture
   R2_CUDA(cudaEventCreate(&ev0_));
   R2_CUDA(cudaEventCreate(&ev1_));
@@ -1059,9 +1061,10 @@ RenderBatch::RenderBatch(const std::vector<RenderScene*>& scenes, const std::vec
     for (size_t i = 0; i < n; ++i) {
       cudaStream_t b = ctx_[i]->stream;
       R2_CUDA(cudaStreamWaitEvent(b, evs[n], 0));
-      // the other frames fill the GPU beside a bounce's shadow rays (kBatchMediaRounds)
+      // the other frames fill the GPU beside a bounce's shadow rays and the ends of rounds (kBatchMediaRounds)
       WaveSide side = ctx_[i]->side;
-      if (n > 1) side.bounces = 0;
+      if (total > kBatchForkPaths && n > 1) side.bounces = 0;
+      if (n > 1) Ls[i].roundPaths = std::max<uint32_t>(2 * kRoundPaths / (uint32_t)n, 1u);
       if (n > 1 && Ls[i].mediaRounds == 0) Ls[i].mediaRounds = kBatchMediaRounds;
       launch_render_wave(Ls[i], wave_blocks((uint32_t)npix_[i]), b, side);
       R2_CUDA(cudaEventRecord(evs[i], b));
